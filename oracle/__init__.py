@@ -179,7 +179,7 @@ def build_ref(reference_root: str | None = None, force: bool = False) -> list[Pa
     units = {"ref_bfs": "ref_bfs_unity.cu", "ref_pagerank": "ref_pagerank_unity.cu",
              "ref_pagerank_pull_warp": "ref_pagerank_pull_warp_unity.cu"}
     built = []
-    if not root.exists():
+    if not (root / "bfs").is_dir() or not (root / "pagerank").is_dir():     # absent or empty: nothing to compile
         return [out_dir / f"{k}.cubin" for k in units if (out_dir / f"{k}.cubin").exists()]
     out_dir.mkdir(exist_ok=True)
     for key, unit in units.items():
