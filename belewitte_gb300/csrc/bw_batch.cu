@@ -35,6 +35,9 @@ constexpr int BATCH_PR_UNROLL = 8;
 constexpr int BATCH_BFS_UNROLL = 4;
 constexpr uint32_t BATCH_BU_DIV = 24;     // default push/pull divisor: bottom-up above 1/24 of the unit
 constexpr uint32_t BATCH_PR_L = 8;        // warp sums: windows of 32 x 8 terms
+constexpr uint64_t PACKED_MAX_VERTICES = uint64_t(1) << 29;   // the work list's row ids
+constexpr uint32_t PACKED_MIN_UNIT = 4096;
+constexpr uint64_t PACKED_MIN_WORK = 16384;                   // vertices of the largest unit x iterations
 
 struct BatchArgs {
     const uint32_t *fwd_v, *fwd_e, *rev_v, *rev_e;
@@ -341,6 +344,20 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) k_batch(BatchArgs a)
     }
 }
 
+// Whether the graphs' PageRank runs as one set of rows over the whole GPU
+// (pagerank_run_packed) or inside k_batch, a CTA per graph.  A CTA sums about
+// 0.6 G terms/s, so a large graph ends long after the rest: 512 R-MAT graphs
+// of 1K-200K vertices (343M edges), BFS and 20 iterations, 109 ms in k_batch
+// and 30.5 ms packed on GB300; 16 graphs of 4K-200K 75 and 3.5 ms.  Small
+// graphs balance well on CTAs and need no set-up: 350 graphs of 1K-4K
+// vertices 1.65 and 1.83 ms, of 200-800 0.27 and 0.76 ms.  One iteration of
+// 64 graphs of up to 8K vertices: 0.19 and 0.26 ms (the set-up, 0.15 ms).
+bool packed_pagerank(const bw_graph_view *g, uint32_t max_unit_vertices, uint32_t iterations)
+{
+    return g->vertex_count < PACKED_MAX_VERTICES && max_unit_vertices >= PACKED_MIN_UNIT &&
+           uint64_t(max_unit_vertices) * iterations >= PACKED_MIN_WORK;
+}
+
 }  // namespace
 }  // namespace bw
 
@@ -389,7 +406,19 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
     a.qcap = max_unit_vertices;
     a.levels = levels;
     a.ranks = ranks;
-    a.pr_iters = mode == BW_BATCH_GRAPHS ? pr_iterations : 0;
+    const uint32_t pr = mode == BW_BATCH_GRAPHS ? pr_iterations : 0;
+    BW_CUDA(cudaEventRecord(ctx->ev_start, s));
+    a.pr_iters = pr;
+    if (pr && packed_pagerank(g, max_unit_vertices, pr)) {
+        const int rc = pagerank_run_packed(ctx, g, graph_offsets, graph_count, pr, ranks, s);
+        if (rc == BW_OK) {
+            a.pr_iters = 0;
+        } else if (rc == BW_ERR_OUT_OF_MEMORY) {
+            cudaGetLastError();                  // its scratch (about 5 bytes per edge) does not fit: a CTA per graph
+        } else {
+            return rc;
+        }
+    }
     a.vis_words = bitmap ? static_cast<uint32_t>(words) : 0u;
     a.bu_div = (cfg && cfg->chunk_size) ? cfg->chunk_size : BATCH_BU_DIV;
     const size_t per_cta = static_cast<size_t>(2) * max_unit_vertices;
@@ -401,7 +430,6 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
     a.traversed = reinterpret_cast<unsigned long long *>(scratch + 8);
     a.queues = reinterpret_cast<uint32_t *>(scratch + 64);
     a.contrib = a.pr_iters ? reinterpret_cast<float *>(scratch + 64 + grid * per_cta * sizeof(uint32_t)) : nullptr;
-    BW_CUDA(cudaEventRecord(ctx->ev_start, s));
     k_batch<<<grid, BATCH_THREADS, dyn, s>>>(a);
     BW_CUDA(cudaGetLastError());
     BW_CUDA(cudaEventRecord(ctx->ev_stop, s));

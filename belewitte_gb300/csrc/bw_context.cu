@@ -100,6 +100,7 @@ int ensure_outdeg(bw_context *ctx, const bw_graph_view *g, cudaStream_t s)
 int ensure_pr_scratch(bw_context *ctx, uint64_t n, uint32_t iterations)
 {
     if (n > ctx->pr_n_cap) {
+        ctx->pr_n_cap = 0;               // until all of them have grown
         BW_TRY(grow(&ctx->pr_acc, n));
         // both contribution buffers in one allocation, so one L2
         // access-policy window covers the vector every iteration gathers;

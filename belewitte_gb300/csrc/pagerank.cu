@@ -119,6 +119,11 @@ struct PrArgs {
     const uint32_t *hot_vertex;
     const uint32_t *hot_count;    // device: slots in use
     double base_div;           // (1.0 - 0.85f) / N, computed once on the host
+    // Packed graphs (bw_batch_run): graph i owns the vertices
+    // [goff[i], goff[i + 1]) and has its own base term.
+    const uint32_t *goff;
+    const double *gbase;
+    uint32_t graphs;
 };
 
 __device__ __forceinline__ uint64_t gtid() { return blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; }
@@ -151,6 +156,21 @@ __device__ __forceinline__ float consolidate_div(float acc, double base)
                                               __float_as_uint(scaled), ok);
     if (ok) return __uint_as_float(r);
     return __double2float_rn(__dadd_rn(base, static_cast<double>(scaled)));   // outside the emulated domain
+}
+
+// The graph of vertex v of packed graphs: the last that starts at v or
+// before (an empty one starts where the next does, so it is never the last);
+// NO_GRAPH for a vertex of none, which keeps its rank.
+constexpr uint32_t NO_GRAPH = 0xffffffffu;
+__device__ __forceinline__ uint32_t graph_of(const PrArgs &a, uint64_t v)
+{
+    if (v < a.goff[0] || v >= a.goff[a.graphs]) return NO_GRAPH;
+    uint32_t lo = 0, hi = a.graphs - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) / 2;
+        if (a.goff[mid] <= v) lo = mid; else hi = mid - 1;
+    }
+    return lo;
 }
 
 __device__ __forceinline__ float nodiv_base(uint64_t n)
@@ -627,10 +647,11 @@ __device__ __forceinline__ FinishIn finish_load(const PrArgs &a, uint64_t v)
 }
 
 template<bool NODIV>
-__device__ __forceinline__ float finish_store(const PrArgs &a, uint64_t v, float sum, float base_nd, FinishIn in)
+__device__ __forceinline__ float finish_store(const PrArgs &a, uint64_t v, float sum, float base_nd, FinishIn in,
+                                              double base)
 {
     if constexpr (!NODIV) {
-        const float nr = consolidate_div(sum, a.base_div);
+        const float nr = consolidate_div(sum, base);
         a.pr_out[v] = nr;
         a.contrib_out[in.at] = in.dg ? __fdiv_rn(nr, static_cast<float>(in.dg)) : 0.0f;
         return fabsf(nr - in.prev);
@@ -644,10 +665,23 @@ __device__ __forceinline__ float finish_store(const PrArgs &a, uint64_t v, float
     }
 }
 
+// finish_store of a row of packed graphs (MULTI) or of the run's one graph;
+// g: the row's graph.
+template<bool NODIV, bool MULTI>
+__device__ __forceinline__ float finish_row(const PrArgs &a, uint64_t v, float sum, float base_nd, FinishIn in, uint32_t g)
+{
+    if constexpr (MULTI) {
+        if (g == NO_GRAPH) return 0.0f;
+        return finish_store<NODIV>(a, v, sum, base_nd, in, a.gbase[g]);
+    } else {
+        return finish_store<NODIV>(a, v, sum, base_nd, in, a.base_div);
+    }
+}
+
 template<bool NODIV>
 __device__ __forceinline__ float finish_vertex(const PrArgs &a, uint64_t v, float sum, float base_nd)
 {
-    return finish_store<NODIV>(a, v, sum, base_nd, finish_load<NODIV>(a, v));
+    return finish_store<NODIV>(a, v, sum, base_nd, finish_load<NODIV>(a, v), a.base_div);
 }
 
 // ----------------------------- pull variants ------------------------------
@@ -895,6 +929,7 @@ constexpr int pull_min_blocks(int block) { return block == PULL_WIDE ? 1 : 4; }
 // grows to 228 KB and the 28 KB left to L1 cannot hold the gathers in flight.
 constexpr uint32_t PULL_WIDE_HUBS = 24288, PULL_NARROW_HUBS = 0;
 constexpr int GATHER_UNROLL = 16;   // 512 edges = one unrolled round
+constexpr uint32_t PACKED_CHUNK = 256;   // items a block takes at a time from packed graphs' list, at most
 
 // Work-list construction.
 //  * Rows are partitioned, stably, into the rows with in-edges and the rows
@@ -1024,10 +1059,12 @@ struct LongRowDigit {
 struct LongRowPut {
     const uint32_t *len_in, *row_in;
     uint32_t *len_out, *row_out;
+    uint32_t *pos_of;              // where row i of the input went (nullptr: not kept)
     __device__ __forceinline__ void put(uint32_t pos, uint64_t i) const
     {
         len_out[pos] = len_in[i];
         row_out[pos] = row_in[i];
+        if (pos_of) pos_of[i] = pos;
     }
 };
 
@@ -1055,6 +1092,23 @@ __global__ void k_piece_emit(const uint32_t *__restrict__ off, const uint32_t *_
         long_count[r] = 0;
         for (; p < off[r + 1]; p += SEG_EDGES)
             work[out++] = make_uint4(r, (r + 1) | LONG_FLAG, p, min(p + SEG_EDGES, off[r + 1]));
+    }
+}
+
+// Packed graphs: the pieces again, in row order (so that a block's items are
+// one graph's), each with its place among the sorted ones; npos: the first
+// piece of long row i in row order, pos_of and ppos: its sorted place.
+__global__ void k_piece_emit_rows(const uint32_t *__restrict__ off, const uint32_t *__restrict__ long_row,
+                                  const uint32_t *__restrict__ long_total, const uint32_t *__restrict__ pos_of,
+                                  const uint32_t *__restrict__ ppos, const uint32_t *__restrict__ npos,
+                                  uint4 *__restrict__ work)
+{
+    const uint64_t L = *long_total;
+    for (uint64_t i = gtid(); i < L; i += gthreads()) {
+        const uint32_t r = long_row[i], e = off[r + 1];
+        uint32_t out = npos[i], sorted = ppos[pos_of[i]];
+        for (uint32_t p = off[r]; p < e; p += SEG_EDGES)
+            work[out++] = make_uint4(sorted++, LONG_FLAG, p, min(p + SEG_EDGES, e));
     }
 }
 
@@ -1276,8 +1330,10 @@ __device__ __noinline__ float batch_sequential_sum(const float *vals, uint32_t b
 
 // One gathered value: from the shared-memory hub cache when the source is
 // among the first `hubs` entries, else from global memory.
+template<bool L1 = false>
 __device__ __forceinline__ float gather1(const float *__restrict__ src, const float *hub, uint32_t hubs, uint32_t i)
 {
+    if constexpr (L1) return __ldg(src + i);          // packed graphs
     // L2 only: random lines would only evict one another from L1 (measured
     // on GB300: ER(4M, 67M) 278 -> 268 us per iteration; reading the next
     // tier of hubs through L1 instead gained nothing on R-MAT-22)
@@ -1296,7 +1352,7 @@ __device__ __forceinline__ float gather_first(const uint2 *__restrict__ pk, uint
 
 // Gather src[rev_e[e0 + k]] for k in [0, len) (len <= SEG_EDGES) into buf
 // (FIRST with pk: the first iteration's values and translation).
-template<bool FIRST>
+template<bool FIRST, bool L1>
 __device__ __forceinline__ void gather_into(const uint32_t *__restrict__ rev_e, const float *__restrict__ src,
                                             const float *hub, uint32_t hubs,
                                             uint32_t e0, uint32_t len, float *buf, unsigned lane,
@@ -1314,7 +1370,7 @@ __device__ __forceinline__ void gather_into(const uint32_t *__restrict__ rev_e, 
         for (int u = 0; u < GATHER_UNROLL; u++) {
             const uint32_t k = base + u * 32 + lane;
             if (FIRST && pk) v[u] = k < len ? gather_first(pk, gat_out, idx[u], e0 + k) : 0.0f;
-            else v[u] = k < len ? gather1(src, hub, hubs, idx[u]) : 0.0f;
+            else v[u] = k < len ? gather1<L1>(src, hub, hubs, idx[u]) : 0.0f;
         }
 #pragma unroll
         for (int u = 0; u < GATHER_UNROLL; u++) {
@@ -1644,7 +1700,8 @@ __device__ __forceinline__ float combine_pieces(const PrArgs &a, const float *rv
 
 // FIRST: the div variants' first iteration, which also translates the
 // sources when the hub-first order was taken (first_pk; no hub cache then).
-template<bool NODIV, int BLOCK, bool FIRST = false>
+// MULTI: the rows are those of packed graphs.
+template<bool NODIV, int BLOCK, bool FIRST = false, bool MULTI = false>
 __global__ void __launch_bounds__(BLOCK, pull_min_blocks(BLOCK)) k_pr_pull_items(PrArgs a)
 {
     constexpr int PULL_WARPS = BLOCK / 32;
@@ -1665,11 +1722,30 @@ __global__ void __launch_bounds__(BLOCK, pull_min_blocks(BLOCK)) k_pr_pull_items
         reinterpret_cast<float4 *>(hub)[i] = __ldg(reinterpret_cast<const float4 *>(src) + i);
     __syncthreads();
     float dsum = 0.0f;
+    // Packed graphs: a block takes a chunk of items in list order at a time (at
+    // least four chunks per block in all), so that it gathers from one graph's few hundred KB, most of them in L1;
+    // otherwise every warp strides over the whole list.
+    __shared__ uint32_t s_chunk;
+    uint64_t it = warp, step = warps, end = a.work_count;
+    const uint32_t chunk = max(static_cast<uint32_t>(PULL_WARPS),
+                               min(PACKED_CHUNK, a.work_count / (4 * gridDim.x) / PULL_WARPS * PULL_WARPS));
+    auto next_chunk = [&]() {
+        __syncthreads();
+        if (threadIdx.x == 0) s_chunk = atomicAdd(a.sum_ctr + 2, 1u);
+        __syncthreads();
+        const uint64_t from = uint64_t(s_chunk) * chunk;
+        end = min(uint64_t(a.work_count), from + chunk);
+        it = from + wib;
+        return from < a.work_count;
+    };
+    if constexpr (MULTI) step = PULL_WARPS;
+    bool more = true;
+    if constexpr (MULTI) more = next_chunk();
+    for (; more; more = MULTI && next_chunk())
     // the next item's descriptor is loaded one item ahead
-    uint4 w_next = warp < a.work_count ? a.work[warp] : make_uint4(0, 0, 0, 0);
-    for (uint64_t it = warp; it < a.work_count; it += warps) {
+    for (uint4 w_next = it < end ? a.work[it] : make_uint4(0, 0, 0, 0); it < end; it += step) {
         const uint4 w = w_next;
-        if (it + warps < a.work_count) w_next = a.work[it + warps];
+        if (it + step < end) w_next = a.work[it + step];
         const uint32_t r0 = w.x, r1 = w.y & ROW_MASK, e0 = w.z, e1 = w.w;
         if (w.y & LONG_FLAG) {
             // exact piece: store the gathered terms in edge order (the
@@ -1690,14 +1766,14 @@ __global__ void __launch_bounds__(BLOCK, pull_min_blocks(BLOCK)) k_pr_pull_items
                     const uint32_t k = base + u * 32 + lane;
                     if (k < len) {
                         const float v = (FIRST && pk) ? gather_first(pk, gat_out, idx[u], e0 + k)
-                                                      : gather1(src, hub, hubs, idx[u]);
+                                                      : gather1<MULTI>(src, hub, hubs, idx[u]);
                         __stcg(a.vals + e0 + k, v);
                         part += v;
                     }
                 }
             }
             for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(FULL_MASK, part, o);
-            if (lane == 0) a.piece_sum[it] = part;   // pieces lead the list: item = piece
+            if (lane == 0) a.piece_sum[MULTI ? w.x : it] = part;   // pieces lead the list: item = piece
             continue;
         }
         // up to 32 rows rows[r0 + l]: lane l owns one; its row end and
@@ -1705,22 +1781,24 @@ __global__ void __launch_bounds__(BLOCK, pull_min_blocks(BLOCK)) k_pr_pull_items
         const uint32_t rows = r1 - r0, len = e1 - e0;
         uint32_t row = 0;
         FinishIn fin{0.0f, 0u, 0u};
+        uint32_t graph = 0;
         if (lane < rows) {
             row = a.rows[r0 + lane];
             fin = finish_load<NODIV>(a, row);
+            if constexpr (MULTI) graph = graph_of(a, row);
         }
         if (w.y & CONST_FLAG) {                            // no in-edges: the sum is +0
-            if (lane < rows) dsum += finish_store<NODIV>(a, row, 0.0f, base_nd, fin);
+            if (lane < rows) dsum += finish_row<NODIV, MULTI>(a, row, 0.0f, base_nd, fin, graph);
             continue;
         }
         if (lane < rows) s_end[lane] = a.rev_v[row + 1] - e0;
-        gather_into<FIRST>(ge, src, hub, hubs, e0, len, buf, lane, pk, gat_out);
+        gather_into<FIRST, MULTI>(ge, src, hub, hubs, e0, len, buf, lane, pk, gat_out);
         __syncwarp();
         if (lane < rows) {
             const uint32_t b = lane ? s_end[lane - 1] : 0u, e = s_end[lane];
             float sum = 0.0f;
             for (uint32_t i = b; i < e; i++) sum = __fadd_rn(sum, buf[i]);
-            dsum += finish_store<NODIV>(a, row, sum, base_nd, fin);
+            dsum += finish_row<NODIV, MULTI>(a, row, sum, base_nd, fin, graph);
         }
         __syncwarp();
     }
@@ -1755,7 +1833,7 @@ constexpr int LONG_SUM_THREADS = 256;
 constexpr int LONG_SUM_BLOCKS_PER_SM = 2;            // registers <= 128
 constexpr uint32_t LONG_SUM_WARP_SMEM = BATCH_RING > 33 * PIECE_L ? BATCH_RING : 33 * PIECE_L;   // floats
 constexpr size_t LONG_SUM_SMEM = (LONG_SUM_THREADS / 32) * LONG_SUM_WARP_SMEM * sizeof(float);
-template<bool NODIV>
+template<bool NODIV, bool MULTI = false>
 __global__ void __launch_bounds__(LONG_SUM_THREADS, LONG_SUM_BLOCKS_PER_SM) k_pr_long_sums(PrArgs a, uint32_t *ctr)
 {
     extern __shared__ __align__(16) float long_smem[];   // per warp: the batch ring or a piece's stage
@@ -1784,7 +1862,7 @@ __global__ void __launch_bounds__(LONG_SUM_THREADS, LONG_SUM_BLOCKS_PER_SM) k_pr
                 len = a.rev_v[row + 1] - beg;
             }
             const float sum = batch_sequential_sum(a.vals, beg, len, ring, lane);
-            if (k < L) dsum += finish_store<NODIV>(a, row, sum, base_nd, fin);
+            if (k < L) dsum += finish_row<NODIV, MULTI>(a, row, sum, base_nd, fin, MULTI ? graph_of(a, row) : 0u);
         } else {
             job -= MB;
             const uint4 w = a.work[job];
@@ -1807,7 +1885,8 @@ __global__ void __launch_bounds__(LONG_SUM_THREADS, LONG_SUM_BLOCKS_PER_SM) k_pr
                 __syncwarp();                         // orders every lane's reads after lane 0's acquire
                 const float total = combine_pieces(a, rv, n, p0, pieces, stage_w, lane);
                 if (lane == 0) {
-                    dsum += finish_vertex<NODIV>(a, row, total, base_nd);
+                    dsum += finish_row<NODIV, MULTI>(a, row, total, base_nd, finish_load<NODIV>(a, row),
+                                                     MULTI ? graph_of(a, row) : 0u);
                     a.long_count[row] = 0;
                 }
             }
@@ -1820,7 +1899,27 @@ __global__ void __launch_bounds__(LONG_SUM_THREADS, LONG_SUM_BLOCKS_PER_SM) k_pr
         if (atomicAdd(&ctr[1], 1u) + 1 == warps) {
             ctr[0] = 0;
             ctr[1] = 0;
+            ctr[2] = 0;                               // k_pr_pull_items' chunks (packed graphs)
         }
+    }
+}
+
+// Packed graphs: each graph's base term; initial ranks 1/N_i and
+// contributions (k_pr_init's, per graph).
+__global__ void k_packed_base(const uint32_t *__restrict__ goff, uint32_t graphs, double *__restrict__ gbase)
+{
+    for (uint32_t i = static_cast<uint32_t>(gtid()); i < graphs; i += static_cast<uint32_t>(gthreads()))
+        gbase[i] = (1.0 - static_cast<double>(DAMPING)) / static_cast<double>(goff[i + 1] - goff[i]);
+}
+
+__global__ void k_packed_init(PrArgs a, float *__restrict__ pr, float *__restrict__ contrib)
+{
+    for (uint64_t v = gtid(); v < a.n; v += gthreads()) {
+        const uint32_t g = graph_of(a, v), d = a.deg[v];
+        if (g == NO_GRAPH) continue;
+        const float init = __fdiv_rn(1.0f, static_cast<float>(a.goff[g + 1] - a.goff[g]));
+        pr[v] = init;
+        contrib[v] = d ? __fdiv_rn(init, static_cast<float>(d)) : 0.0f;
     }
 }
 
@@ -1855,6 +1954,7 @@ int check_reps(const bw_graph_view *g, int reps)
 // Per-run state of one PageRank execution.
 struct PrRun {
     uint4 *work = nullptr;
+    uint4 *sorted = nullptr;           // packed graphs: the pieces by decreasing row length (work has them in row order)
     uint32_t *long_count = nullptr;    // arrival counters per long row
     uint32_t *scratch = nullptr;       // every other per-run array (one allocation)
     float *vals = nullptr;             // exact long rows: gathered terms (edge-indexed)
@@ -1956,7 +2056,8 @@ int launch_degrees(bw_context *ctx, const bw_graph_view *g, int variant, uint32_
     return BW_OK;
 }
 
-int build_segments(bw_context *ctx, const bw_graph_view *g, uint32_t seg_long, PrRun &run, cudaStream_t s)
+int build_segments(bw_context *ctx, const bw_graph_view *g, uint32_t seg_long, PrRun &run, cudaStream_t s,
+                   bool packed = false)
 {
     const uint64_t n = g->vertex_count, m = g->edge_count;
     if (n > ROW_MASK) return BW_ERR_TOO_LARGE;
@@ -1981,6 +2082,8 @@ int build_segments(bw_context *ctx, const bw_graph_view *g, uint32_t seg_long, P
     const uint64_t o_tot = at; at += al(12);   // lengths, giant rows, long-sum counters (tot + 8)
     const uint64_t o_sort = at; at += al(sortk::digit_sort_words<LONG_SORT_BINS>(LONG_SORT_GRID));
     const uint64_t o_part = at; at += al(std::max(sortk::scan_parts(lcap + 1), sortk::scan_parts(2 * windows + 1)));
+    const uint64_t o_of = at; at += al(packed ? lcap : 0);
+    const uint64_t o_npos = at; at += al(packed ? lcap + 1 : 0);
     BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&run.scratch), at * sizeof(uint32_t), s));
     BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&run.work), cap * sizeof(uint4), s));
     BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&run.long_count), n * sizeof(uint32_t), s));
@@ -2004,16 +2107,26 @@ int build_segments(bw_context *ctx, const bw_graph_view *g, uint32_t seg_long, P
         g->rev_vertices, n, seg_long, part_e, part_l, tiles, run.rows, S + o_lkey0, S + o_lid0);
     // 2. long rows by decreasing length (long_row_key), their pieces in that order
     BW_CUDA((sortk::digit_sort<LONG_SORT_BINS, LONG_SORT_WARPS>(
-        LongRowDigit{S + o_lkey0}, LongRowPut{S + o_lkey0, S + o_lid0, S + o_lkey1, S + o_lid1}, lcap,
+        LongRowDigit{S + o_lkey0},
+        LongRowPut{S + o_lkey0, S + o_lid0, S + o_lkey1, S + o_lid1, packed ? S + o_of : nullptr}, lcap,
         run.long_total, LONG_SORT_GRID, S + o_sort, s)));
     const uint32_t *long_len = S + o_lkey1;
     run.long_rows = S + o_lid1;
     k_piece_count<<<grid, 256, 0, s>>>(long_len, run.long_total, lcap, pcnt);
     BW_CUDA(cudaMemsetAsync(pcnt + lcap, 0, sizeof(uint32_t), s));
     BW_CUDA(sortk::scan_exclusive(pcnt, ppos, lcap + 1, part, s));
+    if (packed) BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&run.sorted),
+                                         (m / SEG_EDGES + lcap + 1) * sizeof(uint4), s));
     k_piece_emit<<<grid, 256, 0, s>>>(g->rev_vertices, run.long_rows, long_len, run.long_total, ppos,
-                                      run.work, run.long_count, run.giant_total, run.giant_pieces);
-    BW_CUDA(cudaMemsetAsync(run.sum_ctr, 0, 2 * sizeof(uint32_t), s));
+                                      packed ? run.sorted : run.work, run.long_count, run.giant_total, run.giant_pieces);
+    if (packed) {
+        k_piece_count<<<grid, 256, 0, s>>>(S + o_lkey0, run.long_total, lcap, pcnt);
+        BW_CUDA(sortk::scan_exclusive(pcnt, S + o_npos, lcap + 1, part, s));
+        k_piece_emit_rows<<<grid, 256, 0, s>>>(g->rev_vertices, S + o_lid0, run.long_total, S + o_of, ppos, S + o_npos,
+                                               run.work);
+        ctx->launches += 5;
+    }
+    BW_CUDA(cudaMemsetAsync(run.sum_ctr, 0, 4 * sizeof(uint32_t), s));
     // 3. short and CONST items after the pieces: a warp per 32 windows of
     //    32 rows
     const uint64_t seg_warps = (windows + 31) / 32;
@@ -2042,6 +2155,7 @@ int build_segments(bw_context *ctx, const bw_graph_view *g, uint32_t seg_long, P
 void free_run(PrRun &run, cudaStream_t s)
 {
     if (run.work) cudaFreeAsync(run.work, s);
+    if (run.sorted) cudaFreeAsync(run.sorted, s);
     if (run.long_count) cudaFreeAsync(run.long_count, s);
     if (run.scratch) cudaFreeAsync(run.scratch, s);
     if (run.vals) cudaFreeAsync(run.vals, s);
@@ -2588,6 +2702,71 @@ int bw_pagerank_run(bw_context *ctx, const bw_graph_view *g, int variant,
 }
 
 }  // extern "C"
+
+// PageRank of many packed graphs (bw_batch_run) as one set of rows: the
+// work-list kernels over the concatenated reverse CSR, every row with the
+// base term of its graph, so each graph's ranks are those of a vertex-pull
+// run on it alone, bit for bit.  A CTA per graph leaves the GPU to the
+// largest graphs at the end; one row set is shared evenly.  On 343M edges of
+// R-MAT graphs (GB300) an iteration takes 1.4 ms, 4.1 ps per edge, bound by
+// the latency of the gathers and of the shared-memory sums behind them (L1TEX
+// 72%, issue 46%); with every warp striding over the whole list and L2-only
+// gathers it took 2.06 ms.  Asynchronous on `s`; the scratch goes back to the
+// context's pool in stream order.
+int bw::pagerank_run_packed(bw_context *ctx, const bw_graph_view *g, const uint32_t *goff, uint32_t graphs,
+                            uint32_t iterations, float *ranks, cudaStream_t s)
+{
+    const uint64_t n = g->vertex_count;
+    BW_TRY(ensure_pr_scratch(ctx, n, 1));
+    PrRun run;
+    const int rc = build_segments(ctx, g, SEG_LONG, run, s, true);
+    if (rc != BW_OK) {
+        free_run(run, s);
+        return rc;
+    }
+    double *gbase = nullptr;
+    const cudaError_t e = ctx_malloc_async(ctx, reinterpret_cast<void **>(&gbase), graphs * sizeof(double), s);
+    if (e != cudaSuccess) free_run(run, s);
+    BW_CUDA(e);
+    PrArgs a{};
+    a.rev_v = g->rev_vertices; a.rev_e = g->rev_edges;
+    a.n = n; a.m = g->edge_count;
+    a.deg = ctx->pr_deg;
+    a.gat_e = g->rev_edges;
+    a.goff = goff; a.gbase = gbase; a.graphs = graphs;
+    a.work = run.work; a.long_count = run.long_count; a.vals = run.vals; a.rows = run.rows;
+    a.long_rows = run.long_rows; a.long_total = run.long_total; a.giant_total = run.giant_total;
+    a.giant_pieces = run.giant_pieces; a.piece_sum = run.piece_sum; a.piece_map = run.piece_map;
+    a.sum_ctr = run.sum_ctr;
+    a.pr_out = ranks;
+    a.diff = ctx->pr_diffs;
+    constexpr size_t smem = pull_fixed_smem(PULL_WIDE);
+    auto body = [&]() -> int {
+        BW_CUDA(cudaFuncSetAttribute(k_pr_long_sums<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(LONG_SUM_SMEM)));
+        BW_CUDA(cudaFuncSetAttribute(k_pr_pull_items<false, PULL_WIDE, false, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        k_row_lengths<<<ctx->sm_count * 4, 256, 0, s>>>(g->fwd_vertices, n, ctx->pr_deg);
+        k_packed_base<<<std::min<uint32_t>((graphs + 255) / 256, 256), 256, 0, s>>>(goff, graphs, gbase);
+        k_packed_init<<<ctx->sm_count * 8, 256, 0, s>>>(a, ranks, ctx->pr_buf[0]);
+        for (uint32_t j = 1; j <= iterations; j++) {
+            a.contrib_in = ctx->pr_buf[(j - 1) & 1];
+            a.contrib_out = ctx->pr_buf[j & 1];
+            // rows without in-edges keep rank and contribution from the second iteration on
+            a.count_dev = j > 2 ? run.count_nonconst : run.count_all;
+            k_pr_pull_items<false, PULL_WIDE, false, true><<<ctx->sm_count, PULL_WIDE, smem, s>>>(a);
+            PrArgs b = a;
+            b.work = run.sorted;
+            k_pr_long_sums<false, true><<<ctx->sm_count * LONG_SUM_BLOCKS_PER_SM, LONG_SUM_THREADS, LONG_SUM_SMEM, s>>>(b, b.sum_ctr);
+        }
+        BW_CUDA(cudaGetLastError());
+        return BW_OK;
+    };
+    const int done = body();
+    cudaFreeAsync(gbase, s);
+    free_run(run, s);
+    return done;
+}
 
 // A schedule run in either loop mode, with the per-iteration diffs (the
 // learned PageRank run's entry).
