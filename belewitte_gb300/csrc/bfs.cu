@@ -86,6 +86,7 @@ __global__ void k_bfs_init_side(int32_t *levels, uint64_t n, uint32_t root, uint
         ctl->traversed = 0;
         ctl->max_levels = max_levels;
         ctl->skip = 0;
+        ctl->edges = 0;
         if (outdeg) {
             const uint32_t d = outdeg[root];
             const float l = __log2f(1.0f + static_cast<float>(d));
@@ -100,13 +101,21 @@ __global__ void k_bfs_init_side(int32_t *levels, uint64_t n, uint32_t root, uint
 
 namespace {
 
-// Device-loop step: runs after every level inside the conditional body.
-// Logs the level, advances the depth and ends the loop when the level
-// visited nothing or the level cap is reached (status = LEVEL_LIMIT).
-__global__ void k_bfs_step(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap,
-                           cudaGraphConditionalHandle loop)
+// The host loop's read of a level's counts (getFrontier(), bfs/bfs.cu:13-18),
+// and of the totals: written to the host, then the number it waits for.
+__global__ void k_bfs_post(const BfsCtl *ctl, int slot, BfsMail *mail, uint32_t seq)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    mail->slot = ctl->slot[slot];
+    mail->edges = ctl->edges;
+    __threadfence_system();
+    *reinterpret_cast<volatile uint32_t *>(&mail->seq) = seq;
+}
+
+// Device-loop step, after every level: logs the level, advances the depth;
+// true when the level visited nothing or the level cap is reached (status =
+// LEVEL_LIMIT).
+__device__ __forceinline__ bool step_level(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap)
+{
     const int32_t L = ctl->depth;
     const LevelSlot s = ctl->slot[L % 3];
     if (log && static_cast<uint32_t>(L) < log_cap) log[L] = s;
@@ -120,7 +129,27 @@ __global__ void k_bfs_step(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap,
         ctl->status = BW_ERR_LEVEL_LIMIT;
         stop = true;
     }
-    if (stop) cudaGraphSetConditional(loop, 0);
+    return stop;
+}
+
+// In the graph's conditional body: ends the loop.
+__global__ void k_bfs_step(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap,
+                           cudaGraphConditionalHandle loop)
+{
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (step_level(ctl, log, log_cap)) cudaGraphSetConditional(loop, 0);
+}
+
+// Launched by the host, which waits for it.
+__global__ void k_bfs_step_post(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap, BfsMail *mail, uint32_t seq)
+{
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    mail->stop = step_level(ctl, log, log_cap) ? 1u : 0u;
+    mail->status = ctl->status;
+    mail->levels_done = ctl->levels_done;
+    mail->visited = ctl->visited;
+    __threadfence_system();
+    *reinterpret_cast<volatile uint32_t *>(&mail->seq) = seq;
 }
 
 // Sum of out-degrees of reached vertices (TEPS numerator).
@@ -140,12 +169,13 @@ struct Launch {
     BfsKernelFn k2;    // hub kernel after frontier-push
     unsigned block, grid;
     size_t smem;
+    unsigned grid2;    // of the hub kernel
 };
 
-int plan_launch(const bw_context *ctx, int variant, bool side, const bw_launch_config *cfg,
+int plan_launch(const bw_context *ctx, const bw_graph_view *g, int variant, bool side, const bw_launch_config *cfg,
                 Launch *out)
 {
-    Launch l{nullptr, nullptr, 256, static_cast<unsigned>(ctx->sm_count) * 8, 0};
+    Launch l{nullptr, nullptr, 256, static_cast<unsigned>(ctx->sm_count) * 8, 0, 0};
     const uint32_t W = (cfg && cfg->warp_size) ? cfg->warp_size : 32;
     const uint32_t C = (cfg && cfg->chunk_size) ? cfg->chunk_size : 32;
     if (variant >= 0 && variant < 16) {
@@ -184,6 +214,19 @@ int plan_launch(const bw_context *ctx, int variant, bool side, const bw_launch_c
         l.smem = (l.block / W) * (C * 4 + (C + 1) * 4);
         if (l.smem > ctx->max_smem_per_block) return BW_ERR_INVALID_ARGUMENT;
     }
+    // A graph smaller than the grid gets the blocks that have work: starting
+    // and retiring 1216 idle blocks is most of a small level.
+    l.grid2 = hub_grid(l.grid, l.block);
+    const uint64_t n = g->vertex_count, m = g->edge_count;
+    auto blocks = [](uint64_t items, uint64_t per_block) { return std::max<uint64_t>(1, (items + per_block - 1) / per_block); };
+    uint64_t need;
+    if (variant < 16) need = blocks(m, 4 * uint64_t(l.block));                        // 4 edges a thread
+    else if (variant < 20) need = blocks(n, 4 * uint64_t(l.block));                   // vertex-push: 4 depths a thread
+    else if (variant >= 24 && variant < 32) need = blocks(n, uint64_t(C) * (l.block / W));
+    else need = blocks(n, l.block);
+    l.grid = static_cast<unsigned>(std::min<uint64_t>(l.grid, need));
+    // at most this many hub chunks in a level (ensure_bfs_scratch), one per warp
+    l.grid2 = static_cast<unsigned>(std::min<uint64_t>(l.grid2, blocks(2 * m / 256 + n / 256, 8)));
     *out = l;
     return BW_OK;
 }
@@ -212,8 +255,8 @@ BfsArgs make_args(bw_context *ctx, const bw_graph_view *g, int32_t *levels, int3
 int launch(const Launch &l, const BfsArgs &a, cudaStream_t s)
 {
     l.k<<<l.grid, l.block, l.smem, s>>>(a);
-    // the hub-chunk kernel is built for 256-thread blocks: the same threads
-    if (l.k2) l.k2<<<hub_grid(l.grid, l.block), 256, 0, s>>>(a);
+    // the hub-chunk kernel is built for 256-thread blocks
+    if (l.k2) l.k2<<<l.grid2, 256, 0, s>>>(a);
     BW_CUDA(cudaGetLastError());
     return BW_OK;
 }
@@ -240,20 +283,26 @@ void fill_stats(const LevelSlot &s, int variant, bw_bfs_level_stats *out)
     out->device_ms = 0.0f;
 }
 
+// Posts level slot `slot` (and the edge total) and waits for it.
+int post_and_wait(bw_context *ctx, int slot, cudaStream_t s)
+{
+    const uint32_t seq = ++ctx->mail_seq;
+    k_bfs_post<<<1, 1, 0, s>>>(ctx->bfs_ctl, slot, ctx->mail, seq);
+    BW_CUDA(cudaGetLastError());
+    return bfs_wait(ctx, seq, s);
+}
+
+// ctl->edges is zero since the run's initialisation.
 int traversed_edges(bw_context *ctx, const bw_graph_view *g, int32_t *levels, cudaStream_t s,
                     uint64_t *out)
 {
     *out = 0;
     if (!g->fwd_vertices) return BW_OK;
-    unsigned long long *d = nullptr;
-    BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&d), sizeof *d, s));
-    BW_CUDA(cudaMemsetAsync(d, 0, sizeof *d, s));
-    k_traversed<<<ctx->sm_count * 4, 256, 0, s>>>(levels, g->fwd_vertices, g->vertex_count, d);
-    unsigned long long h = 0;
-    BW_CUDA(cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, s));
-    BW_CUDA(cudaFreeAsync(d, s));
-    BW_CUDA(cudaStreamSynchronize(s));
-    *out = h;
+    const uint64_t n = g->vertex_count;
+    const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, uint64_t(ctx->sm_count) * 4));
+    k_traversed<<<grid, 256, 0, s>>>(levels, g->fwd_vertices, n, &ctx->bfs_ctl->edges);
+    BW_TRY(post_and_wait(ctx, 0, s));
+    *out = ctx->mail->edges;
     return BW_OK;
 }
 
@@ -271,7 +320,7 @@ int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, u
         const int v = schedule[i];
         if (v < 0 || v >= VARIANT_COUNT) return BW_ERR_UNKNOWN_VARIANT;
         if (!planned[v]) {
-            BW_TRY(plan_launch(ctx, v, side, cfg, &plans[v]));
+            BW_TRY(plan_launch(ctx, g, v, side, cfg, &plans[v]));
             planned[v] = true;
         }
     }
@@ -291,13 +340,11 @@ int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, u
         if (time_levels) BW_CUDA(cudaEventRecord(ctx->level_events[0], s));
         BW_TRY(launch(plans[v], a, s));
         if (time_levels) BW_CUDA(cudaEventRecord(ctx->level_events[1], s));
-        // getFrontier() (bfs/bfs.cu:13-18): read this level's slot back.
-        BW_CUDA(cudaMemcpyAsync(&ctx->bfs_ctl_host->slot[level % 3], &ctx->bfs_ctl->slot[level % 3],
-                                sizeof(LevelSlot), cudaMemcpyDeviceToHost, s));
-        BW_CUDA(cudaStreamSynchronize(s));
-        const LevelSlot sl = ctx->bfs_ctl_host->slot[level % 3];
+        BW_TRY(post_and_wait(ctx, static_cast<int>(level % 3), s));
+        const LevelSlot sl = ctx->mail->slot;
         if (stats && level < stats_cap) {
             fill_stats(sl, v, &stats[level]);
+            if (time_levels) BW_CUDA(cudaEventSynchronize(ctx->level_events[1]));
             if (time_levels)
                 BW_CUDA(cudaEventElapsedTime(&stats[level].device_ms, ctx->level_events[0], ctx->level_events[1]));
         }
@@ -306,20 +353,27 @@ int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, u
         if (sl.frontier == 0) break;
     }
     BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
-    BW_CUDA(cudaEventSynchronize(ctx->ev_stop));
-    BW_CUDA(cudaEventElapsedTime(&total_ms, ctx->ev_start, ctx->ev_stop));
     if (result) {
+        BW_TRY(traversed_edges(ctx, g, levels, s, &result->traversed_edges));
+        BW_CUDA(cudaEventSynchronize(ctx->ev_stop));
+        BW_CUDA(cudaEventElapsedTime(&total_ms, ctx->ev_start, ctx->ev_stop));
         result->level_count = level;
         result->visited = visited;
         result->device_ms = total_ms;
-        BW_TRY(traversed_edges(ctx, g, levels, s, &result->traversed_edges));
     }
     return status;
 }
 
-// Device-loop traversal: one CUDA graph whose conditional WHILE node runs
-// [level kernel(s) -> step kernel] until the step kernel clears the loop
-// condition.  No host round trip per level.
+// Device-loop traversal.  The level's kernels read the depth and their queue's
+// length on the device, and a step kernel keeps the totals.  The first
+// DEVICE_LOOP_LAUNCHED rounds are launched by the host, which only waits for
+// the step's verdict: most traversals end there, and building a CUDA graph
+// (0.25 ms) would cost them more than all their launches.  A traversal that
+// goes on continues in a graph whose conditional WHILE node runs the same
+// kernels until the step kernel clears the loop condition, with no host round
+// trip per level.
+constexpr uint32_t DEVICE_LOOP_LAUNCHED = 48;
+
 int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t root,
               int32_t *levels, const bw_launch_config *cfg, uint32_t max_levels, bool side,
               bw_bfs_result *result, bw_bfs_level_stats *stats, uint32_t stats_cap,
@@ -328,7 +382,7 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
     const uint64_t n = g->vertex_count;
     if (max_levels == 0) max_levels = static_cast<uint32_t>(std::min<uint64_t>(n + 1, 0xffffffffULL));
     Launch plan;
-    BW_TRY(plan_launch(ctx, variant, side, cfg, &plan));
+    BW_TRY(plan_launch(ctx, g, variant, side, cfg, &plan));
     const bool cluster_path = variant == V_FRONTIER_PUSH;
     if (cluster_path) {
         BW_TRY(ensure_outdeg(ctx, g, s));   // frontier edge volumes gate the cluster path
@@ -337,85 +391,94 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
     LevelSlot *log = nullptr;
     const uint32_t log_cap = stats ? std::min(stats_cap, max_levels) : 0;
     if (log_cap) BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&log), log_cap * sizeof(LevelSlot), s));
-
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    int rc = BW_OK;
-    auto fail = [&](cudaError_t e, const char *what) {
-        set_last_error(e, what);
-        rc = e == cudaErrorMemoryAllocation ? BW_ERR_OUT_OF_MEMORY : BW_ERR_CUDA;
+    BfsArgs a = make_args(ctx, g, levels, -1, cfg);
+    if (cluster_path) {
+        // small frontiers: the cluster kernel runs many levels per launch
+        a.skip_check = 1;
+        a.log = log;
+        a.log_cap = log_cap;
+    }
+    auto level_kernels = [&](cudaStream_t to) {
+        if (cluster_path) bfs_cluster_kernel(side ? 1 : 0)<<<CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), to>>>(a);
+        plan.k<<<plan.grid, plan.block, plan.smem, to>>>(a);
+        if (plan.k2) plan.k2<<<plan.grid2, 256, 0, to>>>(a);
     };
-    do {
-        cudaError_t e = cudaGraphCreate(&graph, 0);
-        if (e != cudaSuccess) { fail(e, "cudaGraphCreate"); break; }
-        cudaGraphConditionalHandle handle;
-        e = cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault);
-        if (e != cudaSuccess) { fail(e, "cudaGraphConditionalHandleCreate"); break; }
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = handle;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t cnode;
-        e = cudaGraphAddNode(&cnode, graph, nullptr, nullptr, 0, &cp);
-        if (e != cudaSuccess) { fail(e, "cudaGraphAddNode(conditional)"); break; }
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        // Capture the body on a private stream.
-        cudaStream_t cap;
-        e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
-        if (e != cudaSuccess) { fail(e, "cudaStreamCreate"); break; }
-        // BW_LAUNCH_L2_WINDOW: the captured kernels keep the depth array persisting in L2
-        L2Window win_cap;
-        if (cfg && (cfg->flags & BW_LAUNCH_L2_WINDOW) &&
-            l2_window_begin(ctx, cap, levels, n * sizeof(int32_t), win_cap, false) != BW_OK) {
-            cudaStreamDestroy(cap);
-            rc = BW_ERR_CUDA;
-            break;
+    BfsMail end{};                          // the last round's
+    auto traverse = [&]() -> int {
+        k_bfs_init_side<<<ctx->sm_count * 4, 256, 0, s>>>(levels, n, root, ctx->queue[0], ctx->bfs_ctl, max_levels,
+                                                         (side || cluster_path) ? ctx->outdeg : nullptr);
+        BW_CUDA(cudaGetLastError());
+        BW_CUDA(cudaEventRecord(ctx->ev_start, s));
+        for (uint32_t i = 0; i < DEVICE_LOOP_LAUNCHED && !end.stop; i++) {
+            level_kernels(s);
+            const uint32_t seq = ++ctx->mail_seq;
+            k_bfs_step_post<<<1, 32, 0, s>>>(ctx->bfs_ctl, log, log_cap, ctx->mail, seq);
+            BW_CUDA(cudaGetLastError());
+            BW_TRY(bfs_wait(ctx, seq, s));
+            end = *ctx->mail;
         }
-        e = cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
-        if (e == cudaSuccess) {
-            BfsArgs a = make_args(ctx, g, levels, -1, cfg);
-            if (cluster_path) {
-                // small frontiers: the cluster kernel runs many levels per launch
-                a.skip_check = 1;
-                a.log = log;
-                a.log_cap = log_cap;
-                bfs_cluster_kernel(side ? 1 : 0)<<<CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), cap>>>(a);
-            }
-            plan.k<<<plan.grid, plan.block, plan.smem, cap>>>(a);
-            if (plan.k2) plan.k2<<<hub_grid(plan.grid, plan.block), 256, 0, cap>>>(a);
-            k_bfs_step<<<1, 32, 0, cap>>>(ctx->bfs_ctl, log, log_cap, handle);
-            cudaGraph_t captured = body;
-            e = cudaStreamEndCapture(cap, &captured);
-            if (e != cudaSuccess) fail(e, "cudaStreamEndCapture");
+        if (end.stop) {
+            BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
         } else {
-            fail(e, "cudaStreamBeginCaptureToGraph");
+            // BW_LAUNCH_L2_WINDOW: the captured kernels keep the depth array persisting in L2
+            const bool window = cfg && (cfg->flags & BW_LAUNCH_L2_WINDOW);
+            auto capture = [&](cudaStream_t cap, cudaGraph_t body, cudaGraphConditionalHandle handle) -> int {
+                L2Window win;
+                if (window) BW_TRY(l2_window_begin(ctx, cap, levels, n * sizeof(int32_t), win, false));
+                BW_CUDA(cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+                level_kernels(cap);
+                k_bfs_step<<<1, 32, 0, cap>>>(ctx->bfs_ctl, log, log_cap, handle);
+                cudaGraph_t captured = body;
+                const cudaError_t e = cudaStreamEndCapture(cap, &captured);
+                l2_window_end(win);                 // before its stream goes
+                BW_CUDA(e);
+                return BW_OK;
+            };
+            auto loop = [&](cudaGraph_t graph, cudaStream_t cap) -> int {
+                cudaGraphConditionalHandle handle;
+                BW_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
+                cudaGraphNodeParams cp = {};
+                cp.type = cudaGraphNodeTypeConditional;
+                cp.conditional.handle = handle;
+                cp.conditional.type = cudaGraphCondTypeWhile;
+                cp.conditional.size = 1;
+                cudaGraphNode_t cnode;
+                BW_CUDA(cudaGraphAddNode(&cnode, graph, nullptr, nullptr, 0, &cp));
+                BW_TRY(capture(cap, cp.conditional.phGraph_out[0], handle));
+                cudaGraphExec_t exec = nullptr;
+                BW_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+                cudaError_t e = cudaGraphLaunch(exec, s);
+                if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_stop, s);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(ctx->bfs_ctl_host, ctx->bfs_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+                cudaGraphExecDestroy(exec);
+                BW_CUDA(e);
+                end.status = ctx->bfs_ctl_host->status;
+                end.levels_done = ctx->bfs_ctl_host->levels_done;
+                end.visited = ctx->bfs_ctl_host->visited;
+                return BW_OK;
+            };
+            cudaGraph_t graph = nullptr;
+            cudaStream_t cap = nullptr;             // the caller's may be the legacy default stream
+            BW_CUDA(cudaGraphCreate(&graph, 0));
+            const cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
+            const int rc = e == cudaSuccess ? loop(graph, cap) : BW_ERR_CUDA;
+            if (cap) cudaStreamDestroy(cap);
+            cudaGraphDestroy(graph);
+            BW_CUDA(e);
+            BW_TRY(rc);
         }
-        l2_window_end(win_cap);                 // before its stream goes
-        cudaStreamDestroy(cap);
-        if (rc) break;
-        e = cudaGraphInstantiate(&exec, graph, 0);
-        if (e != cudaSuccess) { fail(e, "cudaGraphInstantiate"); break; }
-    } while (0);
-    if (rc) {
-        if (graph) cudaGraphDestroy(graph);
+        return BW_OK;
+    };
+    const int rc = traverse();
+    if (rc != BW_OK) {
         if (log) cudaFreeAsync(log, s);
         return rc;
     }
-
-    k_bfs_init_side<<<ctx->sm_count * 4, 256, 0, s>>>(levels, n, root, ctx->queue[0], ctx->bfs_ctl, max_levels,
-                                                     (side || cluster_path) ? ctx->outdeg : nullptr);
-    BW_CUDA(cudaGetLastError());
-    BW_CUDA(cudaEventRecord(ctx->ev_start, s));
-    BW_CUDA(cudaGraphLaunch(exec, s));
-    BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
-    BW_CUDA(cudaMemcpyAsync(ctx->bfs_ctl_host, ctx->bfs_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
-    BW_CUDA(cudaStreamSynchronize(s));
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
-    const BfsCtl c = *ctx->bfs_ctl_host;
     if (log_cap) {
-        const uint32_t got = std::min(c.levels_done, log_cap);
+        BW_CUDA(cudaStreamSynchronize(s));
+        const uint32_t got = std::min(end.levels_done, log_cap);
         LevelSlot *tmp = new LevelSlot[got ? got : 1];
         BW_CUDA(cudaMemcpy(tmp, log, got * sizeof(LevelSlot), cudaMemcpyDeviceToHost));
         for (uint32_t i = 0; i < got; i++) fill_stats(tmp[i], variant, &stats[i]);
@@ -423,14 +486,15 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
         BW_CUDA(cudaFreeAsync(log, s));
     }
     if (result) {
-        float ms = 0.0f;
-        BW_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
-        result->level_count = c.levels_done;
-        result->visited = c.visited;
-        result->device_ms = ms;
         BW_TRY(traversed_edges(ctx, g, levels, s, &result->traversed_edges));
+        float ms = 0.0f;
+        BW_CUDA(cudaEventSynchronize(ctx->ev_stop));
+        BW_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
+        result->level_count = end.levels_done;
+        result->visited = end.visited;
+        result->device_ms = ms;
     }
-    return c.status ? static_cast<int>(c.status) : BW_OK;
+    return end.status ? static_cast<int>(end.status) : BW_OK;
 }
 
 int prepare(bw_context *ctx, const bw_graph_view *g, int reps, bool side, int32_t *levels,
@@ -480,12 +544,12 @@ int bfs_prepare(bw_context *ctx, const bw_graph_view *g, int reps, bool side, in
                 cudaStream_t s)
 { return prepare(ctx, g, reps, side, levels, root, s); }
 
-int bfs_plan(const bw_context *ctx, int variant, bool side, const bw_launch_config *cfg, BfsKernelFn *k,
-             BfsKernelFn *k2, unsigned *block, unsigned *grid, size_t *smem)
+int bfs_plan(const bw_context *ctx, const bw_graph_view *g, int variant, bool side, const bw_launch_config *cfg,
+             BfsKernelFn *k, BfsKernelFn *k2, unsigned *block, unsigned *grid, size_t *smem, unsigned *grid2)
 {
     Launch l;
-    BW_TRY(plan_launch(ctx, variant, side, cfg, &l));
-    *k = l.k; *k2 = l.k2; *block = l.block; *grid = l.grid; *smem = l.smem;
+    BW_TRY(plan_launch(ctx, g, variant, side, cfg, &l));
+    *k = l.k; *k2 = l.k2; *block = l.block; *grid = l.grid; *smem = l.smem; *grid2 = l.grid2;
     return BW_OK;
 }
 
@@ -494,6 +558,8 @@ BfsArgs bfs_args(bw_context *ctx, const bw_graph_view *g, int32_t *levels, int32
 { return make_args(ctx, g, levels, depth, cfg); }
 
 int bfs_variant_reps(int v) { return variant_reps(v); }
+
+int bfs_read_slot(bw_context *ctx, int slot, cudaStream_t s) { return post_and_wait(ctx, slot, s); }
 
 int bfs_traversed(bw_context *ctx, const bw_graph_view *g, int32_t *levels, cudaStream_t s, uint64_t *out)
 { return traversed_edges(ctx, g, levels, s, out); }
@@ -554,7 +620,7 @@ int bw_bfs_level(bw_context *ctx, const bw_graph_view *g, int variant, int32_t *
     const bool side = g->fwd_vertices != nullptr;
     if (side) BW_TRY(ensure_outdeg(ctx, g, as_stream(stream)));
     if (!side && (variant == V_FRONTIER_PUSH)) return BW_ERR_MISSING_REPRESENTATION;
-    BW_TRY(plan_launch(ctx, variant, side, cfg, &plan));
+    BW_TRY(plan_launch(ctx, g, variant, side, cfg, &plan));
     cudaStream_t s = as_stream(stream);
     BfsArgs a = make_args(ctx, g, levels, depth, cfg);
     BW_TRY(launch(plan, a, s));

@@ -1,5 +1,6 @@
 #include <algorithm>
 // Context, scratch management, launch geometry and representation builders.
+#include <chrono>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -57,7 +58,11 @@ int ensure_bfs_scratch(bw_context *ctx, uint64_t n, uint64_t m)
     if (!ctx->bfs_ctl) {
         BW_CUDA(cudaMalloc(reinterpret_cast<void **>(&ctx->bfs_ctl), sizeof(BfsCtl)));
         BW_CUDA(cudaMemset(ctx->bfs_ctl, 0, sizeof(BfsCtl)));
-        BW_CUDA(cudaMallocHost(reinterpret_cast<void **>(&ctx->bfs_ctl_host), sizeof(BfsCtl)));
+        constexpr size_t at = (sizeof(BfsCtl) + 127) & ~size_t(127);       // the mail on lines of its own
+        BW_CUDA(cudaMallocHost(reinterpret_cast<void **>(&ctx->bfs_ctl_host), at + sizeof(BfsMail)));
+        ctx->mail = reinterpret_cast<BfsMail *>(reinterpret_cast<char *>(ctx->bfs_ctl_host) + at);
+        std::memset(ctx->mail, 0, sizeof(BfsMail));
+        ctx->mail_seq = 0;
     }
     if (n > ctx->bfs_n_cap) {
         BW_TRY(grow(&ctx->queue[0], n));
@@ -72,6 +77,21 @@ int ensure_bfs_scratch(bw_context *ctx, uint64_t n, uint64_t m)
         ctx->heavy_cap = hcap;
     }
     return BW_OK;
+}
+
+// A level of a few microseconds is worth polling for; a longer one (or a
+// kernel that failed, which the synchronisation reports) is not.
+int bfs_wait(bw_context *ctx, uint32_t seq, cudaStream_t s)
+{
+    auto posted = [&]() { return __atomic_load_n(&ctx->mail->seq, __ATOMIC_ACQUIRE) == seq; };
+    const auto start = std::chrono::steady_clock::now();
+    for (;;) {
+        for (int i = 0; i < 64; i++)
+            if (posted()) return BW_OK;
+        if (std::chrono::steady_clock::now() - start > std::chrono::milliseconds(1)) break;
+    }
+    BW_CUDA(cudaStreamSynchronize(s));
+    return posted() ? BW_OK : BW_ERR_CUDA;
 }
 
 __global__ void k_row_lengths(const uint32_t *__restrict__ off, uint64_t n,

@@ -14,8 +14,9 @@ namespace bw {
 // Implemented in bfs.cu (shared with the fixed-variant paths).
 int bfs_prepare(bw_context *ctx, const bw_graph_view *g, int reps, bool side, int32_t *levels,
                 uint32_t root, cudaStream_t s);
-int bfs_plan(const bw_context *ctx, int variant, bool side, const bw_launch_config *cfg, BfsKernelFn *k,
-             BfsKernelFn *k2, unsigned *block, unsigned *grid, size_t *smem);
+int bfs_plan(const bw_context *ctx, const bw_graph_view *g, int variant, bool side, const bw_launch_config *cfg,
+             BfsKernelFn *k, BfsKernelFn *k2, unsigned *block, unsigned *grid, size_t *smem, unsigned *grid2);
+int bfs_read_slot(bw_context *ctx, int slot, cudaStream_t s);   // the level's counts into ctx->mail->slot
 BfsArgs bfs_args(bw_context *ctx, const bw_graph_view *g, int32_t *levels, int32_t depth,
                  const bw_launch_config *cfg);
 int bfs_variant_reps(int v);
@@ -340,18 +341,19 @@ struct PredictArgs {
     int fallback;
     float threshold;
     uint64_t n, m;
-    cudaGraphConditionalHandle sw;
+    cudaGraphConditionalHandle sw;   // set when the loop runs in a graph
+    bool in_graph;
     int32_t cluster_k;          // frontier-push's candidate index for cluster-sized frontiers, or -1
 };
 
-// Runs before every level inside the device loop: features of the current
-// frontier (stats of the previous level, or the root), MLP forward, the
-// SWITCH handle for this level's variant.  One block of 128 threads: the
-// parameters are staged in shared memory, each thread computes hidden
-// units, lane 0 of warp 0 takes the softmax and the decision.
+// Before every level of the device loop: features of the current frontier
+// (stats of the previous level, or the root), MLP forward, this level's
+// variant in ctl->variant (and the graph's SWITCH handle).  One block of 128
+// threads: the parameters are staged in shared memory, each thread computes
+// hidden units, lane 0 of warp 0 takes the softmax and the decision.
 constexpr int PREDICT_THREADS = 128;
 
-__global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_predict(PredictArgs a)
+__device__ void predict_level(const PredictArgs &a)
 {
     extern __shared__ float sp[];
     __shared__ float x[F], h1[H], h2[H], z[BW_MLP_MAX_CLASSES];
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_predict(PredictArgs a)
         if (s.qlen > 0 && s.qlen <= CLUSTER_CAP && s.fedges <= CLUSTER_EDGE_CAP) {
             if (tid == 0) {
                 c->variant = a.cluster_k;
-                cudaGraphSetConditional(a.sw, static_cast<unsigned>(a.cluster_k));
+                if (a.in_graph) cudaGraphSetConditional(a.sw, static_cast<unsigned>(a.cluster_k));
             }
             return;
         }
@@ -412,13 +414,16 @@ __global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_predict(PredictArgs a)
         const float pbest = expf(z[best] - mx) / den;
         if (pbest < a.threshold) best = a.fallback;
         c->variant = best;
-        cudaGraphSetConditional(a.sw, static_cast<unsigned>(best));
+        if (a.in_graph) cudaGraphSetConditional(a.sw, static_cast<unsigned>(best));
     }
 }
 
-__global__ void k_bfs_step_learned(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap, cudaGraphConditionalHandle loop)
+__global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_predict(PredictArgs a) { predict_level(a); }
+
+// After every level: its entry in the log, the totals; true when the
+// traversal is over.
+__device__ __forceinline__ bool step_learned(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int32_t L = ctl->depth;
     LevelSlot s = ctl->slot[L % 3];
     if (log && static_cast<uint32_t>(L) < log_cap) {
@@ -435,7 +440,32 @@ __global__ void k_bfs_step_learned(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap
         ctl->status = BW_ERR_LEVEL_LIMIT;
         stop = true;
     }
-    if (stop) cudaGraphSetConditional(loop, 0);
+    return stop;
+}
+
+__global__ void k_bfs_step_learned(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap, cudaGraphConditionalHandle loop)
+{
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (step_learned(ctl, log, log_cap)) cudaGraphSetConditional(loop, 0);
+}
+
+// Both, launched by the host, which waits for the next level's variant.
+__global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_next(PredictArgs a, bool step, LevelSlot *log, uint32_t log_cap,
+                                                              BfsMail *mail, uint32_t seq)
+{
+    __shared__ bool s_stop;
+    BfsCtl *c = a.ctl;
+    if (threadIdx.x == 0) s_stop = step && step_learned(c, log, log_cap);
+    __syncthreads();
+    if (!s_stop) predict_level(a);
+    if (threadIdx.x != 0) return;
+    mail->variant = c->variant;
+    mail->stop = s_stop ? 1u : 0u;
+    mail->status = c->status;
+    mail->levels_done = c->levels_done;
+    mail->visited = c->visited;
+    __threadfence_system();
+    *reinterpret_cast<volatile uint32_t *>(&mail->seq) = seq;
 }
 
 // Undo a profiled level run: every vertex it visited is in its next-frontier
@@ -461,7 +491,7 @@ void slot_stats(const LevelSlot &sl, int variant, bw_bfs_level_stats *out)
 
 struct Plan {
     BfsKernelFn k, k2;
-    unsigned block, grid;
+    unsigned block, grid, grid2;
     size_t smem;
 };
 
@@ -723,8 +753,8 @@ int bw_bfs_profile(bw_context *ctx, const bw_graph_view *g, uint32_t root, int32
     BW_TRY(bfs_prepare(ctx, g, reps, true, levels, root, s));
     std::vector<Plan> plans(K);
     for (uint32_t k = 0; k < K; k++)
-        BW_TRY(bfs_plan(ctx, candidates[k], true, nullptr, &plans[k].k, &plans[k].k2, &plans[k].block,
-                        &plans[k].grid, &plans[k].smem));
+        BW_TRY(bfs_plan(ctx, g, candidates[k], true, nullptr, &plans[k].k, &plans[k].k2, &plans[k].block,
+                        &plans[k].grid, &plans[k].smem, &plans[k].grid2));
     if (repeats == 0) repeats = 1;
     if (sample_every == 0) sample_every = 1;
     const uint64_t n = g->vertex_count, m = g->edge_count;
@@ -744,7 +774,7 @@ int bw_bfs_profile(bw_context *ctx, const bw_graph_view *g, uint32_t root, int32
     auto run_one = [&](uint32_t k) {
         BfsArgs a = bfs_args(ctx, g, levels, static_cast<int32_t>(L), nullptr);
         plans[k].k<<<plans[k].grid, plans[k].block, plans[k].smem, s>>>(a);
-        if (plans[k].k2) plans[k].k2<<<hub_grid(plans[k].grid, plans[k].block), 256, 0, s>>>(a);
+        if (plans[k].k2) plans[k].k2<<<plans[k].grid2, 256, 0, s>>>(a);
     };
     for (; L < max_levels; L++) {
         float lmax;
@@ -815,8 +845,8 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
     BW_TRY(bfs_prepare(ctx, g, reps, true, levels, root, s));
     std::vector<Plan> plans(K);
     for (uint32_t k = 0; k < K; k++)
-        BW_TRY(bfs_plan(ctx, sw->candidates[k], true, nullptr, &plans[k].k, &plans[k].k2, &plans[k].block,
-                        &plans[k].grid, &plans[k].smem));
+        BW_TRY(bfs_plan(ctx, g, sw->candidates[k], true, nullptr, &plans[k].k, &plans[k].k2, &plans[k].block,
+                        &plans[k].grid, &plans[k].smem, &plans[k].grid2));
     const uint64_t n = g->vertex_count, m = g->edge_count;
     if (max_levels == 0) max_levels = static_cast<uint32_t>(std::min<uint64_t>(n + 1, 0xffffffffULL));
 
@@ -843,12 +873,10 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
             const int c = pick(probs, K, sw->fallback, sw->threshold);
             BfsArgs a = bfs_args(ctx, g, levels, static_cast<int32_t>(L), nullptr);
             plans[c].k<<<plans[c].grid, plans[c].block, plans[c].smem, s>>>(a);
-            if (plans[c].k2) plans[c].k2<<<hub_grid(plans[c].grid, plans[c].block), 256, 0, s>>>(a);
+            if (plans[c].k2) plans[c].k2<<<plans[c].grid2, 256, 0, s>>>(a);
             BW_CUDA(cudaGetLastError());
-            BW_CUDA(cudaMemcpyAsync(&ctx->bfs_ctl_host->slot[L % 3], &ctx->bfs_ctl->slot[L % 3], sizeof(LevelSlot),
-                                    cudaMemcpyDeviceToHost, s));
-            BW_CUDA(cudaStreamSynchronize(s));
-            cur = ctx->bfs_ctl_host->slot[L % 3];
+            BW_TRY(bfs_read_slot(ctx, static_cast<int>(L % 3), s));
+            cur = ctx->mail->slot;
             if (stats && L < stats_cap) slot_stats(cur, sw->candidates[c], &stats[L]);
             visited += cur.frontier;
             edges_visited += cur.fedges;
@@ -856,24 +884,94 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
             if (cur.frontier == 0) break;
         }
         BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
-        BW_CUDA(cudaEventSynchronize(ctx->ev_stop));
         if (result) {
+            BW_TRY(bfs_traversed(ctx, g, levels, s, &result->traversed_edges));
             float ms = 0.0f;
+            BW_CUDA(cudaEventSynchronize(ctx->ev_stop));
             BW_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
             result->level_count = L;
             result->visited = visited;
             result->device_ms = ms;
-            BW_TRY(bfs_traversed(ctx, g, levels, s, &result->traversed_edges));
         }
         return rc;
     }
     if (loop_mode != BW_LOOP_GRAPH) return BW_ERR_INVALID_ARGUMENT;
 
-    // Device loop: WHILE { predict -> SWITCH(K level bodies) -> step }.
+    // Device loop.  As in run_graph (bfs.cu), the host launches the first
+    // rounds { step, predict -> level } and waits for each round's variant;
+    // building the graph would cost a traversal of a few levels 0.35 ms.  A
+    // longer one goes on in a graph: WHILE { predict -> SWITCH(K level bodies)
+    // -> step }.
+    constexpr uint32_t ROUNDS_LAUNCHED = 48;
     BW_TRY(bfs_cluster_prepare());          // frontier-push's small-frontier kernel, if a candidate
     LevelSlot *log = nullptr;
     const uint32_t log_cap = stats ? std::min(stats_cap, max_levels) : 0;
     if (log_cap) BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&log), log_cap * sizeof(LevelSlot), s));
+    int32_t cluster_k = -1;
+    if (!(sw->flags & BW_SWITCH_MLP_ONLY))
+        for (uint32_t k = 0; k < K; k++)
+            if (sw->candidates[k] == 32) cluster_k = static_cast<int32_t>(k);   // frontier-push
+    BfsArgs a = bfs_args(ctx, g, levels, -1, nullptr);
+    a.skip_check = 1;
+    a.log = log;
+    a.log_cap = log_cap;
+    BfsMail end{};
+    auto rounds = [&]() -> int {
+        k_bfs_init_side<<<ctx->sm_count * 4, 256, 0, s>>>(levels, n, root, ctx->queue[0], ctx->bfs_ctl, max_levels,
+                                                         ctx->outdeg);
+        BW_CUDA(cudaGetLastError());
+        BW_CUDA(cudaEventRecord(ctx->ev_start, s));
+        const PredictArgs pa{ctx->bfs_ctl, sw->params, K, sw->fallback, sw->threshold, n, m, {}, false, cluster_k};
+        for (uint32_t i = 0; i < ROUNDS_LAUNCHED; i++) {
+            const uint32_t seq = ++ctx->mail_seq;
+            k_bfs_next<<<1, PREDICT_THREADS, param_count(K) * sizeof(float), s>>>(pa, i > 0, log, log_cap, ctx->mail, seq);
+            BW_CUDA(cudaGetLastError());
+            BW_TRY(bfs_wait(ctx, seq, s));
+            end = *ctx->mail;
+            if (end.stop) break;
+            const Plan &p = plans[end.variant];
+            // the level log needs every level's statistics; otherwise only a
+            // handed-over level's, which the next prediction reads
+            if (sw->candidates[end.variant] == 32)
+                bfs_cluster_kernel(log_cap ? 1 : 2)<<<CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), s>>>(a);
+            p.k<<<p.grid, p.block, p.smem, s>>>(a);
+            if (p.k2) p.k2<<<p.grid2, 256, 0, s>>>(a);
+            if (i + 1 == ROUNDS_LAUNCHED) {      // the graph's first round predicts: close this one
+                const uint32_t last = ++ctx->mail_seq;
+                k_bfs_next<<<1, PREDICT_THREADS, param_count(K) * sizeof(float), s>>>(pa, true, log, log_cap, ctx->mail, last);
+                BW_CUDA(cudaGetLastError());
+                BW_TRY(bfs_wait(ctx, last, s));
+                end = *ctx->mail;
+            }
+        }
+        if (end.stop) BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
+        return BW_OK;
+    };
+    if (const int rc = rounds(); rc != BW_OK) {
+        if (log) cudaFreeAsync(log, s);
+        return rc;
+    }
+    auto finish = [&]() -> int {
+        if (log_cap) {
+            BW_CUDA(cudaStreamSynchronize(s));
+            const uint32_t got = std::min(end.levels_done, log_cap);
+            std::vector<LevelSlot> tmp(got ? got : 1);
+            BW_CUDA(cudaMemcpy(tmp.data(), log, got * sizeof(LevelSlot), cudaMemcpyDeviceToHost));
+            for (uint32_t i = 0; i < got; i++) slot_stats(tmp[i], sw->candidates[tmp[i].heavy], &stats[i]);
+            BW_CUDA(cudaFreeAsync(log, s));
+        }
+        if (result) {
+            BW_TRY(bfs_traversed(ctx, g, levels, s, &result->traversed_edges));
+            float ms = 0.0f;
+            BW_CUDA(cudaEventSynchronize(ctx->ev_stop));
+            BW_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
+            result->level_count = end.levels_done;
+            result->visited = end.visited;
+            result->device_ms = ms;
+        }
+        return end.status ? static_cast<int>(end.status) : BW_OK;
+    };
+    if (end.stop) return finish();
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int rc = BW_OK;
@@ -901,11 +999,7 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
             fail(e, "handle(switch)"); break;
         }
         // predict kernel node
-        int32_t cluster_k = -1;
-        if (!(sw->flags & BW_SWITCH_MLP_ONLY))
-            for (uint32_t k = 0; k < K; k++)
-                if (sw->candidates[k] == 32) cluster_k = static_cast<int32_t>(k);   // frontier-push
-        PredictArgs pa{ctx->bfs_ctl, sw->params, K, sw->fallback, sw->threshold, n, m, swh, cluster_k};
+        PredictArgs pa{ctx->bfs_ctl, sw->params, K, sw->fallback, sw->threshold, n, m, swh, true, cluster_k};
         cudaKernelNodeParams kp = {};
         void *pargs[] = {&pa};
         kp.func = reinterpret_cast<void *>(k_bfs_predict);
@@ -922,10 +1016,6 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
         sp.conditional.size = K;
         cudaGraphNode_t snode;
         if ((e = cudaGraphAddNode(&snode, body, &pnode, nullptr, 1, &sp)) != cudaSuccess) { fail(e, "switch node"); break; }
-        BfsArgs a = bfs_args(ctx, g, levels, -1, nullptr);
-        a.skip_check = 1;
-        a.log = log;
-        a.log_cap = log_cap;
         for (uint32_t k = 0; k < K && rc == BW_OK; k++) {
             cudaGraph_t kb = sp.conditional.phGraph_out[k];
             void *kargs[] = {&a};
@@ -954,7 +1044,7 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
             if (plans[k].k2) {
                 cudaKernelNodeParams lp2 = lp;
                 lp2.func = reinterpret_cast<void *>(plans[k].k2);
-                lp2.gridDim = dim3(hub_grid(plans[k].grid, plans[k].block));
+                lp2.gridDim = dim3(plans[k].grid2);
                 lp2.blockDim = dim3(256);
                 lp2.sharedMemBytes = 0;
                 cudaGraphNode_t n2;
@@ -980,33 +1070,16 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
         if (log) cudaFreeAsync(log, s);
         return rc;
     }
-    k_bfs_init_side<<<ctx->sm_count * 4, 256, 0, s>>>(levels, n, root, ctx->queue[0], ctx->bfs_ctl, max_levels,
-                                                     ctx->outdeg);
-    BW_CUDA(cudaGetLastError());
-    BW_CUDA(cudaEventRecord(ctx->ev_start, s));
     BW_CUDA(cudaGraphLaunch(exec, s));
     BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
     BW_CUDA(cudaMemcpyAsync(ctx->bfs_ctl_host, ctx->bfs_ctl, sizeof(BfsCtl), cudaMemcpyDeviceToHost, s));
     BW_CUDA(cudaStreamSynchronize(s));
     cudaGraphExecDestroy(exec);
     cudaGraphDestroy(graph);
-    const BfsCtl c = *ctx->bfs_ctl_host;
-    if (log_cap) {
-        const uint32_t got = std::min(c.levels_done, log_cap);
-        std::vector<LevelSlot> tmp(got ? got : 1);
-        BW_CUDA(cudaMemcpy(tmp.data(), log, got * sizeof(LevelSlot), cudaMemcpyDeviceToHost));
-        for (uint32_t i = 0; i < got; i++) slot_stats(tmp[i], sw->candidates[tmp[i].heavy], &stats[i]);
-        BW_CUDA(cudaFreeAsync(log, s));
-    }
-    if (result) {
-        float ms = 0.0f;
-        BW_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
-        result->level_count = c.levels_done;
-        result->visited = c.visited;
-        result->device_ms = ms;
-        BW_TRY(bfs_traversed(ctx, g, levels, s, &result->traversed_edges));
-    }
-    return c.status ? static_cast<int>(c.status) : BW_OK;
+    end.status = ctx->bfs_ctl_host->status;
+    end.levels_done = ctx->bfs_ctl_host->levels_done;
+    end.visited = ctx->bfs_ctl_host->visited;
+    return finish();
 }
 
 }  // extern "C"
