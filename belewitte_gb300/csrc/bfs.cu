@@ -148,6 +148,7 @@ __global__ void k_bfs_step_post(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap, B
     mail->status = ctl->status;
     mail->levels_done = ctl->levels_done;
     mail->visited = ctl->visited;
+    mail->slot = ctl->slot[(ctl->depth + 2) % 3];     // the next level's input
     __threadfence_system();
     *reinterpret_cast<volatile uint32_t *>(&mail->seq) = seq;
 }
@@ -223,6 +224,7 @@ int plan_launch(const bw_context *ctx, const bw_graph_view *g, int variant, bool
     if (variant < 16) need = blocks(m, 4 * uint64_t(l.block));                        // 4 edges a thread
     else if (variant < 20) need = blocks(n, 4 * uint64_t(l.block));                   // vertex-push: 4 depths a thread
     else if (variant >= 24 && variant < 32) need = blocks(n, uint64_t(C) * (l.block / W));
+    else if (variant == V_FRONTIER_PUSH) need = blocks(n, 32);                        // 8 warps of 4 rows
     else need = blocks(n, l.block);
     l.grid = static_cast<unsigned>(std::min<uint64_t>(l.grid, need));
     // at most this many hub chunks in a level (ensure_bfs_scratch), one per warp
@@ -398,8 +400,8 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
         a.log = log;
         a.log_cap = log_cap;
     }
-    auto level_kernels = [&](cudaStream_t to) {
-        if (cluster_path) bfs_cluster_kernel(side ? 1 : 0)<<<CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), to>>>(a);
+    auto level_kernels = [&](cudaStream_t to, bool small) {
+        if (cluster_path && small) bfs_cluster_kernel(side ? 1 : 0)<<<CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), to>>>(a);
         plan.k<<<plan.grid, plan.block, plan.smem, to>>>(a);
         if (plan.k2) plan.k2<<<plan.grid2, 256, 0, to>>>(a);
     };
@@ -410,7 +412,7 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
         BW_CUDA(cudaGetLastError());
         BW_CUDA(cudaEventRecord(ctx->ev_start, s));
         for (uint32_t i = 0; i < DEVICE_LOOP_LAUNCHED && !end.stop; i++) {
-            level_kernels(s);
+            level_kernels(s, i == 0 || cluster_frontier(end.slot));
             const uint32_t seq = ++ctx->mail_seq;
             k_bfs_step_post<<<1, 32, 0, s>>>(ctx->bfs_ctl, log, log_cap, ctx->mail, seq);
             BW_CUDA(cudaGetLastError());
@@ -426,7 +428,7 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
                 L2Window win;
                 if (window) BW_TRY(l2_window_begin(ctx, cap, levels, n * sizeof(int32_t), win, false));
                 BW_CUDA(cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-                level_kernels(cap);
+                level_kernels(cap, true);
                 k_bfs_step<<<1, 32, 0, cap>>>(ctx->bfs_ctl, log, log_cap, handle);
                 cudaGraph_t captured = body;
                 const cudaError_t e = cudaStreamEndCapture(cap, &captured);

@@ -268,18 +268,19 @@ __global__ void __launch_bounds__(512) k_bfs_edge(BfsArgs a)
 
 // ---------------------------------------------------------------------------
 // vertex-push (bfs/vertex_push.cu:3-26): thread per vertex; a frontier
-// vertex's owner walks its CSR row.  Depths are scanned 4 per thread.  A
-// row longer than BFS_PUSH_HEAVY is expanded by the owner's whole warp
-// (lane-strided, coalesced) instead of by its one thread, whose serial
-// chain of relaxations would otherwise hold the level: a hub's row is the
-// level's critical path.
+// vertex's owner walks its CSR row.  Depths are scanned 4 per thread.  The
+// rows of a warp's frontier vertices are expanded as one concatenation, an
+// edge per lane, BFS_PUSH_UNROLL in flight: neighbours in id are hubs
+// together on R-MAT, and one row after the other a warp's chain of
+// relaxations holds the level.  A whole traversal on GB300 (host loop, rows
+// one by one before): R-MAT-16 371 -> 157 us, R-MAT-22 symmetrised 1719 ->
+// 1127, BA(2M, 8) 1778 -> 785.
 // ---------------------------------------------------------------------------
-constexpr uint32_t BFS_PUSH_HEAVY = 32;
 constexpr int BFS_PUSH_UNROLL = 8;
 // Rows above BFS_PUSH_GIANT edges are cut into HUB_CHUNK chunks for
 // k_bfs_hub_chunks (the level's second kernel), as frontier-push does: one
 // warp expanding a hub of R-MAT's lowest ids would hold the level.
-constexpr uint32_t BFS_PUSH_GIANT = 1024;
+constexpr uint32_t BFS_PUSH_GIANT = 256;
 
 __device__ __forceinline__ void queue_hub_chunks(const BfsArgs &a, LevelSlot *slot, uint32_t v, uint32_t s,
                                                  uint32_t e)
@@ -287,6 +288,43 @@ __device__ __forceinline__ void queue_hub_chunks(const BfsArgs &a, LevelSlot *sl
     const uint32_t chunks = (e - s + HUB_CHUNK - 1) / HUB_CHUNK;
     const uint32_t base = atomicAdd(&slot->heavy, chunks);
     for (uint32_t c = 0; c < chunks; c++) a.heavy[base + c] = make_uint2(v, s + c * HUB_CHUNK);
+}
+
+// The row that edge k of a warp's concatenated rows belongs to: the last lane
+// whose exclusive prefix is <= k (that lane's row is not empty).  Every lane
+// calls.
+__device__ __forceinline__ uint32_t concat_row(uint32_t excl, uint32_t k)
+{
+    uint32_t l = 0;
+#pragma unroll
+    for (uint32_t b = 16; b > 0; b >>= 1)
+        if (__shfl_sync(FULL_MASK, excl, l + b) <= k) l += b;
+    return l;
+}
+
+// Relaxes up to U neighbours (NO_VERTEX: none): their depths are all in
+// flight before the first relaxation, the relaxations' atomics before the
+// first result, and only a neighbour not yet visited costs an atomic.
+constexpr uint32_t NO_VERTEX = 0xffffffffu;
+template<int U>
+__device__ __forceinline__ void claim_all(int32_t *lv, int32_t nd, const uint32_t (&u)[U], bool (&won)[U])
+{
+    int32_t d[U];
+#pragma unroll
+    for (int j = 0; j < U; j++) d[j] = u[j] != NO_VERTEX ? lv[u[j]] : nd;
+#pragma unroll
+    for (int j = 0; j < U; j++) d[j] = d[j] > nd ? atomicMin(&lv[u[j]], nd) : nd;
+#pragma unroll
+    for (int j = 0; j < U; j++) won[j] = d[j] > nd;
+}
+template<int U, class Visit>
+__device__ __forceinline__ void relax_all(int32_t *lv, int32_t nd, const uint32_t (&u)[U], Visit visit)
+{
+    bool won[U];
+    claim_all(lv, nd, u, won);
+#pragma unroll
+    for (int j = 0; j < U; j++)
+        if (won[j]) visit(u[j]);
 }
 
 // Relaxes the neighbours E[first + k * step] (k < BFS_PUSH_UNROLL, below
@@ -298,17 +336,12 @@ __device__ __forceinline__ void relax_neighbours(const BfsArgs &a, const uint32_
                                                  Side<SIDE> &side, uint32_t *qnext, LevelSlot *slot)
 {
     uint32_t u[BFS_PUSH_UNROLL];
-    int32_t d[BFS_PUSH_UNROLL];
 #pragma unroll
     for (int k = 0; k < BFS_PUSH_UNROLL; k++) {
         const uint32_t i = first + k * step;
-        u[k] = i < end ? __ldg(E + i) : 0u;
+        u[k] = i < end ? __ldg(E + i) : NO_VERTEX;
     }
-#pragma unroll
-    for (int k = 0; k < BFS_PUSH_UNROLL; k++) d[k] = first + k * step < end ? lv[u[k]] : nd;
-#pragma unroll
-    for (int k = 0; k < BFS_PUSH_UNROLL; k++)
-        if (d[k] > nd && atomicMin(&lv[u[k]], nd) > nd) { cnt.hit(&slot->frontier); side.visit(a, qnext, slot, u[k]); }
+    relax_all(lv, nd, u, [&](uint32_t w) { cnt.hit(&slot->frontier); side.visit(a, qnext, slot, w); });
 }
 
 template<int RED, bool SIDE>
@@ -323,21 +356,28 @@ __global__ void __launch_bounds__(512) k_bfs_vertex_push(BfsArgs a)
     Side<SIDE> side;
     const unsigned lane = threadIdx.x & 31;
     const uint64_t n = a.n, stride = gthreads();
-    // every lane calls it (warp-uniform loops); rows [s, e) of frontier
-    // vertices, empty for the others
-    auto relax_batch = [&](uint32_t first, uint32_t step, uint32_t end) {
-        relax_neighbours(a, a.fwd_e, lv, nd, first, step, end, cnt, side, qnext, slot);
-    };
+    // every lane calls it; rows [s, e) of frontier vertices, empty for the others
     auto expand = [&](uint32_t v, uint32_t s, uint32_t e) {
-        const bool giant = e - s > BFS_PUSH_GIANT;
-        if (giant) queue_hub_chunks(a, slot, v, s, e);
-        const bool heavy = !giant && e - s > BFS_PUSH_HEAVY;
-        if (!heavy && !giant)
-            for (uint32_t i = s; i < e; i += BFS_PUSH_UNROLL) relax_batch(i, 1, e);
-        for (unsigned hv = __ballot_sync(FULL_MASK, heavy); hv; hv &= hv - 1) {
-            const unsigned l = __ffs(hv) - 1;
-            const uint32_t hs = __shfl_sync(FULL_MASK, s, l), he = __shfl_sync(FULL_MASK, e, l);
-            for (uint32_t base = hs; base < he; base += 32 * BFS_PUSH_UNROLL) relax_batch(base + lane, 32, he);
+        if (e - s > BFS_PUSH_GIANT) {
+            queue_hub_chunks(a, slot, v, s, e);
+            e = s;
+        }
+        if (!__any_sync(FULL_MASK, e > s)) return;
+        uint32_t incl = e - s;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL_MASK, incl, o);
+            if (lane >= static_cast<unsigned>(o)) incl += y;
+        }
+        const uint32_t total = __shfl_sync(FULL_MASK, incl, 31), excl = incl - (e - s), from = s - excl;
+        for (uint32_t k0 = 0; k0 < total; k0 += 32 * BFS_PUSH_UNROLL) {
+            uint32_t u[BFS_PUSH_UNROLL];
+#pragma unroll
+            for (int j = 0; j < BFS_PUSH_UNROLL; j++) {
+                const uint32_t k = k0 + j * 32 + lane, row = concat_row(excl, k);
+                const uint32_t at = __shfl_sync(FULL_MASK, from, row) + k;
+                u[j] = k < total ? __ldg(a.fwd_e + at) : NO_VERTEX;
+            }
+            relax_all(lv, nd, u, [&](uint32_t w) { cnt.hit(&slot->frontier); side.visit(a, qnext, slot, w); });
         }
     };
     const uint64_t groups = (reinterpret_cast<uintptr_t>(lv) & 15) ? 0 : n >> 2;
@@ -506,18 +546,22 @@ __global__ void __launch_bounds__(512) k_bfs_vwarp(BfsArgs a)
 
 // ---------------------------------------------------------------------------
 // frontier-push (GB300 variant): top-down over the frontier queue only.
-// A warp takes 32 queue entries; their rows are concatenated (warp prefix
-// sum of degrees) and the warp's lanes sweep the concatenation, so every
-// lane does the same amount of edge work and reads within a row coalesce.
+// A warp takes up to 32 queue entries; their rows are concatenated (warp
+// prefix sum of degrees) and the warp's lanes sweep the concatenation,
+// FRONTIER_UNROLL edges in flight each, so every lane does the same amount
+// of edge work and reads within a row coalesce.  A level is a chain of
+// dependent accesses per step (index, depth, claim): with one edge in flight
+// per lane a traversal of BA(2M, 8) took 714 us on GB300 and takes 399 with
+// four, and the whole of a hub chunk in flight.
 // Rows above HEAVY_DEGREE are cut into HUB_CHUNK chunks queued for
 // k_bfs_hub_chunks, which spreads a hub over the whole GPU.
 // Always emits the next queue.
 // ---------------------------------------------------------------------------
+constexpr int FRONTIER_UNROLL = 4;
+
 template<bool SIDE>
 __global__ void __launch_bounds__(256) k_bfs_frontier_push(BfsArgs a)
 {
-    __shared__ uint32_t s_excl[8][32];
-    __shared__ uint32_t s_start[8][32];
     __shared__ uint32_t s_stage[8][WARP_STAGE];
     if (a.skip_check && *((volatile uint32_t *) &a.ctl->skip)) return;
     const int32_t depth = level_depth(a), nd = depth + 1;
@@ -535,18 +579,18 @@ __global__ void __launch_bounds__(256) k_bfs_frontier_push(BfsArgs a)
     WarpQueue wq;
     wq.stage = s_stage[wib];
 
-    for (uint64_t t = warp * 32; t < qlen; t += warps * 32) {
+    // a short queue is spread over the warps, down to a row each
+    const uint32_t per = static_cast<uint32_t>(min(uint64_t(32), (qlen + warps - 1) / warps));
+    for (uint64_t t = warp * per; t < qlen; t += warps * per) {
         const uint64_t i = t + lane;
         uint32_t v = 0, s = 0, d = 0;
-        if (i < qlen) {
+        if (lane < per && i < qlen) {
             v = qin[i];
             s = a.fwd_v[v];
             d = a.fwd_v[v + 1] - s;
         }
         if (d > HEAVY_DEGREE) {
-            const uint32_t chunks = (d + HUB_CHUNK - 1) / HUB_CHUNK;
-            const uint32_t base = atomicAdd(&slot->heavy, chunks);
-            for (uint32_t c = 0; c < chunks; c++) a.heavy[base + c] = make_uint2(v, s + c * HUB_CHUNK);
+            queue_hub_chunks(a, slot, v, s, s + d);
             d = 0;
         }
         uint32_t incl = d;
@@ -554,31 +598,29 @@ __global__ void __launch_bounds__(256) k_bfs_frontier_push(BfsArgs a)
             const uint32_t y = __shfl_up_sync(FULL_MASK, incl, o);
             if (lane >= static_cast<unsigned>(o)) incl += y;
         }
-        const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
-        s_excl[wib][lane] = incl - d;
-        s_start[wib][lane] = s;
-        __syncwarp();
-        // edge k of the concatenated rows: a per-lane cursor over the rows'
-        // exclusive offsets; whole-warp steps, so that the new vertices are
-        // staged with one ballot per step
-        uint32_t seg = 0;
-        for (uint32_t k0 = 0; k0 < total; k0 += 32) {
-            const uint32_t k = k0 + lane;
-            bool got = false;
-            uint32_t u = 0;
-            if (k < total) {
-                while (seg < 31 && s_excl[wib][seg + 1] <= k) seg++;
-                u = __ldg(a.fwd_e + s_start[wib][seg] + (k - s_excl[wib][seg]));
-                got = relax(lv, u, nd);
+        const uint32_t total = __shfl_sync(FULL_MASK, incl, 31), excl = incl - d, from = s - excl;
+        // whole-warp steps, so that the new vertices are staged with one
+        // ballot each
+        for (uint32_t k0 = 0; k0 < total; k0 += 32 * FRONTIER_UNROLL) {
+            uint32_t u[FRONTIER_UNROLL];
+            bool won[FRONTIER_UNROLL];
+#pragma unroll
+            for (int j = 0; j < FRONTIER_UNROLL; j++) {
+                const uint32_t k = k0 + j * 32 + lane, row = concat_row(excl, k);
+                const uint32_t at = __shfl_sync(FULL_MASK, from, row) + k;
+                u[j] = k < total ? __ldg(a.fwd_e + at) : NO_VERTEX;
             }
-            if (got) {
-                cnt.hit(&slot->frontier);
-                if constexpr (SIDE) side.visit(a, nullptr, nullptr, u);
-                else if (a.skip_check) fe += a.outdeg[u];
+            claim_all(lv, nd, u, won);
+#pragma unroll
+            for (int j = 0; j < FRONTIER_UNROLL; j++) {
+                if (won[j]) {
+                    cnt.hit(&slot->frontier);
+                    if constexpr (SIDE) side.visit(a, nullptr, nullptr, u[j]);
+                    else if (a.skip_check) fe += a.outdeg[u[j]];
+                }
+                wq.add(won[j], u[j], qnext, &slot->qlen);
             }
-            wq.add(got, u, qnext, &slot->qlen);
         }
-        __syncwarp();
     }
     wq.flush(qnext, &slot->qlen);
     cnt.finish(&slot->frontier);
@@ -606,20 +648,23 @@ __global__ void __launch_bounds__(256) k_bfs_hub_chunks(BfsArgs a)
     for (uint64_t c = warp; c < chunks; c += warps) {
         const uint2 h = a.heavy[c];
         const uint32_t end = min(h.y + HUB_CHUNK, a.fwd_v[h.x + 1]);
-        for (uint32_t i0 = h.y; i0 < end; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            bool got = false;
-            uint32_t u = 0;
-            if (i < end) {
-                u = __ldcs(a.fwd_e + i);
-                got = relax(lv, u, nd);
-            }
-            if (got) {
+        // the whole chunk in flight
+        uint32_t u[HUB_CHUNK / 32];
+        bool won[HUB_CHUNK / 32];
+#pragma unroll
+        for (int j = 0; j < static_cast<int>(HUB_CHUNK / 32); j++) {
+            const uint32_t i = h.y + j * 32 + lane;
+            u[j] = i < end ? __ldcs(a.fwd_e + i) : NO_VERTEX;
+        }
+        claim_all(lv, nd, u, won);
+#pragma unroll
+        for (int j = 0; j < static_cast<int>(HUB_CHUNK / 32); j++) {
+            if (won[j]) {
                 cnt.hit(&slot->frontier);
-                if constexpr (SIDE) side.visit(a, nullptr, nullptr, u);
-                else if (a.skip_check) fe += a.outdeg[u];
+                if constexpr (SIDE) side.visit(a, nullptr, nullptr, u[j]);
+                else if (a.skip_check) fe += a.outdeg[u[j]];
             }
-            wq.add(got, u, qnext, &slot->qlen);
+            wq.add(won[j], u[j], qnext, &slot->qlen);
         }
     }
     wq.flush(qnext, &slot->qlen);

@@ -252,6 +252,9 @@ constexpr unsigned CLUSTER_THREADS = 1024;
 constexpr uint32_t CLUSTER_LIST = 4096;            // frontier entries per block list
 constexpr uint32_t CLUSTER_CAP = CLUSTER_LIST * CLUSTER_CTAS;   // frontier vertices the cluster kernel takes
 constexpr unsigned long long CLUSTER_EDGE_CAP = 65536;        // and their out-edges
+// A frontier the cluster kernel takes on (unless a row is too long for it).
+__host__ __device__ inline bool cluster_frontier(const LevelSlot &s)
+{ return s.qlen > 0 && s.qlen <= CLUSTER_CAP && s.fedges <= CLUSTER_EDGE_CAP; }
 
 // Reference Backend::computeDivision (Backend.cpp:52-70).
 void compute_division(uint64_t count, uint32_t sm, uint32_t max_tpb,

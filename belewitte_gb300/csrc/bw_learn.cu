@@ -366,7 +366,7 @@ __device__ void predict_level(const PredictArgs &a)
         // a frontier the cluster kernel takes goes to frontier-push (the
         // decision is uniform: every thread reads the same slot)
         const LevelSlot s = c->slot[(L + 2) % 3];
-        if (s.qlen > 0 && s.qlen <= CLUSTER_CAP && s.fedges <= CLUSTER_EDGE_CAP) {
+        if (cluster_frontier(s)) {
             if (tid == 0) {
                 c->variant = a.cluster_k;
                 if (a.in_graph) cudaGraphSetConditional(a.sw, static_cast<unsigned>(a.cluster_k));
@@ -464,6 +464,7 @@ __global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_next(PredictArgs a, boo
     mail->status = c->status;
     mail->levels_done = c->levels_done;
     mail->visited = c->visited;
+    mail->slot = c->slot[(c->depth + 2) % 3];         // the next level's input
     __threadfence_system();
     *reinterpret_cast<volatile uint32_t *>(&mail->seq) = seq;
 }
@@ -932,7 +933,7 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
             const Plan &p = plans[end.variant];
             // the level log needs every level's statistics; otherwise only a
             // handed-over level's, which the next prediction reads
-            if (sw->candidates[end.variant] == 32)
+            if (sw->candidates[end.variant] == 32 && cluster_frontier(end.slot))
                 bfs_cluster_kernel(log_cap ? 1 : 2)<<<CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), s>>>(a);
             p.k<<<p.grid, p.block, p.smem, s>>>(a);
             if (p.k2) p.k2<<<p.grid2, 256, 0, s>>>(a);
