@@ -28,6 +28,7 @@
 // that overflows are reported to the caller, which then runs the plain loop.
 #pragma once
 #include <stdint.h>
+#include <string.h>
 
 #if defined(__CUDACC__)
 #define BWS_HD __host__ __device__ __forceinline__
@@ -133,5 +134,61 @@ BWS_HD bool in_domain(uint32_t sb)
     const uint32_t k = exponent_of(sb);
     return !(sb >> 31) && k != 0 && k != 0xffu;
 }
+
+// The map of a run of terms from two chains of float additions.  The
+// binade's smallest even and odd significands, 2^23 and 2^23 + 1, are
+// themselves running sums; adding the run to each of them in order gives
+// the two increments as differences of bit patterns: two additions a term,
+// where step_select and compose_short take about 30 instructions.  While a
+// chain stays in the binade its increments are those of every significand of
+// its parity (the rounding depends on nothing else).  A chain that leaves the
+// binade ends at or above 2^24, so its increment takes every significand of
+// its parity, none smaller than the chain's start, out of the binade as well:
+// all that the map then has to say.  Terms that are negative, infinite or NaN
+// are outside the domain (CHAIN_TERM_MAX).
+BWS_HD float float_of(uint32_t b)
+{
+#if defined(__CUDA_ARCH__)
+    return __uint_as_float(b);
+#else
+    float f;
+    memcpy(&f, &b, sizeof f);
+    return f;
+#endif
+}
+BWS_HD uint32_t float_bits(float f)
+{
+#if defined(__CUDA_ARCH__)
+    return __float_as_uint(f);
+#else
+    uint32_t b;
+    memcpy(&b, &f, sizeof b);
+    return b;
+#endif
+}
+BWS_HD float add_rn(float a, float b)
+{
+#if defined(__CUDA_ARCH__)
+    return __fadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+struct Chain {
+    float e, o;
+};
+BWS_HD Chain chain_start(uint32_t k) { return Chain{float_of(k << 23), float_of((k << 23) + 1u)}; }
+BWS_HD void chain_add(Chain &c, float x)
+{
+    c.e = add_rn(c.e, x);
+    c.o = add_rn(c.o, x);
+}
+BWS_HD Map chain_map(const Chain &c, uint32_t k)
+{
+    return Map{saturate(float_bits(c.e) - (k << 23)), saturate(float_bits(c.o) - (k << 23) - 1u)};
+}
+// The largest bit pattern of a chain's terms, at most this when they are all
+// in the domain.
+constexpr uint32_t CHAIN_TERM_MAX = 0x7f7fffffu;
 
 }  // namespace bwseq

@@ -16,15 +16,15 @@ namespace bw {
 // next window's loads in flight).  Terms at row positions below
 // SERIAL_TERMS are added by lane 0 in order: there the sum doubles every
 // few terms, and a binade crossing costs the map scan a restart.  The rest
-// uses the binade maps of bw_seqsum.h: each lane composes the maps of its L
-// consecutive terms as a tree (depth log2 L, branch-free steps), the warp
-// scans the lanes' maps, and the lane that holds the next binade crossing
-// adds that term with one float addition.  `stage` holds 33 x L floats of
+// uses the binade maps of bw_seqsum.h: each lane has the map of its L
+// consecutive terms from two chains of float additions, the warp scans the
+// lanes' maps, and the lane that holds the next binade crossing finds it with
+// the plain additions.  `stage` holds 33 x L floats of
 // shared memory per warp; load(i) returns the row's term at position i
 // (called for i < e only).  False when a
 // term or the sum leaves the maps' domain (the caller then runs the plain
 // loop); `sb` is warp-uniform.
-constexpr uint32_t SERIAL_TERMS = 1024;   // measured: 64 was 23% slower on R-MAT-22
+constexpr uint32_t SERIAL_TERMS = 1024;
 
 template<uint32_t L, class Load>
 __device__ __forceinline__ bool warp_sequential_continue_load(Load load, uint32_t b, uint32_t e, uint32_t &sb,
@@ -85,22 +85,17 @@ __device__ __forceinline__ bool warp_sequential_continue_load(Load load, uint32_
             }
             if (!in_domain(sb)) { ok = false; break; }
             const uint32_t K = exponent_of(sb), A = significand_of(sb);
-            // this lane's terms as maps (inactive terms: +0, the identity),
-            // composed as a tree
-            Map t[L];
-            bool good = true;
+            // the map of this lane's terms (inactive terms: +0, the identity)
+            Chain chain = chain_start(K);
+            uint32_t worst = 0;
 #pragma unroll
             for (uint32_t u = 0; u < L; u++) {
-                const bool live = first + u >= pos && first + u < lim;
-                t[u] = step_select(live ? x[u] : 0u, K, good);
+                const uint32_t xu = first + u >= pos && first + u < lim ? x[u] : 0u;
+                worst = max(worst, xu);
+                chain_add(chain, __uint_as_float(xu));
             }
-#pragma unroll
-            for (uint32_t st = 1; st < L; st <<= 1) {
-#pragma unroll
-                for (uint32_t u = 0; u + st < L; u += 2 * st) t[u] = compose_short(t[u], t[u + st]);
-            }
-            const Map m = saturated(t[0]);
-            if (__any_sync(FULL_MASK, !good)) { ok = false; break; }
+            const Map m = chain_map(chain, K);
+            if (__any_sync(FULL_MASK, worst > CHAIN_TERM_MAX)) { ok = false; break; }
             Map incl = m;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -119,21 +114,15 @@ __device__ __forceinline__ bool warp_sequential_continue_load(Load load, uint32_
             const unsigned f = __ffs(cross) - 1;
             uint32_t nb = 0, np = 0;
             if (lane == f) {
-                uint32_t acc = a0;
+                float acc = __uint_as_float(bits_of(K, a0));
 #pragma unroll
                 for (uint32_t u = 0; u < L; u++) {
                     if (np == 0 && first + u >= pos && first + u < lim) {
-                        Map tu;
-                        step(x[u], K, tu);
-                        const uint32_t bu = apply(tu, acc);
-                        if (bu >= TOP) {
-                            nb = __float_as_uint(__fadd_rn(__uint_as_float(bits_of(K, acc)), __uint_as_float(x[u])));
-                            np = first + u + 1;
-                        } else {
-                            acc = bu;
-                        }
+                        acc = __fadd_rn(acc, __uint_as_float(x[u]));
+                        if (exponent_of(__float_as_uint(acc)) != K) np = first + u + 1;
                     }
                 }
+                nb = __float_as_uint(acc);
             }
             np = __shfl_sync(FULL_MASK, np, f);
             sb = __shfl_sync(FULL_MASK, nb, f);

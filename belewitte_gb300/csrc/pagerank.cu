@@ -182,6 +182,20 @@ __device__ __forceinline__ void add_diff(float *slot, float d)
     if ((threadIdx.x & 31) == 0 && d != 0.0f) atomicAdd(slot, d);
 }
 
+// The same with one atomic per block: thousands of warps' float atomics on
+// one word are a microsecond or two of a launch, and each rounds the sum.
+// Every thread calls; `scratch`: 32 floats of shared memory that nothing else
+// uses from here on.
+__device__ __forceinline__ void add_diff_block(float *slot, float d, float *scratch)
+{
+    const unsigned lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(FULL_MASK, d, o);
+    __syncthreads();
+    if (lane == 0) scratch[wib] = d;
+    __syncthreads();
+    if (wib == 0) add_diff(slot, lane < blockDim.x / 32 ? scratch[lane] : 0.0f);
+}
+
 // ----------------------------- degrees ------------------------------------
 // Histogram of a source-id stream with warp aggregation of equal ids
 // (one atomic per distinct id per warp step).  Counting inEdges of the
@@ -1026,31 +1040,53 @@ __global__ void k_piece_count(const uint32_t *__restrict__ long_len, const uint3
         pieces[i] = i < L ? (long_len[i] + SEG_EDGES - 1) / SEG_EDGES : 0u;
 }
 
-// Exact long rows above GIANT_ROW terms are summed piece-parallel (binade
-// maps per piece, combined by the row's last piece); shorter ones in
-// batches of 32, one row per lane.  A lane's row is a chain of dependent
-// additions with only a few dozen of its terms in flight (the warp's
-// shared-memory ring): the longest batch rows set the kernel's critical
-// path, which bounds their length.
-constexpr uint32_t GIANT_ROW = 2048;
+// Exact long rows of at least giant_row(m) terms are summed piece-parallel
+// (binade maps per piece, combined by the row's last piece); shorter ones in
+// batches of 32, one row per lane.  A giant row costs a start, the arrivals
+// and a combination, about 6 us of a warp; a batch row is a chain of dependent
+// additions, some 10 to 20 cycles a term with its terms on the way from L2.
+// On a small graph the longest chain is the whole kernel, on a large one the
+// warps' total work is.  Iterations of vertex-pull on GB300 (us, one build) with giant
+// rows from 512 / 1024 / 2048 / 4096 terms:
+//   R-MAT, 50,021 vertices (1M edges)  28 / 33 / 42 / 57
+//   R-MAT-20 (16M)                    119 / 96 / 115 / 123
+//   R-MAT-21 (32M)                      - / 165 / 152 / -
+//   R-MAT-22 (64M)                      - / 309 / 281 / 281
+//   R-MAT-24 (260M)                     - / 1296 / 1162 / 1090 (8192: 1089)
+constexpr uint32_t GIANT_LEAST = 512;
+constexpr uint64_t MEGA = uint64_t(1) << 20;
+__host__ __device__ constexpr uint32_t giant_row(uint64_t m)
+{
+    return m < 8 * MEGA ? GIANT_LEAST : m < 24 * MEGA ? 1024 : m < 128 * MEGA ? 2048 : 4096;
+}
+// The sums' shape: below SUM_SMALL_EDGES one block per SM whose warps hold
+// eight stages of the batch rows (a chain's speed is the terms in flight:
+// R-MAT-20 96 us an iteration, 103 with three stages and three blocks), above
+// three stages and three blocks per SM (R-MAT-24 1162 us, 1215 with two
+// blocks).
+constexpr uint32_t SUM_STAGES = 3, SUM_STAGES_SMALL = 8;
+constexpr int SUM_BLOCKS = 3, SUM_BLOCKS_SMALL = 1;
+constexpr uint64_t SUM_SMALL_EDGES = 24 * MEGA;
 
 // Long rows are put in decreasing length order by one stable counting sort
-// on this key (smaller key, earlier row).  Rows of at most GIANT_ROW terms
-// (the batch rows) get one key per length, so their order is exact: rows of
-// equal length in row order.  The giant rows come first, in 64 classes per
-// octave of length (1.1% wide), each class in row order: their order only
-// schedules their pieces.
-constexpr uint32_t LONG_GIANT_KEYS = (32 - 11) * 64;                       // octaves 2^11 .. 2^31
+// on this key (smaller key, earlier row).  Rows below LONG_CLASSED terms get
+// one key per length, so their order is exact: rows of equal length in row
+// order.  The longer rows come first, in 64 classes per octave of length
+// (1.1% wide), each class in row order: their order only schedules their
+// sums.  A giant-row threshold is a power of two from LONG_CLASSED on, where
+// a class begins, so the giant rows lead the list.
+constexpr uint32_t LONG_CLASSED = 512;
+constexpr uint32_t LONG_GIANT_KEYS = (32 - 9) * 64;                        // octaves 2^9 .. 2^31
 constexpr int LONG_SORT_BINS = 4096, LONG_SORT_WARPS = 4, LONG_SORT_GRID = 64;
-static_assert(LONG_GIANT_KEYS + GIANT_ROW <= LONG_SORT_BINS, "every key is a bin");
+static_assert(LONG_GIANT_KEYS + LONG_CLASSED <= LONG_SORT_BINS, "every key is a bin");
 __device__ __forceinline__ uint32_t long_row_key(uint32_t len)
 {
-    if (len > GIANT_ROW) {
-        const uint32_t b = 31u - static_cast<uint32_t>(__clz(len));              // 11 .. 31
-        const uint32_t cls = (b - 11u) * 64u + ((len >> (b - 6u)) & 63u);      // grows with len
+    if (len >= LONG_CLASSED) {
+        const uint32_t b = 31u - static_cast<uint32_t>(__clz(len));              // 9 .. 31
+        const uint32_t cls = (b - 9u) * 64u + ((len >> (b - 6u)) & 63u);      // grows with len
         return LONG_GIANT_KEYS - 1u - cls;
     }
-    return LONG_GIANT_KEYS + (GIANT_ROW - len);
+    return LONG_GIANT_KEYS + (LONG_CLASSED - 1u - len);
 }
 struct LongRowDigit {
     const uint32_t *len;
@@ -1069,18 +1105,20 @@ struct LongRowPut {
 };
 
 // Pieces of sorted long row i at [ppos[i], ppos[i + 1]); the arrival
-// counters cleared; the number of rows above GIANT_ROW and of their pieces.
+// counters cleared; the number of giant rows (at least `giant` edges) and of
+// their pieces.  A piece's item: {row, its number in the row | LONG_FLAG,
+// edge_begin, edge_end}.
 __global__ void k_piece_emit(const uint32_t *__restrict__ off, const uint32_t *__restrict__ long_row,
                              const uint32_t *__restrict__ long_len, const uint32_t *__restrict__ long_total,
                              const uint32_t *__restrict__ ppos, uint4 *__restrict__ work,
                              uint32_t *__restrict__ long_count, uint32_t *__restrict__ giant_total,
-                             uint32_t *__restrict__ giant_pieces)
+                             uint32_t *__restrict__ giant_pieces, uint32_t giant)
 {
     const uint64_t L = *long_total;
     uint64_t lo = 0, hi = L;                       // giant rows come first (lengths decrease)
     while (lo < hi) {
         const uint64_t mid = (lo + hi) / 2;
-        if (long_len[mid] > GIANT_ROW) lo = mid + 1; else hi = mid;
+        if (long_len[mid] >= giant) lo = mid + 1; else hi = mid;
     }
     if (gtid() == 0) {
         *giant_total = static_cast<uint32_t>(lo);
@@ -1088,10 +1126,10 @@ __global__ void k_piece_emit(const uint32_t *__restrict__ off, const uint32_t *_
     }
     for (uint64_t i = gtid(); i < L; i += gthreads()) {
         const uint32_t r = long_row[i];
-        uint32_t out = ppos[i], p = off[r];
+        uint32_t out = ppos[i], p = off[r], q = 0;
         long_count[r] = 0;
         for (; p < off[r + 1]; p += SEG_EDGES)
-            work[out++] = make_uint4(r, (r + 1) | LONG_FLAG, p, min(p + SEG_EDGES, off[r + 1]));
+            work[out++] = make_uint4(r, q++ | LONG_FLAG, p, min(p + SEG_EDGES, off[r + 1]));
     }
 }
 
@@ -1242,8 +1280,8 @@ __global__ void __launch_bounds__(SEG_WARPS * 32) k_seg_emit(const uint32_t *__r
 // its own row strided from the others (one 16-byte load per lane and
 // instruction) keeps L1TEX on 32 lines per load: measured on GB300, about
 // 88 cycles a term.  Instead the warp stages its 32 rows through a ring of
-// BATCH_STAGES stages in shared memory with coalesced 16-byte cp.async
-// copies, issued BATCH_STAGES - 1 stages ahead.  Stage c of a row is the
+// STAGES stages in shared memory with coalesced 16-byte cp.async
+// copies, issued STAGES - 1 stages ahead.  Stage c of a row is the
 // 16-byte aligned window of BATCH_TERMS floats at (beg & ~3) + c *
 // BATCH_TERMS; window positions before beg or past the row's end add +0,
 // which leaves the running sum unchanged (it starts at +0 and is never -0:
@@ -1254,8 +1292,7 @@ __global__ void __launch_bounds__(SEG_WARPS * 32) k_seg_emit(const uint32_t *__r
 constexpr uint32_t BATCH_TERMS = 16;
 constexpr uint32_t BATCH_CHUNKS = BATCH_TERMS / 4;          // 16-byte chunks of a row per stage
 constexpr uint32_t BATCH_SLOT = BATCH_TERMS + 4;            // padded: conflict-free 16-byte reads
-constexpr uint32_t BATCH_STAGES = 3;
-constexpr uint32_t BATCH_RING = BATCH_STAGES * 32 * BATCH_SLOT;   // floats per warp
+__host__ __device__ constexpr uint32_t batch_ring(uint32_t stages) { return stages * 32 * BATCH_SLOT; }   // floats per warp
 static_assert(BATCH_TERMS % 4 == 0 && 32 % BATCH_CHUNKS == 0, "whole chunks; whole rows per copy");
 
 __device__ __forceinline__ void cp_async16(float *dst, const float *src, uint32_t bytes)
@@ -1268,6 +1305,7 @@ template<int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // Out of line: its registers are allocated apart from the giant-row path's.
+template<uint32_t STAGES>
 __device__ __noinline__ float batch_sequential_sum(const float *vals, uint32_t beg, uint32_t len, float *ring,
                                                    unsigned lane)
 {
@@ -1285,7 +1323,7 @@ __device__ __noinline__ float batch_sequential_sum(const float *vals, uint32_t b
         ce[i] = __shfl_sync(FULL_MASK, end, r);
     }
     auto issue = [&](uint32_t c) {
-        float *st = ring + (c % BATCH_STAGES) * (32 * BATCH_SLOT);
+        float *st = ring + (c % STAGES) * (32 * BATCH_SLOT);
 #pragma unroll
         for (uint32_t i = 0; i < COPIES; i++) {
             const uint32_t r = i * ROWS_PER_COPY + lane / BATCH_CHUNKS, g = cg[i] + c * BATCH_TERMS;
@@ -1294,18 +1332,18 @@ __device__ __noinline__ float batch_sequential_sum(const float *vals, uint32_t b
         }
     };
 #pragma unroll 1
-    for (uint32_t c = 0; c + 1 < BATCH_STAGES; c++) {
+    for (uint32_t c = 0; c + 1 < STAGES; c++) {
         if (c < stages) issue(c);
         cp_async_commit();
     }
     float acc = 0.0f;
 #pragma unroll 1
     for (uint32_t c = 0; c < stages; c++) {
-        if (c + BATCH_STAGES - 1 < stages) issue(c + BATCH_STAGES - 1);
+        if (c + STAGES - 1 < stages) issue(c + STAGES - 1);
         cp_async_commit();
-        cp_async_wait<BATCH_STAGES - 1>();           // this lane's copies of stage c are done
+        cp_async_wait<STAGES - 1>();           // this lane's copies of stage c are done
         __syncwarp();                                // ... and every lane's
-        const float4 *mine = reinterpret_cast<const float4 *>(ring + (c % BATCH_STAGES) * (32 * BATCH_SLOT) +
+        const float4 *mine = reinterpret_cast<const float4 *>(ring + (c % STAGES) * (32 * BATCH_SLOT) +
                                                               lane * BATCH_SLOT);
         float x[BATCH_TERMS];
 #pragma unroll
@@ -1322,7 +1360,7 @@ __device__ __noinline__ float batch_sequential_sum(const float *vals, uint32_t b
             for (uint32_t t = 0; t < BATCH_TERMS; t++)
                 acc = __fadd_rn(acc, first + t >= beg && first + t < end ? x[t] : 0.0f);
         }
-        __syncwarp();                                // the slot is free for stage c + BATCH_STAGES
+        __syncwarp();                                // the slot is free for stage c + STAGES
     }
     cp_async_wait<0>();
     return acc;
@@ -1405,14 +1443,14 @@ __device__ __noinline__ float warp_plain_sum(const float *vals, uint32_t n, unsi
 // vals[]) and the fused pull-segmented kernel (terms gathered into the
 // warp's shared-memory buffer).
 constexpr uint32_t PIECE_L = SEG_EDGES / 32;        // terms per lane: one window per piece
-constexpr uint32_t SERIAL_PIECES = SERIAL_TERMS / SEG_EDGES;
-static_assert(SERIAL_TERMS % SEG_EDGES == 0, "the serial start covers whole pieces");
-static_assert(GIANT_ROW >= SERIAL_TERMS, "giant rows go past the serial start");
+constexpr uint32_t START_PIECES = 1;                // a giant row's start: evaluated in order by one warp
+constexpr uint32_t START_TERMS = START_PIECES * SEG_EDGES;
+static_assert(GIANT_LEAST >= START_TERMS && GIANT_LEAST >= LONG_CLASSED, "giant rows hold the serial start");
 // Piece records, two uint4 per piece: r0 = {kind | tg << 8, K | K2 << 8, M1.e, M1.o},
 // r1 = {bits of term tg, M2.e, M2.o, 0}
 constexpr uint32_t REC_NONE = 0;      // evaluated exactly by the combination
 constexpr uint32_t REC_BINADE = 1;    // M1: the piece's terms in binade K
-constexpr uint32_t REC_STATE = 2;     // r0.y: the running sum after the serial start
+constexpr uint32_t REC_STATE = 2;     // r0.y: the running sum after the row's start
 constexpr uint32_t REC_CROSS = 3;     // M1: terms before tg in K; tg crosses into K2; M2: the rest in K2
 
 __device__ __forceinline__ uint32_t atomic_add_acq_rel(uint32_t *p, uint32_t v)
@@ -1422,35 +1460,28 @@ __device__ __forceinline__ uint32_t atomic_add_acq_rel(uint32_t *p, uint32_t v)
     return old;
 }
 
-// The sum of rv[0, SERIAL_TERMS) in row order: coalesced loads of the whole
+// The sum of rv[0, START_TERMS) in row order: coalesced loads of the whole
 // range, then lane 0 adds the terms from shared memory (four per load).
-// `stage` is 16-byte aligned and holds 32 x PIECE_L floats.
+// `stage` is 16-byte aligned and holds START_TERMS floats.
 __device__ __forceinline__ uint32_t warp_serial_start(const float *rv, float *stage, unsigned lane)
 {
-    constexpr uint32_t HALF = 32 * PIECE_L;
-    static_assert(SERIAL_TERMS == 2 * HALF, "the serial start is two stages");
-    float v[2][PIECE_L];
+    float v[START_TERMS / 32];
 #pragma unroll
-    for (uint32_t h = 0; h < 2; h++)
+    for (uint32_t u = 0; u < START_TERMS / 32; u++) v[u] = __ldcg(rv + u * 32 + lane);
 #pragma unroll
-        for (uint32_t u = 0; u < PIECE_L; u++) v[h][u] = __ldcg(rv + h * HALF + u * 32 + lane);
+    for (uint32_t u = 0; u < START_TERMS / 32; u++) stage[u * 32 + lane] = v[u];
+    __syncwarp();
     float acc = 0.0f;
-#pragma unroll
-    for (uint32_t h = 0; h < 2; h++) {
-#pragma unroll
-        for (uint32_t u = 0; u < PIECE_L; u++) stage[u * 32 + lane] = v[h][u];
-        __syncwarp();
-        if (lane == 0) {
-            const float4 *s4 = reinterpret_cast<const float4 *>(stage);
+    if (lane == 0) {
+        const float4 *s4 = reinterpret_cast<const float4 *>(stage);
 #pragma unroll 8
-            for (uint32_t i = 0; i < HALF / 4; i++) {
-                const float4 q = s4[i];
-                acc = __fadd_rn(acc, q.x); acc = __fadd_rn(acc, q.y);
-                acc = __fadd_rn(acc, q.z); acc = __fadd_rn(acc, q.w);
-            }
+        for (uint32_t i = 0; i < START_TERMS / 4; i++) {
+            const float4 q = s4[i];
+            acc = __fadd_rn(acc, q.x); acc = __fadd_rn(acc, q.y);
+            acc = __fadd_rn(acc, q.z); acc = __fadd_rn(acc, q.w);
         }
-        __syncwarp();
     }
+    __syncwarp();
     return __shfl_sync(FULL_MASK, __float_as_uint(acc), 0);
 }
 
@@ -1465,30 +1496,32 @@ __device__ __forceinline__ bwseq::Map warp_compose(bwseq::Map m, unsigned lane)
     return m;
 }
 
-// A lane's PIECE_L maps of terms x in binade K composed as a tree (with
-// skip != ~0, the terms at positions first + u <= skip are replaced by +0,
-// the identity).
-__device__ __forceinline__ bwseq::Map lane_maps(const uint32_t (&x)[PIECE_L], uint32_t K, uint32_t first,
-                                                uint32_t skip, bool &good)
+// The terms of a staged piece: term k is at k + k / 32, so that the lanes'
+// runs of PIECE_L terms are read without bank conflicts.
+__device__ __forceinline__ float staged(const float *stage, uint32_t k) { return stage[k + (k >> 5)]; }
+
+// The map in binade K of a lane's terms first .. first + PIECE_L - 1, those
+// below `from` left out; `worst` takes their largest bit pattern.
+__device__ __forceinline__ bwseq::Map lane_map(const float *stage, uint32_t K, uint32_t first, uint32_t from,
+                                               uint32_t &worst)
 {
     using namespace bwseq;
-    Map t[PIECE_L];
+    Chain c = chain_start(K);
+    worst = 0;
 #pragma unroll
-    for (uint32_t u = 0; u < PIECE_L; u++)
-        t[u] = step_select(skip == 0xffffffffu || first + u > skip ? x[u] : 0u, K, good);
-#pragma unroll
-    for (uint32_t st = 1; st < PIECE_L; st <<= 1) {
-#pragma unroll
-        for (uint32_t u = 0; u + st < PIECE_L; u += 2 * st) t[u] = compose_short(t[u], t[u + st]);
+    for (uint32_t u = 0; u < PIECE_L; u++) {
+        const float x = first + u >= from ? staged(stage, first + u) : 0.0f;
+        worst = max(worst, __float_as_uint(x));
+        chain_add(c, x);
     }
-    return saturated(t[0]);
+    return chain_map(c, K);
 }
 
-// The record of a piece's terms under the guessed running sum `guess` at
-// its start (valid in lane 0): lane l holds the piece's terms l * PIECE_L
-// .. l * PIECE_L + PIECE_L - 1 (past the piece's end: +0, the identity).
+// The record of a staged piece (past the piece's end: +0, the identity) under
+// the guessed running sum `guess` at its start (valid in lane 0): lane l
+// holds the piece's terms l * PIECE_L .. l * PIECE_L + PIECE_L - 1.
 // REC_NONE when the guess or a term is outside the maps' domain.
-__device__ __forceinline__ void record_of_terms(const uint32_t (&x)[PIECE_L], uint32_t guess, unsigned lane,
+__device__ __forceinline__ void record_of_terms(const float *stage, uint32_t guess, unsigned lane,
                                                 uint4 &r0, uint4 &r1)
 {
     using namespace bwseq;
@@ -1496,9 +1529,9 @@ __device__ __forceinline__ void record_of_terms(const uint32_t (&x)[PIECE_L], ui
     r1 = make_uint4(0u, 0u, 0u, 0u);
     if (!in_domain(guess)) return;
     const uint32_t K = exponent_of(guess), first = lane * PIECE_L;
-    bool good = true;
-    const Map m = lane_maps(x, K, first, 0xffffffffu, good);
-    if (__any_sync(FULL_MASK, !good)) return;
+    uint32_t worst;
+    const Map m = lane_map(stage, K, first, 0u, worst);
+    if (__any_sync(FULL_MASK, worst > CHAIN_TERM_MAX)) return;
     Map incl = m;                                     // lanes' maps scanned
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1513,30 +1546,25 @@ __device__ __forceinline__ void record_of_terms(const uint32_t (&x)[PIECE_L], ui
         r0 = make_uint4(REC_BINADE, K, __shfl_sync(FULL_MASK, incl.e, 31), __shfl_sync(FULL_MASK, incl.o, 31));
         return;
     }
-    // the guessed crossing: the first lane whose run leaves the binade finds the term
+    // the guessed crossing: the first lane whose run leaves the binade finds
+    // the term, with the map of its terms before it
     const unsigned f = __ffs(cross) - 1;
     uint32_t tg = 0, xb = 0, nb = 0;
     Map pm = identity();
     if (lane == f) {
-        uint32_t acc = a0;
-        bool found = false;
-#pragma unroll
+        Chain before = chain_start(K);
+        float acc = __uint_as_float(bits_of(K, a0));
+#pragma unroll 1
         for (uint32_t u = 0; u < PIECE_L; u++) {
-            if (!found) {
-                Map st;
-                step(x[u], K, st);
-                const uint32_t bu = apply(st, acc);
-                if (bu >= TOP) {
-                    found = true;
-                    tg = first + u;
-                    xb = x[u];
-                    nb = __float_as_uint(__fadd_rn(__uint_as_float(bits_of(K, acc)), __uint_as_float(x[u])));
-                } else {
-                    acc = bu;
-                    pm = compose(pm, st);
-                }
-            }
+            const float x = staged(stage, first + u);
+            acc = __fadd_rn(acc, x);
+            nb = __float_as_uint(acc);
+            tg = first + u;
+            xb = __float_as_uint(x);
+            if (exponent_of(nb) != K) break;
+            chain_add(before, x);
         }
+        pm = chain_map(before, K);
     }
     tg = __shfl_sync(FULL_MASK, tg, f);
     xb = __shfl_sync(FULL_MASK, xb, f);
@@ -1545,24 +1573,21 @@ __device__ __forceinline__ void record_of_terms(const uint32_t (&x)[PIECE_L], ui
                            Map{__shfl_sync(FULL_MASK, pm.e, f), __shfl_sync(FULL_MASK, pm.o, f)});
     if (!in_domain(nb)) return;
     const uint32_t K2 = exponent_of(nb);
-    const Map m2 = warp_compose(lane_maps(x, K2, first, tg, good), lane);   // the terms after tg
+    const Map m2 = warp_compose(lane_map(stage, K2, first, tg + 1, worst), lane);   // the terms after tg
     r0 = make_uint4(REC_CROSS | (tg << 8), K | (K2 << 8), m1.e, m1.o);
     r1 = make_uint4(xb, m2.e, m2.o, 0u);
 }
 
-// The record of piece q >= SERIAL_PIECES of a giant row (valid in lane 0).
-__device__ __forceinline__ void piece_record(const PrArgs &a, const float *rv, uint32_t n, uint32_t p0, uint32_t q,
+// The record of a giant row's piece q >= START_PIECES, the terms
+// tv[0, len) (valid in lane 0); p0: the row's first piece.
+__device__ __forceinline__ void piece_record(const PrArgs &a, const float *tv, uint32_t len, uint32_t p0, uint32_t q,
                                              float *stage, unsigned lane, uint4 &r0, uint4 &r1)
 {
-    using namespace bwseq;
-    r0 = make_uint4(REC_NONE, 0u, 0u, 0u);
-    r1 = make_uint4(0u, 0u, 0u, 0u);
-    const uint32_t b = q * SEG_EDGES, len = min(SEG_EDGES, n - b);
     float v[PIECE_L];                                // the terms, coalesced (issued first)
 #pragma unroll
     for (uint32_t u = 0; u < PIECE_L; u++) {
         const uint32_t k = u * 32 + lane;
-        v[u] = k < len ? __ldcg(rv + b + k) : 0.0f;
+        v[u] = k < len ? __ldcg(tv + k) : 0.0f;
     }
     // The guess: the earlier pieces' sums added in float.  Its error (a few
     // ulps) is far below the sequential sum's own drift from the exact sum,
@@ -1571,6 +1596,7 @@ __device__ __forceinline__ void piece_record(const PrArgs &a, const float *rv, u
     // is narrow, and every piece adds all the sums before it.)
     constexpr uint32_t PRE_U = 4;
     float pre = 0.0f;
+#pragma unroll 1
     for (uint32_t i0 = 0; i0 < q; i0 += 32 * PRE_U) {
         float f[PRE_U];
 #pragma unroll
@@ -1583,19 +1609,11 @@ __device__ __forceinline__ void piece_record(const PrArgs &a, const float *rv, u
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pre += __shfl_xor_sync(FULL_MASK, pre, o);   // same bits in every lane
-    // restage so that lane l holds terms l*PIECE_L .. (element k at k + k / 32)
 #pragma unroll
     for (uint32_t u = 0; u < PIECE_L; u++) stage[u * 33 + lane] = v[u];
     __syncwarp();
-    uint32_t x[PIECE_L];
-#pragma unroll
-    for (uint32_t u = 0; u < PIECE_L; u++) {
-        const uint32_t k = lane * PIECE_L + u;
-        x[u] = __float_as_uint(stage[k + (k >> 5)]);   // past the end: +0, the identity
-    }
-    __syncwarp();
-    const uint32_t guess = __float_as_uint(pre);
-    record_of_terms(x, guess, lane, r0, r1);
+    record_of_terms(stage, __float_as_uint(pre), lane, r0, r1);
+    __syncwarp();                                    // the stage is free for the next job
 }
 
 // The exact evaluation of piece q from the running sum `sb` (rare: kept
@@ -1624,11 +1642,10 @@ __device__ __forceinline__ bool piece_advance(uint32_t q, const uint4 &r0, const
             sb = bits_of(K, a1);
             return true;
         }
-        Map st;
-        if (kind == REC_CROSS && a1 < TOP && step(r1.x, K, st) && apply(st, a1) >= TOP) {
+        if (kind == REC_CROSS && a1 < TOP) {
             const uint32_t nb = __float_as_uint(__fadd_rn(__uint_as_float(bits_of(K, a1)), __uint_as_float(r1.x)));
             const uint32_t K2 = (r0.y >> 8) & 0xffu;
-            if (in_domain(nb) && exponent_of(nb) == K2) {
+            if (in_domain(nb) && exponent_of(nb) == K2) {          // K2 > K: the term crosses here too
                 const uint32_t a3 = apply(Map{r1.y, r1.z}, significand_of(nb));
                 if (a3 < TOP) {
                     sb = bits_of(K2, a3);
@@ -1692,7 +1709,7 @@ __device__ __forceinline__ float combine_records(const uint4 *rec, uint32_t firs
 __device__ __forceinline__ float combine_pieces(const PrArgs &a, const float *rv, uint32_t n, uint32_t p0,
                                                 uint32_t pieces, float *stage, unsigned lane)
 {
-    return combine_records(a.piece_map + 2 * static_cast<uint64_t>(p0), SERIAL_PIECES, pieces, lane,
+    return combine_records(a.piece_map + 2 * static_cast<uint64_t>(p0), START_PIECES, pieces, lane,
                            [&](uint32_t q, uint32_t sb) { return piece_exact(rv, n, q, sb, stage, lane); },
                            [&]() { return warp_plain_sum(rv, n, lane); });
 }
@@ -1802,7 +1819,7 @@ __global__ void __launch_bounds__(BLOCK, pull_min_blocks(BLOCK)) k_pr_pull_items
         }
         __syncwarp();
     }
-    add_diff(a.diff, dsum);
+    add_diff_block(a.diff, dsum, smem_f);
 }
 
 // Long-row sums of the exact variants (vertex-pull, vertex-pull-nodiv),
@@ -1810,47 +1827,54 @@ __global__ void __launch_bounds__(BLOCK, pull_min_blocks(BLOCK)) k_pr_pull_items
 // in vals[] (edge order) and every piece's float sum in piece_sum[].  Jobs
 // are taken in order from a counter (no static share, so a warp that drew a
 // long job takes fewer):
-//  * first batches of 32 long rows of at most GIANT_ROW terms and similar
+//  * first batches of 32 long rows below giant_row(m) terms and of similar
 //    length, one row per lane (batch_sequential_sum): the longest chains of
 //    dependent additions start first.
-//  * then the pieces of the rows above GIANT_ROW terms, longest rows
-//    first.  Piece 0 adds the row's first SERIAL_TERMS terms in order (one
-//    lane, from shared memory).  Every later piece guesses the running sum at its start (the
-//    float sums of the pieces before it, added in float) and records, in
-//    the guessed binade, the map of its terms -- or, when the guess crosses
-//    into the next binade inside the piece, the map of the terms before the
-//    crossing term, that term, and the map of the terms after it in the new
-//    binade.  The row's last piece to finish combines the records in order,
-//    scanning runs of map records with the warp: a record that holds for
-//    the true running sum (same binade, crossing where recorded) is applied,
-//    any other piece is evaluated exactly from the true running sum
-//    (warp_sequential_continue).  The guesses only decide how much work the
-//    combination does, never its result.
+//  * then the pieces of the giant rows, longest rows first.  Piece 0 adds the
+//    row's first START_TERMS terms in order (one lane, from shared memory).
+//    Every later piece guesses the running sum at its start (the float sums
+//    of the pieces before it, added in float) and records, in the guessed
+//    binade, the map of its terms -- or, when the guess crosses into the next
+//    binade inside the piece, the map of the terms before the crossing term,
+//    that term, and the map of the terms after it in the new binade.  A map
+//    comes from two chains of float additions (bw_seqsum.h, Chain).  The row's
+//    last piece to finish combines the records in order, scanning runs of map
+//    records with the warp: a record that holds for the true running sum (same
+//    binade, crossing where recorded) is applied, any other piece is evaluated
+//    exactly from the true running sum (warp_sequential_continue).  The
+//    guesses only decide how much work the combination does, never its result.
+// Bound by the latency of each job's loads and arrival.  With term-by-term
+// maps (about 500 instructions a lane and piece, the first 1024 terms serial)
+// warps also waited for instructions: on R-MAT-22 35.2M warp instructions and
+// 90 us a launch, with the chains 20.6M and 61 us.  Taking the next job while
+// one is worked on made it slower (the claimed job waits for a long one:
+// R-MAT-20 115 -> 151 us an iteration).
 // Every sum is the reference's sequential loop, bit-identical.  The last
 // warp to finish resets the job counters for the next iteration; each
 // giant row's combining piece resets the row's arrival counter.
 constexpr int LONG_SUM_THREADS = 256;
-constexpr int LONG_SUM_BLOCKS_PER_SM = 2;            // registers <= 128
-constexpr uint32_t LONG_SUM_WARP_SMEM = BATCH_RING > 33 * PIECE_L ? BATCH_RING : 33 * PIECE_L;   // floats
-constexpr size_t LONG_SUM_SMEM = (LONG_SUM_THREADS / 32) * LONG_SUM_WARP_SMEM * sizeof(float);
-template<bool NODIV, bool MULTI = false>
-__global__ void __launch_bounds__(LONG_SUM_THREADS, LONG_SUM_BLOCKS_PER_SM) k_pr_long_sums(PrArgs a, uint32_t *ctr)
+__host__ __device__ constexpr uint32_t long_sum_warp_smem(uint32_t stages)       // floats
+{
+    return batch_ring(stages) > 33 * PIECE_L ? batch_ring(stages) : 33 * PIECE_L;
+}
+constexpr size_t long_sum_smem(uint32_t stages) { return (LONG_SUM_THREADS / 32) * long_sum_warp_smem(stages) * sizeof(float); }
+template<bool NODIV, bool MULTI, uint32_t STAGES, int BLOCKS>
+__global__ void __launch_bounds__(LONG_SUM_THREADS, BLOCKS) k_pr_long_sums(PrArgs a, uint32_t *ctr)
 {
     extern __shared__ __align__(16) float long_smem[];   // per warp: the batch ring or a piece's stage
     resolve_args(a);
     const unsigned lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    float *const ring = long_smem + wib * LONG_SUM_WARP_SMEM;
-    float *const stage_w = ring;
+    float *const ring = long_smem + wib * long_sum_warp_smem(STAGES);
     const uint32_t L = *a.long_total, G = *a.giant_total, PG = *a.giant_pieces;
-    const uint32_t MB = (L - G + 31) / 32;
-    const uint32_t jobs = MB + PG;
+    const uint32_t MB = (L - G + 31) / 32, jobs = MB + PG;
     const float base_nd = nodiv_base(a.n);
     float dsum = 0.0f;
-    for (;;) {
-        uint32_t job = 0;
-        if (lane == 0) job = atomicAdd(&ctr[0], 1u);
-        job = __shfl_sync(FULL_MASK, job, 0);
-        if (job >= jobs) break;
+    if (!MULTI && jobs == 0) return;                  // (the counters are as they were)
+    // each warp's first job is its number, block after block within a job
+    // index, so that the first and longest ones go to different SMs
+    const uint32_t warps = gridDim.x * (blockDim.x / 32);
+    uint32_t job = wib * gridDim.x + blockIdx.x;
+    while (job < jobs) {
         if (job < MB) {
             const uint32_t k = G + job * 32 + lane;
             uint32_t row = 0, beg = 0, len = 0;
@@ -1861,29 +1885,30 @@ __global__ void __launch_bounds__(LONG_SUM_THREADS, LONG_SUM_BLOCKS_PER_SM) k_pr
                 beg = a.rev_v[row];
                 len = a.rev_v[row + 1] - beg;
             }
-            const float sum = batch_sequential_sum(a.vals, beg, len, ring, lane);
+            const float sum = batch_sequential_sum<STAGES>(a.vals, beg, len, ring, lane);
             if (k < L) dsum += finish_row<NODIV, MULTI>(a, row, sum, base_nd, fin, MULTI ? graph_of(a, row) : 0u);
         } else {
-            job -= MB;
-            const uint4 w = a.work[job];
-            const uint32_t row = w.x, beg = a.rev_v[row], n = a.rev_v[row + 1] - beg;
-            const uint32_t q = (w.z - beg) / SEG_EDGES, pieces = (n + SEG_EDGES - 1) / SEG_EDGES, p0 = job - q;
+            const uint32_t at = job - MB;
+            const uint4 w = a.work[at];
+            const uint32_t row = w.x, q = w.y & ROW_MASK, p0 = at - q;
+            const uint32_t beg = w.z - q * SEG_EDGES, n = a.rev_v[row + 1] - beg;
+            const uint32_t pieces = (n + SEG_EDGES - 1) / SEG_EDGES;
             const float *rv = a.vals + beg;
             uint4 r0 = make_uint4(REC_NONE, 0u, 0u, 0u), r1 = make_uint4(0u, 0u, 0u, 0u);
             if (q == 0) {
-                r0 = make_uint4(REC_STATE, warp_serial_start(rv, stage_w, lane), 0u, 0u);
-            } else if (q >= SERIAL_PIECES) {
-                piece_record(a, rv, n, p0, q, stage_w, lane, r0, r1);
+                r0 = make_uint4(REC_STATE, warp_serial_start(rv, ring, lane), 0u, 0u);
+            } else if (q >= START_PIECES) {
+                piece_record(a, a.vals + w.z, w.w - w.z, p0, q, ring, lane, r0, r1);
             }
             uint32_t last = 0;
             if (lane == 0) {
-                a.piece_map[2 * static_cast<uint64_t>(job)] = r0;
-                a.piece_map[2 * static_cast<uint64_t>(job) + 1] = r1;
+                a.piece_map[2 * static_cast<uint64_t>(at)] = r0;
+                a.piece_map[2 * static_cast<uint64_t>(at) + 1] = r1;
                 last = atomic_add_acq_rel(&a.long_count[row], 1u) + 1 == pieces ? 1u : 0u;
             }
             if (__shfl_sync(FULL_MASK, last, 0)) {
                 __syncwarp();                         // orders every lane's reads after lane 0's acquire
-                const float total = combine_pieces(a, rv, n, p0, pieces, stage_w, lane);
+                const float total = combine_pieces(a, rv, n, p0, pieces, ring, lane);
                 if (lane == 0) {
                     dsum += finish_row<NODIV, MULTI>(a, row, total, base_nd, finish_load<NODIV>(a, row),
                                                      MULTI ? graph_of(a, row) : 0u);
@@ -1891,16 +1916,15 @@ __global__ void __launch_bounds__(LONG_SUM_THREADS, LONG_SUM_BLOCKS_PER_SM) k_pr
                 }
             }
         }
+        if (lane == 0) job = warps + atomicAdd(&ctr[0], 1u);
+        job = __shfl_sync(FULL_MASK, job, 0);
     }
-    add_diff(a.diff, dsum);
-    // the last warp out resets the job counter
-    if (lane == 0) {
-        const uint32_t warps = gridDim.x * (blockDim.x / 32);
-        if (atomicAdd(&ctr[1], 1u) + 1 == warps) {
-            ctr[0] = 0;
-            ctr[1] = 0;
-            ctr[2] = 0;                               // k_pr_pull_items' chunks (packed graphs)
-        }
+    add_diff_block(a.diff, dsum, long_smem);
+    // the last block out resets the job counter
+    if (threadIdx.x == 0 && atomicAdd(&ctr[1], 1u) + 1 == gridDim.x) {
+        ctr[0] = 0;
+        ctr[1] = 0;
+        ctr[2] = 0;                                   // k_pr_pull_items' chunks (packed graphs)
     }
 }
 
@@ -1961,7 +1985,7 @@ struct PrRun {
     uint32_t *rows = nullptr;          // rows with in-edges, then rows without
     uint32_t *long_rows = nullptr;     // long rows by decreasing length
     uint32_t *long_total = nullptr;    // device: number of long rows
-    uint32_t *giant_total = nullptr;   // device: how many of them exceed GIANT_ROW
+    uint32_t *giant_total = nullptr;   // device: how many of them are giant rows
     uint32_t *giant_pieces = nullptr;  // device: the pieces of those
     float *piece_sum = nullptr;        // exact pieces: their float sums
     uint4 *piece_map = nullptr;        // giant-row pieces: records (two uint4 each)
@@ -2118,7 +2142,8 @@ int build_segments(bw_context *ctx, const bw_graph_view *g, uint32_t seg_long, P
     if (packed) BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&run.sorted),
                                          (m / SEG_EDGES + lcap + 1) * sizeof(uint4), s));
     k_piece_emit<<<grid, 256, 0, s>>>(g->rev_vertices, run.long_rows, long_len, run.long_total, ppos,
-                                      packed ? run.sorted : run.work, run.long_count, run.giant_total, run.giant_pieces);
+                                      packed ? run.sorted : run.work, run.long_count, run.giant_total, run.giant_pieces,
+                                      giant_row(m));
     if (packed) {
         k_piece_count<<<grid, 256, 0, s>>>(S + o_lkey0, run.long_total, lcap, pcnt);
         BW_CUDA(sortk::scan_exclusive(pcnt, S + o_npos, lcap + 1, part, s));
@@ -2166,10 +2191,20 @@ void free_run(PrRun &run, cudaStream_t s)
 }
 
 // The long-row sums of one iteration of the work-list variants.
-template<bool NODIV>
+template<bool NODIV, bool MULTI, uint32_t STAGES, int BLOCKS>
+void launch_long_sums_as(const bw_context *ctx, const PrArgs &a, cudaStream_t s)
+{
+    constexpr size_t smem = long_sum_smem(STAGES);
+    auto k = k_pr_long_sums<NODIV, MULTI, STAGES, BLOCKS>;
+    // (no-op after the first call; a failure leaves the launch to report it)
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    k<<<ctx->sm_count * BLOCKS, LONG_SUM_THREADS, smem, s>>>(a, a.sum_ctr);
+}
+template<bool NODIV, bool MULTI = false>
 void launch_long_sums(const bw_context *ctx, const PrArgs &a, cudaStream_t s)
 {
-    k_pr_long_sums<NODIV><<<ctx->sm_count * LONG_SUM_BLOCKS_PER_SM, LONG_SUM_THREADS, LONG_SUM_SMEM, s>>>(a, a.sum_ctr);
+    if (a.m < SUM_SMALL_EDGES) launch_long_sums_as<NODIV, MULTI, SUM_STAGES_SMALL, SUM_BLOCKS_SMALL>(ctx, a, s);
+    else launch_long_sums_as<NODIV, MULTI, SUM_STAGES, SUM_BLOCKS>(ctx, a, s);
 }
 
 // The work-list kernel of the div variants; the first iteration's instance
@@ -2421,10 +2456,6 @@ int run_pagerank(bw_context *ctx, const bw_graph_view *g, const int32_t *schedul
     a.acc = ctx->pr_acc;
     a.gat_e = g->rev_edges;
     if (need_exact) {
-        BW_CUDA(cudaFuncSetAttribute(k_pr_long_sums<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(LONG_SUM_SMEM)));
-        BW_CUDA(cudaFuncSetAttribute(k_pr_long_sums<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(LONG_SUM_SMEM)));
         // hub cache entries per block: chunk_size when given, else the
         // default for the shape; never more than the block's share of
         // shared memory allows
@@ -2742,8 +2773,6 @@ int bw::pagerank_run_packed(bw_context *ctx, const bw_graph_view *g, const uint3
     a.diff = ctx->pr_diffs;
     constexpr size_t smem = pull_fixed_smem(PULL_WIDE);
     auto body = [&]() -> int {
-        BW_CUDA(cudaFuncSetAttribute(k_pr_long_sums<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(LONG_SUM_SMEM)));
         BW_CUDA(cudaFuncSetAttribute(k_pr_pull_items<false, PULL_WIDE, false, true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         k_row_lengths<<<ctx->sm_count * 4, 256, 0, s>>>(g->fwd_vertices, n, ctx->pr_deg);
@@ -2757,7 +2786,7 @@ int bw::pagerank_run_packed(bw_context *ctx, const bw_graph_view *g, const uint3
             k_pr_pull_items<false, PULL_WIDE, false, true><<<ctx->sm_count, PULL_WIDE, smem, s>>>(a);
             PrArgs b = a;
             b.work = run.sorted;
-            k_pr_long_sums<false, true><<<ctx->sm_count * LONG_SUM_BLOCKS_PER_SM, LONG_SUM_THREADS, LONG_SUM_SMEM, s>>>(b, b.sum_ctr);
+            launch_long_sums<false, true>(ctx, b, s);
         }
         BW_CUDA(cudaGetLastError());
         return BW_OK;
