@@ -183,7 +183,8 @@ __device__ __forceinline__ void add_diff(float *slot, float d)
 }
 
 // The same with one atomic per block: thousands of warps' float atomics on
-// one word are a microsecond or two of a launch, and each rounds the sum.
+// one word serialise, and each rounds the sum (k_consolidate_div of 1M
+// vertices on GB300: 9,728 of them, 20 us, of which 12 after the last row).
 // Every thread calls; `scratch`: 32 floats of shared memory that nothing else
 // uses from here on.
 __device__ __forceinline__ void add_diff_block(float *slot, float d, float *scratch)
@@ -194,6 +195,11 @@ __device__ __forceinline__ void add_diff_block(float *slot, float d, float *scra
     if (lane == 0) scratch[wib] = d;
     __syncthreads();
     if (wib == 0) add_diff(slot, lane < blockDim.x / 32 ? scratch[lane] : 0.0f);
+}
+__device__ __forceinline__ void add_diff_block(float *slot, float d)
+{
+    __shared__ float scratch[32];
+    add_diff_block(slot, d, scratch);
 }
 
 // ----------------------------- degrees ------------------------------------
@@ -380,44 +386,106 @@ __global__ void __launch_bounds__(256) k_consolidate_div(PrArgs a, int rowlen)
             a.contrib_out[v] = d ? __fdiv_rn(nr, static_cast<float>(d)) : 0.0f;
         }
     }
-    add_diff(a.diff, dsum);
+    add_diff_block(a.diff, dsum);
 }
 
 // ----------------------- edge-list families -------------------------------
 // acc[dst] += contrib[src] per edge (pagerank/edgelist.cu:14-22 and the
 // rev/struct forms).  Forward layouts (source-sorted) scatter with one
-// float atomic per edge.  The reverse SoA layout is destination-sorted:
-// each warp step reduces runs of equal destinations with a segmented
-// shuffle scan and issues one atomic per run.
-template<int LAYOUT>  // 0 fwd SoA, 1 rev SoA, 2 fwd AoS, 3 rev AoS
+// float atomic per edge.
+template<int LAYOUT>  // 0 fwd SoA, 2 fwd AoS
 __global__ void __launch_bounds__(256) k_pr_edge(PrArgs a)
 {
-    const unsigned lane = threadIdx.x & 31;
-    const uint64_t warp = gtid() >> 5, warps = gthreads() >> 5;
     const uint64_t m = a.m;
-    for (uint64_t base = warp * 32; base < m; base += warps * 32) {
-        const uint64_t e = base + lane;
-        uint32_t src = 0, dst = 0xffffffffu;
-        if (e < m) {
-            if constexpr (LAYOUT == 0) { src = __ldcs(a.fwd_in + e); dst = __ldcs(a.fwd_e + e); }
-            else if constexpr (LAYOUT == 1) { dst = __ldcs(a.rev_in + e); src = __ldcs(a.rev_e + e); }
-            else if constexpr (LAYOUT == 2) { const uint2 p = __ldcs(a.fwd_s + e); src = p.x; dst = p.y; }
-            else { const uint2 p = __ldcs(a.rev_s + e); dst = p.x; src = p.y; }
-        }
-        float val = e < m ? __ldg(a.contrib_in + src) : 0.0f;
-        if constexpr (LAYOUT == 1 || LAYOUT == 3) {
-            // segmented suffix sums over runs of equal dst (sorted)
-            for (int o = 1; o < 32; o <<= 1) {
-                const float y = __shfl_down_sync(FULL_MASK, val, o);
-                const uint32_t k = __shfl_down_sync(FULL_MASK, dst, o);
-                if (lane + o < 32 && k == dst) val += y;
+    for (uint64_t e = gtid(); e < m; e += gthreads()) {
+        uint32_t src, dst;
+        if constexpr (LAYOUT == 0) { src = __ldcs(a.fwd_in + e); dst = __ldcs(a.fwd_e + e); }
+        else { const uint2 p = __ldcs(a.fwd_s + e); src = p.x; dst = p.y; }
+        atomicAdd(&a.acc[dst], __ldg(a.contrib_in + src));
+    }
+}
+
+// The reverse layouts are destination-sorted: a lane takes four consecutive
+// edges, U times in flight, and adds equal destinations in registers.  Runs
+// that lie inside a lane are complete; the lanes' first and last runs are
+// joined by one segmented scan per 128 edges, and every run ends in one
+// atomic.  Bound by the gathers (one L1TEX tag each: 76% of peak on 16M edges
+// of R-MAT, 49 us); an edge per lane and a scan per 32 edges took 60 us there,
+// ER(4M, 67M) 337 -> 287 us an iteration, the grid 2048^2 84 -> 58.  U = 2 only
+// where it has work for every warp: R-MAT-22 272 -> 262 us, but R-MAT-14 263
+// -> 320 us for 30 iterations.
+constexpr uint64_t RUN_WIDE_EDGES = uint64_t(24) << 20;
+constexpr uint32_t NO_DST = 0xffffffffu;      // past the last edge (N <= 2^32 - 1)
+
+// k, v: the lane's four destinations (ascending runs over the warp) and values.
+__device__ __forceinline__ void add_runs(float *acc, const uint4 &k, const float4 &v, unsigned lane)
+{
+    const bool b1 = k.y != k.x, b2 = k.z != k.y, b3 = k.w != k.z, single = !b1 && !b2 && !b3;
+    // the first run's and the last run's sums (the same run if `single`)
+    const float head = b1 ? v.x : b2 ? v.x + v.y : v.x + v.y + v.z;
+    float tail = b3 ? v.w : b2 ? v.z + v.w : b1 ? v.y + v.z + v.w : v.x + v.y + v.z + v.w;
+    if (b1 && (b2 || b3)) {                                 // runs in between: y, y and z, or y then z
+        if (b2) atomicAdd(acc + k.y, v.y);
+        else atomicAdd(acc + k.y, v.y + v.z);
+    }
+    if (b2 && b3) atomicAdd(acc + k.z, v.z);
+    // tail: the running sum of the last run since the warp's first edge
+    const uint32_t before = __shfl_up_sync(FULL_MASK, k.w, 1), after = __shfl_down_sync(FULL_MASK, k.x, 1);
+    const bool joins = lane > 0 && before == k.x;
+    const unsigned starts = __ballot_sync(FULL_MASK, !(single && joins));
+    const int from = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float y = __shfl_up_sync(FULL_MASK, tail, o);
+        if (static_cast<int>(lane) - o >= from) tail += y;
+    }
+    const float carry = __shfl_up_sync(FULL_MASK, tail, 1);
+    if (!single && k.x != NO_DST) atomicAdd(acc + k.x, joins ? carry + head : head);
+    if ((lane == 31 || after != k.w) && k.w != NO_DST) atomicAdd(acc + k.w, tail);
+}
+
+template<bool AOS, int U>
+__global__ void __launch_bounds__(256) k_pr_edge_runs(PrArgs a)
+{
+    const unsigned lane = threadIdx.x & 31;
+    const uint64_t warp = gtid() >> 5, warps = gthreads() >> 5, m = a.m;
+    const bool wide = AOS ? (reinterpret_cast<uintptr_t>(a.rev_s) & 15) == 0
+                          : ((reinterpret_cast<uintptr_t>(a.rev_in) | reinterpret_cast<uintptr_t>(a.rev_e)) & 15) == 0;
+    for (uint64_t base = warp * (128 * U); base < m; base += warps * (128 * U)) {
+        uint4 dst[U], src[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint64_t e = base + u * 128 + 4 * lane;
+            if (wide && e + 4 <= m) {
+                if constexpr (AOS) {
+                    const uint4 *p = reinterpret_cast<const uint4 *>(a.rev_s + e);
+                    const uint4 p0 = __ldcs(p), p1 = __ldcs(p + 1);
+                    dst[u] = make_uint4(p0.x, p0.z, p1.x, p1.z);
+                    src[u] = make_uint4(p0.y, p0.w, p1.y, p1.w);
+                } else {
+                    dst[u] = __ldcs(reinterpret_cast<const uint4 *>(a.rev_in + e));
+                    src[u] = __ldcs(reinterpret_cast<const uint4 *>(a.rev_e + e));
+                }
+            } else {
+                auto edge = [&](uint64_t i) {
+                    if (i >= m) return make_uint2(NO_DST, 0u);
+                    return AOS ? __ldcs(a.rev_s + i) : make_uint2(__ldcs(a.rev_in + i), __ldcs(a.rev_e + i));
+                };
+                const uint2 e0 = edge(e), e1 = edge(e + 1), e2 = edge(e + 2), e3 = edge(e + 3);
+                dst[u] = make_uint4(e0.x, e1.x, e2.x, e3.x);
+                src[u] = make_uint4(e0.y, e1.y, e2.y, e3.y);
             }
-            const uint32_t prev = __shfl_up_sync(FULL_MASK, dst, 1);
-            const bool head = lane == 0 || prev != dst;
-            if (e < m && head) atomicAdd(&a.acc[dst], val);
-        } else {
-            if (e < m) atomicAdd(&a.acc[dst], val);
         }
+        float4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            v[u].x = dst[u].x != NO_DST ? __ldg(a.contrib_in + src[u].x) : 0.0f;
+            v[u].y = dst[u].y != NO_DST ? __ldg(a.contrib_in + src[u].y) : 0.0f;
+            v[u].z = dst[u].z != NO_DST ? __ldg(a.contrib_in + src[u].z) : 0.0f;
+            v[u].w = dst[u].w != NO_DST ? __ldg(a.contrib_in + src[u].w) : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) add_runs(a.acc, dst[u], v[u], lane);
     }
 }
 
@@ -772,7 +840,7 @@ __global__ void __launch_bounds__(512) k_pr_vertex_pull_warp(PrArgs a)
         for (uint32_t i = lane; i < cnt; i += W) dsum += finish_vertex<NODIV>(a, v0 + i, my_acc[i], base_nd);
         __syncwarp(mask);
     }
-    add_diff(a.diff, dsum);
+    add_diff_block(a.diff, dsum);
 }
 
 // Tiles of the heavy units queued by this iteration's first kernel
@@ -890,7 +958,7 @@ __global__ void __launch_bounds__(256) k_pr_heavy_finish(PrArgs a)
             dsum += finish_vertex<NODIV>(a, v0 + i, sum, base_nd);
         }
     }
-    add_diff(a.diff, dsum);
+    add_diff_block(a.diff, dsum);
     if (lane == 0 && atomicAdd(&a.heavy_ctr[4], 1u) + 1 == warps) {
         a.heavy_ctr[3] = 0;
         a.heavy_ctr[4] = 0;
@@ -2228,12 +2296,18 @@ int launch_iteration(bw_context *ctx, int variant, PrArgs &a, const Geometry &ge
         if (a.hot_dst) k_pr_edge_hot<0><<<ctx->sm_count * 2, HOT_THREADS, HOT_SLOTS * sizeof(float), s>>>(a);
         else k_pr_edge<0><<<geo.grid, geo.block, 0, s>>>(a);
         break;
-      case PR_REV_EDGE_LIST: k_pr_edge<1><<<geo.grid, geo.block, 0, s>>>(a); break;
+      case PR_REV_EDGE_LIST:
+        if (a.m < RUN_WIDE_EDGES) k_pr_edge_runs<false, 1><<<geo.grid, geo.block, 0, s>>>(a);
+        else k_pr_edge_runs<false, 2><<<geo.grid, geo.block, 0, s>>>(a);
+        break;
       case PR_STRUCT_EDGE_LIST:
         if (a.hot_pairs) k_pr_edge_hot<2><<<ctx->sm_count * 2, HOT_THREADS, HOT_SLOTS * sizeof(float), s>>>(a);
         else k_pr_edge<2><<<geo.grid, geo.block, 0, s>>>(a);
         break;
-      case PR_REV_STRUCT_EDGE_LIST: k_pr_edge<3><<<geo.grid, geo.block, 0, s>>>(a); break;
+      case PR_REV_STRUCT_EDGE_LIST:
+        if (a.m < RUN_WIDE_EDGES) k_pr_edge_runs<true, 1><<<geo.grid, geo.block, 0, s>>>(a);
+        else k_pr_edge_runs<true, 2><<<geo.grid, geo.block, 0, s>>>(a);
+        break;
       case PR_VERTEX_PUSH:
         k_pr_vertex_push<<<geo.grid, geo.block, 0, s>>>(a);
         k_pr_heavy_tiles<0><<<ctx->sm_count * 4, 256, 0, s>>>(a);
