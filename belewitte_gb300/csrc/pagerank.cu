@@ -184,7 +184,7 @@ __device__ __forceinline__ void add_diff(float *slot, float d)
 
 // The same with one atomic per block: thousands of warps' float atomics on
 // one word serialise, and each rounds the sum (k_consolidate_div of 1M
-// vertices on GB300: 9,728 of them, 20 us, of which 12 after the last row).
+// vertices on GB300: 9,728 of them, 20 us, more than half after the last row).
 // Every thread calls; `scratch`: 32 floats of shared memory that nothing else
 // uses from here on.
 __device__ __forceinline__ void add_diff_block(float *slot, float d, float *scratch)
@@ -370,21 +370,43 @@ __global__ void __launch_bounds__(256) k_relabel_edges(const uint32_t *__restric
 
 // consolidateRank (div) for the atomic variants; also produces the next
 // contributions and clears the accumulator (pagerank/pagerank.cu:125-140).
+// A thread takes four vertices with 16-byte accesses where the arrays allow
+// it and there are more vertices than threads (16K vertices, 30 iterations:
+// 1.5 us each longer with four vertices a thread).
+__device__ __forceinline__ float consolidate_vertex(const PrArgs &a, float acc, float prev, uint32_t d, float &dsum,
+                                                    float &contrib)
+{
+    const float nr = consolidate_div(acc, a.base_div);
+    dsum += fabsf(nr - prev);
+    contrib = d ? __fdiv_rn(nr, static_cast<float>(d)) : 0.0f;
+    return nr;
+}
 __global__ void __launch_bounds__(256) k_consolidate_div(PrArgs a, int rowlen)
 {
     float dsum = 0.0f;
     const uint64_t n = a.n;
-    for (uint64_t base = (gtid() >> 5) * 32; base < n; base += (gthreads() >> 5) * 32) {
-        const uint64_t v = base + (threadIdx.x & 31);
-        if (v < n) {
-            const float acc = a.acc[v], prev = a.pr_out[v];
-            const uint32_t d = rowlen ? a.fwd_v[v + 1] - a.fwd_v[v] : a.deg[v];
-            const float nr = consolidate_div(acc, a.base_div);
-            dsum += fabsf(nr - prev);
-            a.pr_out[v] = nr;
-            a.acc[v] = 0.0f;
-            a.contrib_out[v] = d ? __fdiv_rn(nr, static_cast<float>(d)) : 0.0f;
-        }
+    const uint32_t *deg = rowlen ? a.fwd_v : a.deg;
+    const bool wide = ((reinterpret_cast<uintptr_t>(a.acc) | reinterpret_cast<uintptr_t>(a.pr_out) |
+                        reinterpret_cast<uintptr_t>(a.contrib_out) | reinterpret_cast<uintptr_t>(deg)) & 15) == 0;
+    const uint64_t quads = wide && n > gthreads() ? n / 4 : 0;
+    for (uint64_t q = gtid(); q < quads; q += gthreads()) {
+        const float4 acc = reinterpret_cast<const float4 *>(a.acc)[q], prev = reinterpret_cast<const float4 *>(a.pr_out)[q];
+        uint4 d = __ldg(reinterpret_cast<const uint4 *>(deg) + q);
+        if (rowlen) d = make_uint4(d.y - d.x, d.z - d.y, d.w - d.z, __ldg(deg + 4 * q + 4) - d.w);
+        float4 nr, c;
+        nr.x = consolidate_vertex(a, acc.x, prev.x, d.x, dsum, c.x);
+        nr.y = consolidate_vertex(a, acc.y, prev.y, d.y, dsum, c.y);
+        nr.z = consolidate_vertex(a, acc.z, prev.z, d.z, dsum, c.z);
+        nr.w = consolidate_vertex(a, acc.w, prev.w, d.w, dsum, c.w);
+        reinterpret_cast<float4 *>(a.pr_out)[q] = nr;
+        reinterpret_cast<float4 *>(a.acc)[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        reinterpret_cast<float4 *>(a.contrib_out)[q] = c;
+    }
+    for (uint64_t v = 4 * quads + gtid(); v < n; v += gthreads()) {
+        float c;
+        a.pr_out[v] = consolidate_vertex(a, a.acc[v], a.pr_out[v], rowlen ? deg[v + 1] - deg[v] : deg[v], dsum, c);
+        a.acc[v] = 0.0f;
+        a.contrib_out[v] = c;
     }
     add_diff_block(a.diff, dsum);
 }
@@ -859,11 +881,14 @@ __global__ void __launch_bounds__(256) k_pr_heavy_tiles(PrArgs a)
     const uint32_t *V = MODE <= 1 ? a.fwd_v : a.rev_v;
     const uint32_t *E = MODE <= 1 ? a.fwd_e : a.rev_e;
     const float *src = MODE == 3 ? a.pr_in : a.contrib_in;
-    for (;;) {
+    if (tiles == 0) return;                          // (the counters are as they were)
+    const uint32_t warps = gridDim.x * (blockDim.x / 32);    // each warp's first tile is its number
+    auto next = [&]() {
         uint32_t t = 0;
-        if (lane == 0) t = atomicAdd(&a.heavy_ctr[1], 1u);
-        t = __shfl_sync(FULL_MASK, t, 0);
-        if (t >= tiles) break;
+        if (lane == 0) t = warps + atomicAdd(&a.heavy_ctr[1], 1u);
+        return __shfl_sync(FULL_MASK, t, 0);
+    };
+    for (uint32_t t = gtid() >> 5; t < tiles; t = next()) {
         const uint4 q = a.heavy_q[t];
         const uint32_t t0 = q.y, t1 = q.z;
         if constexpr (MODE == 0) {                   // one row: its contribution to every edge
@@ -928,13 +953,11 @@ __global__ void __launch_bounds__(256) k_pr_heavy_tiles(PrArgs a)
         if constexpr (MODE >= 2)
             if (run_row != NO_ROW) atomicAdd(&a.acc[v0 + run_row], run);
     }
-    if (lane == 0) {
-        const uint32_t warps = gridDim.x * (blockDim.x / 32);
-        if (atomicAdd(&a.heavy_ctr[2], 1u) + 1 == warps) {
-            a.heavy_ctr[0] = 0;
-            a.heavy_ctr[1] = 0;
-            a.heavy_ctr[2] = 0;
-        }
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&a.heavy_ctr[2], 1u) + 1 == gridDim.x) {
+        a.heavy_ctr[0] = 0;
+        a.heavy_ctr[1] = 0;
+        a.heavy_ctr[2] = 0;
     }
 }
 
@@ -947,6 +970,7 @@ __global__ void __launch_bounds__(256) k_pr_heavy_finish(PrArgs a)
     const unsigned lane = threadIdx.x & 31;
     const uint64_t warp = gtid() >> 5, warps = gthreads() >> 5;
     const uint32_t chunks = a.heavy_ctr[3];
+    if (chunks == 0) return;                         // (the counters are as they were)
     const float base_nd = nodiv_base(a.n);
     float dsum = 0.0f;
     for (uint64_t k = warp; k < chunks; k += warps) {
@@ -959,7 +983,7 @@ __global__ void __launch_bounds__(256) k_pr_heavy_finish(PrArgs a)
         }
     }
     add_diff_block(a.diff, dsum);
-    if (lane == 0 && atomicAdd(&a.heavy_ctr[4], 1u) + 1 == warps) {
+    if (threadIdx.x == 0 && atomicAdd(&a.heavy_ctr[4], 1u) + 1 == gridDim.x) {
         a.heavy_ctr[3] = 0;
         a.heavy_ctr[4] = 0;
     }

@@ -76,3 +76,15 @@ def test_large(ctx, m):
     want = oracle.pagerank_f64(oracle.PR_DIV, n, h.rev_vertices, h.rev_edges, 3)
     for variant in VARIANTS:
         assert close(bw.pagerank(ctx, g, variant, 3), want), variant
+
+
+@pytest.mark.parametrize("n", [311295, 311296, 311297, 311299, 622593])
+@pytest.mark.parametrize("variant", ["vertex-push", "vertex-push-warp", "edge-list", "rev-edge-list"])
+def test_consolidation_sizes(ctx, n, variant):
+    """Vertex counts around the consolidation's change to four vertices a
+    thread (152 SMs x 8 blocks x 256 threads), every remainder of four."""
+    rng = np.random.default_rng(n)
+    m = 2 * n
+    h = bw.HostGraph.from_edges(n, rng.integers(0, n, m, dtype=np.uint32), rng.integers(0, n, m, dtype=np.uint32))
+    want = oracle.pagerank_f64(oracle.PR_DIV, n, h.rev_vertices, h.rev_edges, 4)
+    assert close(bw.pagerank(ctx, bw.DeviceGraph(h), variant, 4), want)
