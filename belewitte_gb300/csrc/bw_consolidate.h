@@ -92,4 +92,66 @@ BWC_HD uint32_t add_round_bits(uint64_t b_bits, uint32_t x_bits, bool &ok)
     return (static_cast<uint32_t>(e32) << 23) | static_cast<uint32_t>(F & 0x7fffff);
 }
 
+// The same result from about twenty float instructions for nearly every x;
+// `ok` is false when they do not decide it (add_round_bits then does).
+//
+// With hi = fl32(B) and lo = fl32(B - hi), s + e = hi + x exactly (Knuth's
+// two-sum), t = fl32(e + lo) and r + d = s + t exactly (Dekker's fast
+// two-sum), r = fl32(s + t).  What t and lo dropped is below 2^-23 ulp(s)
+// each (|e| and |lo| are at most half an ulp of s), and the double addition
+// that the reference rounds by moves the sum by less than 2^-28 ulp(s): so
+// while |d| stays 2^-19 of half an ulp of r away from the rounding boundary,
+// and r is no power of two, where the boundary below is nearer, rounding B + x
+// once or twice gives r.  Needs hi >= 2^-90 (split_base).
+BWC_HD float f32_add(float a, float b)
+{
+#if defined(__CUDA_ARCH__)
+    return __fadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+BWC_HD uint32_t f32_bits(float f)
+{
+#if defined(__CUDA_ARCH__)
+    return __float_as_uint(f);
+#else
+    uint32_t b;
+    memcpy(&b, &f, sizeof b);
+    return b;
+#endif
+}
+BWC_HD float f32_of(uint32_t b)
+{
+#if defined(__CUDA_ARCH__)
+    return __uint_as_float(b);
+#else
+    float f;
+    memcpy(&f, &b, sizeof f);
+    return f;
+#endif
+}
+struct Base {
+    float hi, lo;
+};
+// hi = 0 (never decided) for a base that is not positive or too small.
+inline Base split_base(double base)
+{
+    if (!(base >= 0x1p-90 && base <= 0x1p60)) return Base{0.0f, 0.0f};
+    const float hi = static_cast<float>(base);
+    return Base{hi, static_cast<float>(base - static_cast<double>(hi))};
+}
+BWC_HD float add_round_split(Base b, float x, bool &ok)
+{
+    const float s = f32_add(b.hi, x), xs = f32_add(s, -b.hi);
+    const float e = f32_add(f32_add(b.hi, -f32_add(s, -xs)), f32_add(x, -xs));
+    const float t = f32_add(e, b.lo), r = f32_add(s, t);
+    const float d = f32_add(t, -f32_add(r, -s));
+    const uint32_t rb = f32_bits(r);
+    // half an ulp of r less 2^-19 of it: (1 - 2^-19) 2^(k - 24)
+    const float limit = f32_of((rb & 0x7f800000u) - (24u << 23) - 32u);
+    ok = b.hi > 0.0f && x >= 0.0f && r < 0x1p100f && (d < 0.0f ? -d : d) < limit && (rb & 0x7fffffu) != 0u;
+    return r;
+}
+
 }  // namespace bwcons

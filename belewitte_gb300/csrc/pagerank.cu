@@ -119,6 +119,7 @@ struct PrArgs {
     const uint32_t *hot_vertex;
     const uint32_t *hot_count;    // device: slots in use
     double base_div;           // (1.0 - 0.85f) / N, computed once on the host
+    bwcons::Base base_split;   // the same as two floats (k_consolidate_div)
     // Packed graphs (bw_batch_run): graph i owns the vertices
     // [goff[i], goff[i + 1]) and has its own base term.
     const uint32_t *goff;
@@ -376,7 +377,9 @@ __global__ void __launch_bounds__(256) k_relabel_edges(const uint32_t *__restric
 __device__ __forceinline__ float consolidate_vertex(const PrArgs &a, float acc, float prev, uint32_t d, float &dsum,
                                                     float &contrib)
 {
-    const float nr = consolidate_div(acc, a.base_div);
+    bool ok;
+    float nr = bwcons::add_round_split(a.base_split, __fmul_rn(DAMPING, acc), ok);
+    if (!ok) nr = consolidate_div(acc, a.base_div);
     dsum += fabsf(nr - prev);
     contrib = d ? __fdiv_rn(nr, static_cast<float>(d)) : 0.0f;
     return nr;
@@ -2550,6 +2553,7 @@ int run_pagerank(bw_context *ctx, const bw_graph_view *g, const int32_t *schedul
     a.rev_s = reinterpret_cast<const uint2 *>(g->rev_struct_edges);
     a.n = n; a.m = g->edge_count;
     a.base_div = (1.0 - static_cast<double>(0.85f)) / static_cast<double>(n);
+    a.base_split = bwcons::split_base(a.base_div);
     a.deg = ctx->pr_deg;
     a.acc = ctx->pr_acc;
     a.gat_e = g->rev_edges;
