@@ -135,7 +135,7 @@ struct Base {
     float hi, lo;
 };
 // hi = 0 (never decided) for a base that is not positive or too small.
-inline Base split_base(double base)
+BWC_HD Base split_base(double base)
 {
     if (!(base >= 0x1p-90 && base <= 0x1p60)) return Base{0.0f, 0.0f};
     const float hi = static_cast<float>(base);

@@ -60,6 +60,17 @@ inline bool is_fused(int v)
 }
 inline bool uses_rowlen(int v) { return v == PR_VERTEX_PUSH || v == PR_VERTEX_PUSH_WARP; }
 
+// The base term of the div variants' consolidation, and as two floats.
+struct BaseTerm {
+    double d;
+    bwcons::Base split;
+};
+__host__ __device__ inline BaseTerm base_term(uint64_t n)
+{
+    const double d = (1.0 - static_cast<double>(0.85f)) / static_cast<double>(n);
+    return BaseTerm{d, bwcons::split_base(d)};
+}
+
 struct PrArgs {
     const uint32_t *fwd_v, *fwd_e, *rev_v, *rev_e, *fwd_in, *rev_in;
     const uint2 *fwd_s, *rev_s;
@@ -118,12 +129,11 @@ struct PrArgs {
     const uint2 *hot_pairs;       // struct-edge-list: translated {in, out}
     const uint32_t *hot_vertex;
     const uint32_t *hot_count;    // device: slots in use
-    double base_div;           // (1.0 - 0.85f) / N, computed once on the host
-    bwcons::Base base_split;   // the same as two floats (k_consolidate_div)
+    BaseTerm base_div;         // (1.0 - 0.85f) / N, computed once on the host
     // Packed graphs (bw_batch_run): graph i owns the vertices
     // [goff[i], goff[i + 1]) and has its own base term.
     const uint32_t *goff;
-    const double *gbase;
+    const BaseTerm *gbase;
     uint32_t graphs;
 };
 
@@ -146,17 +156,23 @@ __device__ __forceinline__ void resolve_args(PrArgs &a)
 // -- a double base term (computed once: IEEE division is correctly rounded,
 // so the host value is the one the reference computes per vertex), a float
 // product, one double addition and the rounding to float.
-// The double addition and the rounding to float are done in integer
-// arithmetic (bw_consolidate.h): bit-identical to the FP64 instructions,
-// which GB300 issues at a small fraction of the FP32 rate.
-__device__ __forceinline__ float consolidate_div(float acc, double base)
+// The double addition and the rounding to float are bit-identical to the FP64
+// instructions, which GB300 issues at a small fraction of the FP32 rate: float
+// arithmetic where it decides the result, else integer arithmetic
+// (bw_consolidate.h).  Integers alone are about 190 instructions a vertex
+// with the rest of k_consolidate_div and bound it: 3.1M vertices on GB300 20.2
+// us, with the floats first 13.6.  vertex-pull: grid 2048^2 110.6 -> 104.4 us
+// an iteration, R-MAT-22 278.5 -> 272.4.
+__device__ __forceinline__ float consolidate_div(float acc, const BaseTerm &base)
 {
     const float scaled = __fmul_rn(DAMPING, acc);
     bool ok;
-    const uint32_t r = bwcons::add_round_bits(static_cast<uint64_t>(__double_as_longlong(base)),
+    const float f = bwcons::add_round_split(base.split, scaled, ok);
+    if (ok) return f;
+    const uint32_t r = bwcons::add_round_bits(static_cast<uint64_t>(__double_as_longlong(base.d)),
                                               __float_as_uint(scaled), ok);
     if (ok) return __uint_as_float(r);
-    return __double2float_rn(__dadd_rn(base, static_cast<double>(scaled)));   // outside the emulated domain
+    return __double2float_rn(__dadd_rn(base.d, static_cast<double>(scaled)));   // outside the emulated domain
 }
 
 // The graph of vertex v of packed graphs: the last that starts at v or
@@ -377,9 +393,7 @@ __global__ void __launch_bounds__(256) k_relabel_edges(const uint32_t *__restric
 __device__ __forceinline__ float consolidate_vertex(const PrArgs &a, float acc, float prev, uint32_t d, float &dsum,
                                                     float &contrib)
 {
-    bool ok;
-    float nr = bwcons::add_round_split(a.base_split, __fmul_rn(DAMPING, acc), ok);
-    if (!ok) nr = consolidate_div(acc, a.base_div);
+    const float nr = consolidate_div(acc, a.base_div);
     dsum += fabsf(nr - prev);
     contrib = d ? __fdiv_rn(nr, static_cast<float>(d)) : 0.0f;
     return nr;
@@ -755,7 +769,7 @@ __device__ __forceinline__ FinishIn finish_load(const PrArgs &a, uint64_t v)
 
 template<bool NODIV>
 __device__ __forceinline__ float finish_store(const PrArgs &a, uint64_t v, float sum, float base_nd, FinishIn in,
-                                              double base)
+                                              const BaseTerm &base)
 {
     if constexpr (!NODIV) {
         const float nr = consolidate_div(sum, base);
@@ -2025,10 +2039,10 @@ __global__ void __launch_bounds__(LONG_SUM_THREADS, BLOCKS) k_pr_long_sums(PrArg
 
 // Packed graphs: each graph's base term; initial ranks 1/N_i and
 // contributions (k_pr_init's, per graph).
-__global__ void k_packed_base(const uint32_t *__restrict__ goff, uint32_t graphs, double *__restrict__ gbase)
+__global__ void k_packed_base(const uint32_t *__restrict__ goff, uint32_t graphs, BaseTerm *__restrict__ gbase)
 {
     for (uint32_t i = static_cast<uint32_t>(gtid()); i < graphs; i += static_cast<uint32_t>(gthreads()))
-        gbase[i] = (1.0 - static_cast<double>(DAMPING)) / static_cast<double>(goff[i + 1] - goff[i]);
+        gbase[i] = base_term(goff[i + 1] - goff[i]);
 }
 
 __global__ void k_packed_init(PrArgs a, float *__restrict__ pr, float *__restrict__ contrib)
@@ -2552,8 +2566,7 @@ int run_pagerank(bw_context *ctx, const bw_graph_view *g, const int32_t *schedul
     a.fwd_s = reinterpret_cast<const uint2 *>(g->fwd_struct_edges);
     a.rev_s = reinterpret_cast<const uint2 *>(g->rev_struct_edges);
     a.n = n; a.m = g->edge_count;
-    a.base_div = (1.0 - static_cast<double>(0.85f)) / static_cast<double>(n);
-    a.base_split = bwcons::split_base(a.base_div);
+    a.base_div = base_term(n);
     a.deg = ctx->pr_deg;
     a.acc = ctx->pr_acc;
     a.gat_e = g->rev_edges;
@@ -2857,8 +2870,8 @@ int bw::pagerank_run_packed(bw_context *ctx, const bw_graph_view *g, const uint3
         free_run(run, s);
         return rc;
     }
-    double *gbase = nullptr;
-    const cudaError_t e = ctx_malloc_async(ctx, reinterpret_cast<void **>(&gbase), graphs * sizeof(double), s);
+    BaseTerm *gbase = nullptr;
+    const cudaError_t e = ctx_malloc_async(ctx, reinterpret_cast<void **>(&gbase), graphs * sizeof(BaseTerm), s);
     if (e != cudaSuccess) free_run(run, s);
     BW_CUDA(e);
     PrArgs a{};
