@@ -308,6 +308,28 @@ int traversed_edges(bw_context *ctx, const bw_graph_view *g, int32_t *levels, cu
     return BW_OK;
 }
 
+// edge-list levels by chunk (k_bfs_edge_chunks), where a level would stream
+// the list from HBM and no launch shape is asked for.
+constexpr uint64_t CHUNKED_EDGES = uint64_t(16) << 20;
+bool chunked(const bw_graph_view *g, int variant, const bw_launch_config *cfg)
+{
+    return variant >= 0 && variant < 4 && g->edge_count >= CHUNKED_EDGES && !(cfg && (cfg->block_size || cfg->grid_size)) &&
+           ((reinterpret_cast<uintptr_t>(g->fwd_in_edges) | reinterpret_cast<uintptr_t>(g->fwd_edges)) & 15) == 0;
+}
+void plan_chunks(const bw_context *ctx, int variant, bool side, Launch *l)
+{
+    l->k = bfs_edge_active_kernel();
+    l->block = 256;
+    l->k2 = bfs_edge_chunk_kernel(variant, side);
+    l->grid = static_cast<unsigned>(ctx->sm_count) * 8;
+    l->grid2 = static_cast<unsigned>(ctx->sm_count) * (side ? 4 : 5);      // one resident wave
+}
+void chunk_args(bw_context *ctx, BfsArgs *a)
+{
+    a->ranges = ctx->heavy;
+    a->active = reinterpret_cast<uint32_t *>(ctx->heavy + (a->m + EDGE_CHUNK - 1) / EDGE_CHUNK);
+}
+
 // Host-loop traversal with a per-level variant schedule.
 int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, uint32_t sched_len,
              uint32_t root, int32_t *levels, const bw_launch_config *cfg, uint32_t max_levels,
@@ -323,6 +345,7 @@ int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, u
         if (v < 0 || v >= VARIANT_COUNT) return BW_ERR_UNKNOWN_VARIANT;
         if (!planned[v]) {
             BW_TRY(plan_launch(ctx, g, v, side, cfg, &plans[v]));
+            if (chunked(g, v, cfg)) plan_chunks(ctx, v, side, &plans[v]);
             planned[v] = true;
         }
     }
@@ -335,11 +358,19 @@ int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, u
     uint32_t level = 0;
     uint64_t visited = 1;
     int status = BW_OK;
+    bool ranges = false;                    // in ctx->heavy, until a push level's hub chunks overwrite them
     for (;;) {
         if (level >= max_levels) { status = BW_ERR_LEVEL_LIMIT; break; }
         const int v = schedule[std::min(level, sched_len - 1)];
         BfsArgs a = make_args(ctx, g, levels, static_cast<int32_t>(level), cfg);
+        const bool chunks = chunked(g, v, cfg), build = chunks && !ranges;
+        if (chunks) chunk_args(ctx, &a);
+        else if (plans[v].k2) ranges = false;
         if (time_levels) BW_CUDA(cudaEventRecord(ctx->level_events[0], s));
+        if (build) {
+            BW_TRY(bfs_edge_ranges(ctx, g, ctx->heavy, s));
+            ranges = true;
+        }
         BW_TRY(launch(plans[v], a, s));
         if (time_levels) BW_CUDA(cudaEventRecord(ctx->level_events[1], s));
         BW_TRY(post_and_wait(ctx, static_cast<int>(level % 3), s));
@@ -385,6 +416,8 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
     if (max_levels == 0) max_levels = static_cast<uint32_t>(std::min<uint64_t>(n + 1, 0xffffffffULL));
     Launch plan;
     BW_TRY(plan_launch(ctx, g, variant, side, cfg, &plan));
+    const bool chunks = chunked(g, variant, cfg);
+    if (chunks) plan_chunks(ctx, variant, side, &plan);
     const bool cluster_path = variant == V_FRONTIER_PUSH;
     if (cluster_path) {
         BW_TRY(ensure_outdeg(ctx, g, s));   // frontier edge volumes gate the cluster path
@@ -394,6 +427,7 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
     const uint32_t log_cap = stats ? std::min(stats_cap, max_levels) : 0;
     if (log_cap) BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&log), log_cap * sizeof(LevelSlot), s));
     BfsArgs a = make_args(ctx, g, levels, -1, cfg);
+    if (chunks) chunk_args(ctx, &a);
     if (cluster_path) {
         // small frontiers: the cluster kernel runs many levels per launch
         a.skip_check = 1;
@@ -411,6 +445,7 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
                                                          (side || cluster_path) ? ctx->outdeg : nullptr);
         BW_CUDA(cudaGetLastError());
         BW_CUDA(cudaEventRecord(ctx->ev_start, s));
+        if (chunks) BW_TRY(bfs_edge_ranges(ctx, g, ctx->heavy, s));
         for (uint32_t i = 0; i < DEVICE_LOOP_LAUNCHED && !end.stop; i++) {
             level_kernels(s, i == 0 || cluster_frontier(end.slot));
             const uint32_t seq = ++ctx->mail_seq;

@@ -29,4 +29,27 @@ BfsKernelFn bfs_edge_kernel(int layout, int reduction, bool side)
     }
 }
 
+template<int RED>
+static BfsKernelFn pick_chunks(bool side)
+{ return side ? k_bfs_edge_chunks<RED, true> : k_bfs_edge_chunks<RED, false>; }
+
+BfsKernelFn bfs_edge_chunk_kernel(int reduction, bool side)
+{
+    switch (reduction) {
+      case RED_NORMAL: return pick_chunks<RED_NORMAL>(side);
+      case RED_BULK: return pick_chunks<RED_BULK>(side);
+      case RED_WARP: return pick_chunks<RED_WARP>(side);
+      default: return pick_chunks<RED_BLOCK>(side);
+    }
+}
+
+BfsKernelFn bfs_edge_active_kernel() { return k_edge_active; }
+
+int bfs_edge_ranges(const bw_context *ctx, const bw_graph_view *g, uint2 *ranges, cudaStream_t s)
+{
+    k_edge_ranges<<<ctx->sm_count * 8, 256, 0, s>>>(g->fwd_in_edges, g->edge_count, ranges);
+    BW_CUDA(cudaGetLastError());
+    return BW_OK;
+}
+
 }  // namespace bw

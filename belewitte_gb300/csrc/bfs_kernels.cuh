@@ -202,6 +202,31 @@ __device__ __forceinline__ uint64_t gtid()
 __device__ __forceinline__ uint64_t gthreads()
 { return uint64_t(gridDim.x) * blockDim.x; }
 
+// Relaxes up to U neighbours (NO_VERTEX: none): their depths are all in
+// flight before the first relaxation, the relaxations' atomics before the
+// first result, and only a neighbour not yet visited costs an atomic.
+constexpr uint32_t NO_VERTEX = 0xffffffffu;
+template<int U>
+__device__ __forceinline__ void claim_all(int32_t *lv, int32_t nd, const uint32_t (&u)[U], bool (&won)[U])
+{
+    int32_t d[U];
+#pragma unroll
+    for (int j = 0; j < U; j++) d[j] = u[j] != NO_VERTEX ? lv[u[j]] : nd;
+#pragma unroll
+    for (int j = 0; j < U; j++) d[j] = d[j] > nd ? atomicMin(&lv[u[j]], nd) : nd;
+#pragma unroll
+    for (int j = 0; j < U; j++) won[j] = d[j] > nd;
+}
+template<int U, class Visit>
+__device__ __forceinline__ void relax_all(int32_t *lv, int32_t nd, const uint32_t (&u)[U], Visit visit)
+{
+    bool won[U];
+    claim_all(lv, nd, u, won);
+#pragma unroll
+    for (int j = 0; j < U; j++)
+        if (won[j]) visit(u[j]);
+}
+
 // ---------------------------------------------------------------------------
 // Edge-list families (bfs/edgelist.cu:3-22, rev_edgelist.cu:3-21,
 // struct_edgelist.cu:3-22, rev_struct_edgelist.cu:3-22).  Every level
@@ -234,6 +259,25 @@ __global__ void __launch_bounds__(512) k_bfs_edge(BfsArgs a)
         }
     };
 
+    // Four edges.  Forward: their depths in flight together (ER(1M, 8M)
+    // edge-list 320 -> 286 us a traversal, R-MAT-16 struct-edge-list 113 -> 105);
+    // the reverse lists, whose quads are mostly one row, lose by it (BA(8.4M, 8)
+    // 4.25 -> 4.47 ms).
+    auto edges = [&](const uint4 &r, const uint4 &c) {
+        if constexpr (LAYOUT == FWD_SOA || LAYOUT == FWD_AOS) {
+            const uint32_t row[4] = {r.x, r.y, r.z, r.w}, col[4] = {c.x, c.y, c.z, c.w};
+            bool want[4];
+            uint32_t u[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) want[k] = lv[row[k]] == depth;
+#pragma unroll
+            for (int k = 0; k < 4; k++) u[k] = want[k] ? col[k] : NO_VERTEX;
+            relax_all(lv, nd, u, [&](uint32_t w) { cnt.hit(&slot->frontier); side.visit(a, qnext, slot, w); });
+        } else {
+            edge(r.x, c.x); edge(r.y, c.y); edge(r.z, c.z); edge(r.w, c.w);
+        }
+    };
+
     const uint64_t m = a.m;
     bool aligned;
     if constexpr (LAYOUT == FWD_SOA) aligned = !((reinterpret_cast<uintptr_t>(a.fwd_in) | reinterpret_cast<uintptr_t>(a.fwd_e)) & 15);
@@ -248,12 +292,12 @@ __global__ void __launch_bounds__(512) k_bfs_edge(BfsArgs a)
             const uint32_t *cols = LAYOUT == FWD_SOA ? a.fwd_e : a.rev_e;
             const uint4 r = __ldcs(reinterpret_cast<const uint4 *>(rows) + g);
             const uint4 c = __ldcs(reinterpret_cast<const uint4 *>(cols) + g);
-            edge(r.x, c.x); edge(r.y, c.y); edge(r.z, c.z); edge(r.w, c.w);
+            edges(r, c);
         } else {
             const uint2 *pairs = LAYOUT == FWD_AOS ? a.fwd_s : a.rev_s;
             const uint4 p0 = __ldcs(reinterpret_cast<const uint4 *>(pairs) + 2 * g);
             const uint4 p1 = __ldcs(reinterpret_cast<const uint4 *>(pairs) + 2 * g + 1);
-            edge(p0.x, p0.y); edge(p0.z, p0.w); edge(p1.x, p1.y); edge(p1.z, p1.w);
+            edges(make_uint4(p0.x, p0.z, p1.x, p1.z), make_uint4(p0.y, p0.w, p1.y, p1.w));
         }
     }
     for (uint64_t e = (groups << 2) + gtid(); e < m; e += stride) {
@@ -264,6 +308,137 @@ __global__ void __launch_bounds__(512) k_bfs_edge(BfsArgs a)
     }
     cnt.finish(&slot->frontier);
     side.finish_block(slot);
+}
+
+// edge-list over chunks of EDGE_CHUNK edges, for lists that L2 does not hold.
+// k_edge_ranges reads the sources once per traversal and writes each chunk's
+// least and largest one.  A level looks at the depths between them first
+// (k_edge_active) and reads the edges of those chunks only where a source of
+// this level is (k_bfs_edge_chunks), shared by all warps, as a hub's edges
+// may be the level.  In a list sorted by source a chunk's range is a few
+// dozen depths; chunks with a range too wide for that are read as before.
+// (The reverse lists have work in nearly every chunk until their last levels.)
+// GB300, BA(8.4M, 8), 134M edges, a traversal from a hub: 1289 us with every
+// level streamed whole, 1029 by chunk (a quiet level 171 -> 25 us, the ranges
+// 80; the two large levels are 60M gathers each).  R-MAT-22 696 -> 687, a root
+// without edges there 94 -> 91.
+constexpr uint32_t ACTIVE_BATCH = 4;                // chunks a warp looks at, 128 depths each in flight
+
+static __global__ void __launch_bounds__(256) k_edge_active(BfsArgs a)
+{
+    constexpr uint32_t RANGE = 2 * EDGE_CHUNK;
+    __shared__ uint32_t s_count[8], s_base;
+    const int32_t depth = level_depth(a);
+    LevelSlot *slot = &a.ctl->slot[depth % 3];
+    const int32_t *lv = a.levels;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint64_t chunks = (a.m + EDGE_CHUNK - 1) / EDGE_CHUNK, step = uint64_t(gridDim.x) * warps * ACTIVE_BATCH;
+    for (uint64_t b0 = uint64_t(blockIdx.x) * warps * ACTIVE_BATCH; b0 < chunks; b0 += step) {
+        const uint64_t first = b0 + wib * ACTIVE_BATCH;
+        const uint2 mine = lane < ACTIVE_BATCH && first + lane < chunks ? a.ranges[first + lane] : make_uint2(1u, 0u);
+        bool hit[ACTIVE_BATCH];
+#pragma unroll
+        for (uint32_t j = 0; j < ACTIVE_BATCH; j++) {
+            const uint32_t lo = __shfl_sync(FULL_MASK, mine.x, j), hi = __shfl_sync(FULL_MASK, mine.y, j);
+            const uint64_t v = uint64_t(lo) + lane;
+            const int32_t d0 = v <= hi ? lv[v] : -1, d1 = v + 32 <= hi ? lv[v + 32] : -1;
+            const int32_t d2 = v + 64 <= hi ? lv[v + 64] : -1, d3 = v + 96 <= hi ? lv[v + 96] : -1;
+            hit[j] = d0 == depth || d1 == depth || d2 == depth || d3 == depth;
+        }
+        unsigned found = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < ACTIVE_BATCH; j++) {
+            const uint32_t lo = __shfl_sync(FULL_MASK, mine.x, j), hi = __shfl_sync(FULL_MASK, mine.y, j);
+            bool any = __any_sync(FULL_MASK, hit[j]) || (hi > lo && hi - lo >= RANGE);
+            for (uint64_t v = uint64_t(lo) + 128 + lane; !any && v - lane <= hi; v += 256) {
+                int32_t d[8];
+#pragma unroll
+                for (uint32_t k = 0; k < 8; k++) d[k] = v + 32 * k <= hi ? lv[v + 32 * k] : -1;
+                bool here = false;
+#pragma unroll
+                for (uint32_t k = 0; k < 8; k++) here = here || d[k] == depth;
+                any = __any_sync(FULL_MASK, here);
+            }
+            if (any) found |= 1u << j;
+        }
+        // append, one atomic per block
+        if (lane == 0) s_count[wib] = __popc(found);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t total = 0;
+            for (uint32_t w = 0; w < warps; w++) {
+                const uint32_t c = s_count[w];
+                s_count[w] = total;
+                total += c;
+            }
+            s_base = total ? atomicAdd(&slot->heavy, total) : 0u;
+        }
+        __syncthreads();
+        if (found >> lane & 1)
+            a.active[s_base + s_count[wib] + __popc(found & ((1u << lane) - 1))] = static_cast<uint32_t>(first + lane);
+        __syncthreads();
+    }
+}
+
+template<int RED, bool SIDE>
+__global__ void __launch_bounds__(256, SIDE ? 4 : 5) k_bfs_edge_chunks(BfsArgs a)
+{
+    constexpr uint32_t STEPS = EDGE_CHUNK / 128;
+    const int32_t depth = level_depth(a), nd = depth + 1;
+    LevelSlot *slot = &a.ctl->slot[depth % 3];
+    if (blockIdx.x == 0 && threadIdx.x == 0) reset_slot(&a.ctl->slot[(depth + 1) % 3]);
+    uint32_t *qnext = (depth & 1) ? a.q0 : a.q1;
+    int32_t *lv = a.levels;
+    Counter<RED> cnt;
+    Side<SIDE> side;
+    const uint32_t lane = threadIdx.x & 31;
+    auto edge = [&](uint32_t row, uint32_t col) {
+        if (lv[row] == depth && relax(lv, col, nd)) { cnt.hit(&slot->frontier); side.visit(a, qnext, slot, col); }
+    };
+    const uint64_t m = a.m, steps = uint64_t(slot->heavy) * STEPS, warps = gthreads() >> 5;
+    for (uint64_t t0 = (gtid() >> 5) * 2; t0 < steps; t0 += warps * 2) {      // (STEPS is even)
+        const uint64_t e = uint64_t(__ldg(a.active + t0 / STEPS)) * EDGE_CHUNK + (t0 % STEPS) * 128 + 4 * lane;
+        if (e + 128 + 4 <= m) {
+            const uint4 r0 = __ldcs(reinterpret_cast<const uint4 *>(a.fwd_in + e)), r1 = __ldcs(reinterpret_cast<const uint4 *>(a.fwd_in + e + 128));
+            const uint4 q0 = __ldcs(reinterpret_cast<const uint4 *>(a.fwd_e + e)), q1 = __ldcs(reinterpret_cast<const uint4 *>(a.fwd_e + e + 128));
+            const uint32_t row[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w}, col[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+            uint32_t u[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) u[k] = lv[row[k]] == depth ? col[k] : NO_VERTEX;
+            relax_all(lv, nd, u, [&](uint32_t w) { cnt.hit(&slot->frontier); side.visit(a, qnext, slot, w); });
+        } else {
+            for (uint64_t i = e; i < m && i < e + 4; i++) edge(a.fwd_in[i], a.fwd_e[i]);
+            for (uint64_t i = e + 128; i < m && i < e + 132; i++) edge(a.fwd_in[i], a.fwd_e[i]);
+        }
+    }
+    cnt.finish(&slot->frontier);
+    side.finish_block(slot);
+}
+
+// A warp per chunk, the chunk's 4 KB in flight; `in` is 16-byte aligned.
+static __global__ void __launch_bounds__(256) k_edge_ranges(const uint32_t *__restrict__ in, uint64_t m,
+                                                            uint2 *__restrict__ ranges)
+{
+    constexpr uint32_t STEPS = EDGE_CHUNK / 128;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t chunks = (m + EDGE_CHUNK - 1) / EDGE_CHUNK;
+    for (uint64_t c = gtid() >> 5; c < chunks; c += gthreads() >> 5) {
+        uint32_t least = 0xffffffffu, most = 0u;
+        auto take = [&](uint32_t r) { least = min(least, r); most = max(most, r); };
+        const uint64_t e0 = c * EDGE_CHUNK + 4 * lane;
+        if (c * EDGE_CHUNK + EDGE_CHUNK <= m) {
+            uint4 r[STEPS];
+#pragma unroll
+            for (uint32_t k = 0; k < STEPS; k++) r[k] = __ldcs(reinterpret_cast<const uint4 *>(in + e0 + k * 128));
+#pragma unroll
+            for (uint32_t k = 0; k < STEPS; k++) { take(r[k].x); take(r[k].y); take(r[k].z); take(r[k].w); }
+        } else {
+            for (uint64_t e = c * EDGE_CHUNK + lane; e < m; e += 32) take(in[e]);
+        }
+        least = __reduce_min_sync(FULL_MASK, least);
+        most = __reduce_max_sync(FULL_MASK, most);
+        if (lane == 0) ranges[c] = make_uint2(least, most);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -300,31 +475,6 @@ __device__ __forceinline__ uint32_t concat_row(uint32_t excl, uint32_t k)
     for (uint32_t b = 16; b > 0; b >>= 1)
         if (__shfl_sync(FULL_MASK, excl, l + b) <= k) l += b;
     return l;
-}
-
-// Relaxes up to U neighbours (NO_VERTEX: none): their depths are all in
-// flight before the first relaxation, the relaxations' atomics before the
-// first result, and only a neighbour not yet visited costs an atomic.
-constexpr uint32_t NO_VERTEX = 0xffffffffu;
-template<int U>
-__device__ __forceinline__ void claim_all(int32_t *lv, int32_t nd, const uint32_t (&u)[U], bool (&won)[U])
-{
-    int32_t d[U];
-#pragma unroll
-    for (int j = 0; j < U; j++) d[j] = u[j] != NO_VERTEX ? lv[u[j]] : nd;
-#pragma unroll
-    for (int j = 0; j < U; j++) d[j] = d[j] > nd ? atomicMin(&lv[u[j]], nd) : nd;
-#pragma unroll
-    for (int j = 0; j < U; j++) won[j] = d[j] > nd;
-}
-template<int U, class Visit>
-__device__ __forceinline__ void relax_all(int32_t *lv, int32_t nd, const uint32_t (&u)[U], Visit visit)
-{
-    bool won[U];
-    claim_all(lv, nd, u, won);
-#pragma unroll
-    for (int j = 0; j < U; j++)
-        if (won[j]) visit(u[j]);
 }
 
 // Relaxes the neighbours E[first + k * step] (k < BFS_PUSH_UNROLL, below

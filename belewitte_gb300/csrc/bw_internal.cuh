@@ -130,7 +130,11 @@ struct BfsArgs {
     uint32_t skip_check;          // device loop with the cluster path: honour ctl->skip
     LevelSlot *log;               // device-loop level log (cluster path)
     uint32_t log_cap;
+    const uint2 *ranges;          // edge-list by chunk: {least, largest} source of every EDGE_CHUNK edges
+    uint32_t *active;             // its chunks with work in this level (slot->heavy of them)
 };
+// Edges per range: 12 bytes a chunk, in the hub-chunk queue's 64 (ensure_bfs_scratch).
+constexpr uint32_t EDGE_CHUNK = 1024;
 
 // ---------------------------------------------------------------------------
 // PageRank scratch
@@ -234,6 +238,9 @@ __global__ void k_row_lengths(const uint32_t *__restrict__ off, uint64_t n,
 using BfsKernelFn = void (*)(BfsArgs);
 // Instantiation tables (bfs_edge.cu, bfs_vertex.cu).
 BfsKernelFn bfs_edge_kernel(int layout, int reduction, bool side);
+BfsKernelFn bfs_edge_active_kernel();
+BfsKernelFn bfs_edge_chunk_kernel(int reduction, bool side);
+int bfs_edge_ranges(const bw_context *ctx, const bw_graph_view *g, uint2 *ranges, cudaStream_t s);
 BfsKernelFn bfs_vertex_kernel(int family, int reduction, bool side);
 BfsKernelFn bfs_frontier_push_kernel(bool side);
 BfsKernelFn bfs_hub_kernel(bool side);
