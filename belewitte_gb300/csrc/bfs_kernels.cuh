@@ -895,17 +895,26 @@ __global__ void __launch_bounds__(256) k_bfs_frontier_pull(BfsArgs a)
 // -- the high-diameter case (2-D grids, BFS tails) where one launch per
 // level would dominate.  A level is then a short chain of dependent
 // accesses, so the kernel keeps all else on chip:
-//  * each block holds a share of the frontier in shared memory as
-//    {vertex, row start, row end}: a level reads no queue and no offsets
-//    from global memory;
+//  * each block holds its part of the frontier in shared memory as {row
+//    start, row end}: a level reads no queue and no offsets from global
+//    memory, and where no row of a warp's 32 is longer than CLUSTER_UNROLL
+//    (meshes) each lane takes its own row, without the search for an edge's
+//    row in the concatenation;
 //  * a neighbour is claimed with one atomicMin on its depth, issued with
 //    its row bounds' loads and the lane's other claims; the winner puts the
 //    bounds in its block's next list;
-//  * after the level's one cluster barrier, every block reads the blocks'
-//    counts and then its equal share of the next frontier from the other
-//    blocks' shared memory (a wavefront found by one block would otherwise
-//    stay with it).  The next lists alternate between two buffers, so the
-//    copy needs no second barrier.
+//  * warps add their counts to their block's in shared memory, and after the
+//    level's one cluster barrier every warp reads the blocks' counts for
+//    itself.  Lists of up to CLUSTER_KEEP rows stay with their block; longer
+//    ones are shared out equally, read from the other blocks' shared memory.
+//    The next lists alternate between two buffers, the counts between three,
+//    so nothing needs a second cluster barrier.
+// Bound by the latency of that chain: on GB300 a level of the 2048 x 2048 grid
+// took 4.5 to 5.0 us and takes 3.1 to 4.0, of a 300 x 300 grid 4.0 and 2.7.
+// More threads a block than the frontier fills only make the barriers dearer
+// (1024 instead of 512: 3.1 and 4.4 us), fewer leave wide frontiers behind
+// (256: 2.5 us on 300 x 300, but 7.4 instead of 6.8 on 5000 x 5000); 16 blocks
+// of 256 in place of 8 of 512: 3.0 and 6.2.
 // Rows above CLUSTER_HEAVY edges are left to the full-GPU kernels (their
 // hub chunks spread such a row over every SM): a frontier with one is not
 // taken on, and a level that finds one hands over.  So do a frontier above
@@ -918,18 +927,18 @@ __global__ void __launch_bounds__(256) k_bfs_frontier_pull(BfsArgs a)
 // ---------------------------------------------------------------------------
 constexpr uint32_t CLUSTER_HEAVY = 1024;           // rows above: the full-GPU kernels
 constexpr int CLUSTER_UNROLL = 4;
-static_assert(CLUSTER_THREADS == 32 * 32, "the block's counts are reduced by one warp, one lane per warp");
-// dynamic shared memory: the level's share and two next lists, each of
-// {vertex, row start, row end}
-constexpr size_t CLUSTER_SMEM = 3 * 3 * CLUSTER_LIST * sizeof(uint32_t);
+constexpr uint32_t CLUSTER_KEEP = 256;             // next lists up to this long stay with their block
+// dynamic shared memory: the level's share {row start, row end} and two next
+// lists {row start, row end}, {vertex}
+constexpr size_t CLUSTER_SMEM = (3 * 2 + 2) * CLUSTER_LIST * sizeof(uint32_t);
 
-struct ClusterCounts {
-    uint32_t frontier;            // new vertices of the level found by this block
-    uint32_t listed;              // of those, in the block's next list
-    unsigned long long fedges;    // their out-edges
-    unsigned long long ls, lq;    // log-degree statistics (STATS == 1), fixed point
-    float lm;
-    uint32_t heavy;               // of those, rows above CLUSTER_HEAVY
+// A block's counts of one level, added up by its warps; read by the others.
+struct __align__(16) ClusterCounts {
+    uint32_t frontier;            // new vertices found (those past CLUSTER_LIST went to the global queue)
+    uint32_t fedges;              // their out-edges (each vertex once: at most M < 2^32 in all)
+    uint32_t heavy;               // != 0: one of them has a row above CLUSTER_HEAVY
+    uint32_t lm_bits;             // STATS == 1: largest log degree
+    unsigned long long ls, lq;    // STATS == 1: log-degree sums, fixed point
 };
 
 // STATS: 0 none; 1 the log-degree statistics of every level (accumulated
@@ -939,15 +948,10 @@ template<int STATS>
 __global__ void __cluster_dims__(CLUSTER_CTAS, 1, 1) __launch_bounds__(CLUSTER_THREADS)
 k_bfs_cluster(BfsArgs a)
 {
-    extern __shared__ uint32_t cl_lists[];
-    __shared__ ClusterCounts s_cnt[2];             // by level parity; read by the other blocks
-    __shared__ ClusterCounts s_tot;                // the cluster's totals
-    __shared__ uint32_t s_pre[CLUSTER_CTAS + 1];    // exclusive prefix of the blocks' next lists
-    __shared__ unsigned long long r_fe[CLUSTER_THREADS / 32];
-    __shared__ uint32_t r_hits[CLUSTER_THREADS / 32], r_heavy[CLUSTER_THREADS / 32];
+    extern __shared__ __align__(16) uint32_t cl_lists[];
+    __shared__ ClusterCounts s_cnt[3];             // by level
     __shared__ unsigned long long r_ls[CLUSTER_THREADS / 32], r_lq[CLUSTER_THREADS / 32];
     __shared__ float r_lm[CLUSTER_THREADS / 32];
-    __shared__ uint32_t s_n, s_cur_n;
     __shared__ unsigned long long s_hand[3];       // this block's part of a handed-over frontier's statistics
     cg::cluster_group cl = cg::this_cluster();
     BfsCtl *ctl = a.ctl;
@@ -961,13 +965,11 @@ k_bfs_cluster(BfsArgs a)
     // the full-GPU kernels
     if (qlen == 0 || qlen > CLUSTER_CAP || fedges > CLUSTER_EDGE_CAP) return;
     int32_t *lv = a.levels;
-    // buffer 0: the level's share; buffers 1 and 2: next lists, alternating
-    uint32_t *lst_v[3], *lst_s[3], *lst_e[3];
-    for (int b = 0; b < 3; b++) {
-        lst_v[b] = cl_lists + (3 * b) * CLUSTER_LIST;
-        lst_s[b] = cl_lists + (3 * b + 1) * CLUSTER_LIST;
-        lst_e[b] = cl_lists + (3 * b + 2) * CLUSTER_LIST;
-    }
+    uint2 *const share = reinterpret_cast<uint2 *>(cl_lists);
+    uint2 *const next_se[2] = {share + CLUSTER_LIST, share + 2 * CLUSTER_LIST};
+    uint32_t *const next_v[2] = {cl_lists + 6 * CLUSTER_LIST, cl_lists + 7 * CLUSTER_LIST};
+    uint32_t ncur;                                 // rows in `cur`, this block's part of the level
+    const uint2 *cur = share;
     {   // this block's share of the level's queue, with the rows' bounds
         const uint32_t *qin = (L & 1) ? a.q1 : a.q0;
         const uint32_t per = (qlen + CLUSTER_CTAS - 1) / CLUSTER_CTAS;
@@ -976,184 +978,178 @@ k_bfs_cluster(BfsArgs a)
         for (uint32_t i = tid; i < cnt; i += CLUSTER_THREADS) {
             const uint32_t v = __ldcg(qin + b + i);
             const uint32_t rs = a.fwd_v[v], re = a.fwd_v[v + 1];
-            lst_v[0][i] = v;
-            lst_s[0][i] = rs;
-            lst_e[0][i] = re;
+            share[i] = make_uint2(rs, re);
             heavy |= re - rs > CLUSTER_HEAVY ? 1u : 0u;
         }
+        if (tid < 3) s_cnt[tid] = ClusterCounts{};
         heavy = __syncthreads_or(heavy);
-        if (tid == 0) {
-            s_cur_n = cnt;
-            s_cnt[1].heavy = heavy;
-        }
+        if (tid == 0) s_cnt[(L + 2) % 3].heavy = heavy;
+        ncur = cnt;
         cl.sync();
         uint32_t any = 0;
-        if (tid < CLUSTER_CTAS) any = cl.map_shared_rank(&s_cnt[1], tid)->heavy;
+        if (tid < CLUSTER_CTAS) any = cl.map_shared_rank(&s_cnt[(L + 2) % 3], tid)->heavy;
         any = __syncthreads_or(any);
         cl.sync();                                   // nobody leaves while its flag may be read
         if (any) return;                             // a hub row: the full-GPU kernels take this level
+        // (the flag is zero then, as the counts of level L + 2 begin)
     }
-    int p = 0;                                       // next lists: buffer 1 + p
+    unsigned long long visited = 0, traversed = 0;   // of the completed levels (the leader's)
+    int p = 0;                                       // the next list being filled
     for (;;) {
         const int32_t nd = L + 1;
         LevelSlot *slot = &ctl->slot[L % 3];
+        ClusterCounts *const cnt = &s_cnt[L % 3];
         uint32_t *qnext = (L & 1) ? a.q0 : a.q1;
         if (leader) reset_slot(&ctl->slot[(L + 1) % 3]);
-        if (tid == 0) s_n = 0;
-        __syncthreads();
-        const uint32_t ncur = s_cur_n;
-        const uint32_t *cs = lst_s[0], *ce = lst_e[0];
-        uint32_t *nv = lst_v[1 + p], *ns = lst_s[1 + p], *ne = lst_e[1 + p];
-        uint32_t hits = 0, heavy = 0;
-        unsigned long long fe = 0;
+        uint2 *const nse = next_se[p];
+        uint32_t *const nv = next_v[p];
+        uint32_t fe = 0, heavy = 0;
         unsigned long long ls = 0, lq = 0;
         float lm = 0.f;
-        // a claimed neighbour u with row [us, ue): its counts and its entry k
-        auto claim = [&](uint32_t u, uint32_t us, uint32_t ue, uint32_t k) {
-            // Next-line prefetch: where vertex ids follow the graph's
-            // geometry (grids, meshes, road networks) the wavefront reaches
-            // u's id neighbours within a few levels, and the first touch of
-            // their lines would put an HBM miss on the level's critical path.
-            if (ue + 32 < a.m) prefetch_l2(a.fwd_e + ue + 32);
-            if (u + 33 <= a.n) prefetch_l2(a.fwd_v + u + 33);
-            if (u + 32 < a.n) prefetch_l2(lv + u + 32);
-            hits++;
-            fe += ue - us;
-            heavy += ue - us > CLUSTER_HEAVY ? 1u : 0u;
-            if constexpr (STATS == 1) {
-                const float l = __log2f(1.0f + static_cast<float>(ue - us));
-                ls += lsum_fx(l); lq += lsq_fx(l); lm = fmaxf(lm, l);
+        // Claims up to CLUSTER_UNROLL neighbours a lane.  A level is a chain
+        // of dependent accesses, so every lane's neighbours go out together:
+        // their row bounds (loaded whether or not the claim wins) and their
+        // atomics are all in flight before any result is used.
+        auto claim = [&](const uint32_t (&u)[CLUSTER_UNROLL]) {
+            uint32_t us[CLUSTER_UNROLL], ue[CLUSTER_UNROLL];
+            int32_t old[CLUSTER_UNROLL];
+#pragma unroll
+            for (int jj = 0; jj < CLUSTER_UNROLL; jj++)
+                old[jj] = u[jj] != NO_VERTEX ? atomicMin(&lv[u[jj]], nd) : nd;
+#pragma unroll
+            for (int jj = 0; jj < CLUSTER_UNROLL; jj++) {
+                us[jj] = ue[jj] = 0;
+                if (u[jj] != NO_VERTEX) {
+                    us[jj] = __ldg(a.fwd_v + u[jj]);
+                    ue[jj] = __ldg(a.fwd_v + u[jj] + 1);
+                }
             }
-            if (k < CLUSTER_LIST) {
-                nv[k] = u;
-                ns[k] = us;
-                ne[k] = ue;
-            } else {                                     // overflow: straight to the global queue
-                qnext[atomicAdd(&slot->qlen, 1u)] = u;
+            // the winners' entries: one shared atomic per warp
+            unsigned wm[CLUSTER_UNROLL];
+            uint32_t total = 0;
+#pragma unroll
+            for (int jj = 0; jj < CLUSTER_UNROLL; jj++) {
+                wm[jj] = __ballot_sync(FULL_MASK, old[jj] > nd);
+                total += __popc(wm[jj]);
+            }
+            if (total == 0) return;
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&cnt->frontier, total);
+            base = __shfl_sync(FULL_MASK, base, 0);
+            const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+            for (int jj = 0; jj < CLUSTER_UNROLL; jj++) {
+                if (old[jj] > nd) {
+                    const uint32_t k = base + __popc(wm[jj] & below);
+                    if (k < CLUSTER_LIST) {
+                        nse[k] = make_uint2(us[jj], ue[jj]);
+                        nv[k] = u[jj];
+                    } else {                             // overflow: straight to the global queue
+                        qnext[atomicAdd(&slot->qlen, 1u)] = u[jj];
+                    }
+                    fe += ue[jj] - us[jj];
+                    heavy |= ue[jj] - us[jj] > CLUSTER_HEAVY ? 1u : 0u;
+                    if constexpr (STATS == 1) {
+                        const float l = __log2f(1.0f + static_cast<float>(ue[jj] - us[jj]));
+                        ls += lsum_fx(l); lq += lsq_fx(l); lm = fmaxf(lm, l);
+                    }
+                    // Next-line prefetch: where vertex ids follow the graph's
+                    // geometry (grids, meshes, road networks) the wavefront
+                    // reaches u's id neighbours within a few levels, and the
+                    // first touch of their lines would put an HBM miss on the
+                    // level's critical path.
+                    if (ue[jj] + 32 < a.m) prefetch_l2(a.fwd_e + ue[jj] + 32);
+                    if (u[jj] + 33 <= a.n) prefetch_l2(a.fwd_v + u[jj] + 33);
+                    if (u[jj] + 32 < a.n) prefetch_l2(lv + u[jj] + 32);
+                }
+                base += __popc(wm[jj]);
             }
         };
-        // 32 entries per warp step, their rows concatenated
+        // 32 rows per warp step
         for (uint32_t t = wib * 32; t < ncur; t += CLUSTER_THREADS) {
             const uint32_t i = t + lane;
-            uint32_t s = 0, d = 0;
-            if (i < ncur) {
-                s = cs[i];
-                d = ce[i] - s;
+            const uint2 se = i < ncur ? cur[i] : make_uint2(0u, 0u);
+            const uint32_t s = se.x, d = se.y - se.x;
+            uint32_t u[CLUSTER_UNROLL];
+            if (__reduce_max_sync(FULL_MASK, d) <= CLUSTER_UNROLL) {
+                // short rows (meshes): a lane's own row
+#pragma unroll
+                for (uint32_t jj = 0; jj < CLUSTER_UNROLL; jj++) u[jj] = jj < d ? __ldg(a.fwd_e + s + jj) : NO_VERTEX;
+                claim(u);
+                continue;
             }
+            // the rows concatenated
             uint32_t incl = d;
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t y = __shfl_up_sync(FULL_MASK, incl, o);
                 if (lane >= static_cast<unsigned>(o)) incl += y;
             }
-            const uint32_t total = __shfl_sync(FULL_MASK, incl, 31), excl = incl - d;
+            const uint32_t total = __shfl_sync(FULL_MASK, incl, 31), excl = incl - d, from = s - excl;
             for (uint32_t k0 = 0; k0 < total; k0 += 32 * CLUSTER_UNROLL) {
-                uint32_t u[CLUSTER_UNROLL];
 #pragma unroll
                 for (int jj = 0; jj < CLUSTER_UNROLL; jj++) {
-                    // edge k of the concatenated rows belongs to the last
-                    // lane whose exclusive prefix is <= k (that lane's row
-                    // is not empty): a binary search over the lanes
-                    const uint32_t k = k0 + jj * 32 + lane;
-                    uint32_t seg = 0;
-#pragma unroll
-                    for (uint32_t b = 16; b > 0; b >>= 1)
-                        if (__shfl_sync(FULL_MASK, excl, seg + b) <= k) seg += b;
-                    const uint32_t rs = __shfl_sync(FULL_MASK, s, seg), ex = __shfl_sync(FULL_MASK, excl, seg);
-                    u[jj] = k < total ? __ldg(a.fwd_e + rs + (k - ex)) : 0xffffffffu;
+                    const uint32_t k = k0 + jj * 32 + lane, row = concat_row(excl, k);
+                    const uint32_t at = __shfl_sync(FULL_MASK, from, row) + k;
+                    u[jj] = k < total ? __ldg(a.fwd_e + at) : NO_VERTEX;
                 }
-                // A level is a chain of dependent accesses, so every lane's
-                // neighbours go out together: their row bounds (loaded
-                // whether or not the claim wins) and their atomics are all
-                // in flight before any result is used.
-                uint32_t us[CLUSTER_UNROLL], ue[CLUSTER_UNROLL];
-                int32_t old[CLUSTER_UNROLL];
-#pragma unroll
-                for (int jj = 0; jj < CLUSTER_UNROLL; jj++) {
-                    us[jj] = ue[jj] = 0;
-                    if (u[jj] != 0xffffffffu) {
-                        us[jj] = __ldg(a.fwd_v + u[jj]);
-                        ue[jj] = __ldg(a.fwd_v + u[jj] + 1);
-                    }
-                }
-#pragma unroll
-                for (int jj = 0; jj < CLUSTER_UNROLL; jj++)
-                    old[jj] = u[jj] != 0xffffffffu ? atomicMin(&lv[u[jj]], nd) : nd;
-                // the winners' entries: one shared atomic per warp and step
-#pragma unroll
-                for (int jj = 0; jj < CLUSTER_UNROLL; jj++) {
-                    const bool win = old[jj] > nd;
-                    const unsigned wm = __ballot_sync(FULL_MASK, win);
-                    if (wm == 0) continue;
-                    uint32_t base = 0;
-                    if (lane == 0) base = atomicAdd(&s_n, static_cast<uint32_t>(__popc(wm)));
-                    base = __shfl_sync(FULL_MASK, base, 0);
-                    if (win) claim(u[jj], us[jj], ue[jj], base + __popc(wm & ((1u << lane) - 1u)));
-                }
+                claim(u);
             }
         }
-        // the block's counts
-        for (int o = 16; o > 0; o >>= 1) {
-            hits += __shfl_xor_sync(FULL_MASK, hits, o);
-            heavy += __shfl_xor_sync(FULL_MASK, heavy, o);
-            fe += __shfl_xor_sync(FULL_MASK, fe, o);
-            if constexpr (STATS == 1) {
+        // the warp's counts
+        fe = __reduce_add_sync(FULL_MASK, fe);
+        if (fe) {
+            heavy = __any_sync(FULL_MASK, heavy);
+            if (lane == 0) {
+                atomicAdd(&cnt->fedges, fe);
+                if (heavy) cnt->heavy = 1;
+            }
+        }
+        if constexpr (STATS == 1) {
+            for (int o = 16; o > 0; o >>= 1) {
                 ls += __shfl_xor_sync(FULL_MASK, ls, o);
                 lq += __shfl_xor_sync(FULL_MASK, lq, o);
                 lm = fmaxf(lm, __shfl_xor_sync(FULL_MASK, lm, o));
             }
-        }
-        if (lane == 0) {
-            r_hits[wib] = hits; r_heavy[wib] = heavy; r_fe[wib] = fe;
-            r_ls[wib] = ls; r_lq[wib] = lq; r_lm[wib] = lm;
-        }
-        __syncthreads();
-        if (wib == 0) {                                  // the block's totals: one warp, in parallel
-            ClusterCounts c{};
-            c.frontier = r_hits[lane]; c.heavy = r_heavy[lane]; c.fedges = r_fe[lane];
-            c.ls = r_ls[lane]; c.lq = r_lq[lane]; c.lm = r_lm[lane];
-            for (int o = 16; o > 0; o >>= 1) {
-                c.frontier += __shfl_xor_sync(FULL_MASK, c.frontier, o);
-                c.heavy += __shfl_xor_sync(FULL_MASK, c.heavy, o);
-                c.fedges += __shfl_xor_sync(FULL_MASK, c.fedges, o);
-                c.ls += __shfl_xor_sync(FULL_MASK, c.ls, o);
-                c.lq += __shfl_xor_sync(FULL_MASK, c.lq, o);
-                c.lm = fmaxf(c.lm, __shfl_xor_sync(FULL_MASK, c.lm, o));
+            if (lane == 0 && ls) {
+                atomicAdd(&cnt->ls, ls);
+                atomicAdd(&cnt->lq, lq);
+                atomicMax(&cnt->lm_bits, __float_as_uint(lm));
             }
-            c.listed = min(s_n, CLUSTER_LIST);
-            if (lane == 0) s_cnt[p] = c;
         }
         cl.sync();                                       // every block's counts, list and overflow are out
-        if (wib == 0) {                                  // the cluster's totals, read by one warp
-            ClusterCounts c{};
-            if (lane < CLUSTER_CTAS) c = *cl.map_shared_rank(&s_cnt[p], lane);
-            uint32_t incl = c.listed;                    // prefix of the lists over ranks
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL_MASK, incl, o);
-                if (lane >= static_cast<unsigned>(o)) incl += y;
-            }
-            if (lane < CLUSTER_CTAS) s_pre[lane + 1] = incl;
-            if (lane == 0) s_pre[0] = 0;
-            for (int o = 16; o > 0; o >>= 1) {
-                c.frontier += __shfl_xor_sync(FULL_MASK, c.frontier, o);
-                c.listed += __shfl_xor_sync(FULL_MASK, c.listed, o);
-                c.heavy += __shfl_xor_sync(FULL_MASK, c.heavy, o);
-                c.fedges += __shfl_xor_sync(FULL_MASK, c.fedges, o);
-                c.ls += __shfl_xor_sync(FULL_MASK, c.ls, o);
-                c.lq += __shfl_xor_sync(FULL_MASK, c.lq, o);
-                c.lm = fmaxf(c.lm, __shfl_xor_sync(FULL_MASK, c.lm, o));
-            }
-            if (lane == 0) s_tot = c;
+        // The cluster's totals, read by every warp for itself: lane q holds
+        // block q's list length and the exclusive prefix of the lists.
+        if (tid == 0) s_cnt[(L + 2) % 3] = ClusterCounts{};     // last read before this barrier, next used after another
+        uint4 c = make_uint4(0u, 0u, 0u, 0u);
+        if (lane < CLUSTER_CTAS) c = *reinterpret_cast<const uint4 *>(cl.map_shared_rank(cnt, lane));
+        const uint32_t listed = min(c.x, CLUSTER_LIST);
+        uint32_t pre = listed;
+#pragma unroll
+        for (uint32_t o = 1; o < CLUSTER_CTAS; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL_MASK, pre, o);
+            if (lane >= o) pre += y;
         }
-        __syncthreads();
-        const uint32_t f = s_tot.frontier, listed_all = s_tot.listed;
-        const unsigned long long fe_all = s_tot.fedges;
-        const unsigned long long ls_all = s_tot.ls, lq_all = s_tot.lq;
-        const float lm_all = s_tot.lm;
-        if (f == 0 || f > CLUSTER_CAP || fe_all > CLUSTER_EDGE_CAP || listed_all < f || s_tot.heavy ||
+        const uint32_t listed_all = __shfl_sync(FULL_MASK, pre, CLUSTER_CTAS - 1);
+        pre -= listed;
+        const uint32_t f = __reduce_add_sync(FULL_MASK, c.x), longest = __reduce_max_sync(FULL_MASK, listed);
+        const unsigned long long fe_all = __reduce_add_sync(FULL_MASK, c.y);
+        const uint32_t any_heavy = __reduce_or_sync(FULL_MASK, c.z), mine = __shfl_sync(FULL_MASK, listed, rank);
+        unsigned long long ls_all = 0, lq_all = 0;
+        float lm_all = 0.f;
+        if constexpr (STATS == 1) {
+            if (leader) {
+                for (unsigned q = 0; q < CLUSTER_CTAS; q++) {
+                    const ClusterCounts *h = cl.map_shared_rank(cnt, q);
+                    ls_all += h->ls; lq_all += h->lq;
+                    lm_all = fmaxf(lm_all, __uint_as_float(h->lm_bits));
+                }
+            }
+        }
+        if (f == 0 || f > CLUSTER_CAP || fe_all > CLUSTER_EDGE_CAP || listed_all < f || any_heavy ||
             static_cast<uint32_t>(L) + 2 > max_levels) {
             // hand level L to the step kernel: the next queue (overflow first,
             // then the blocks' lists) and the level's slot
-            const uint32_t at = (f - listed_all) + s_pre[rank], mine = s_cnt[p].listed;
+            const uint32_t at = (f - listed_all) + __shfl_sync(FULL_MASK, pre, rank);
             for (uint32_t i = tid; i < mine; i += CLUSTER_THREADS) qnext[at + i] = nv[i];
             unsigned long long hls = ls_all, hlq = lq_all;
             float hlm = lm_all;
@@ -1168,7 +1164,7 @@ k_bfs_cluster(BfsArgs a)
                     const float l = __log2f(1.0f + static_cast<float>(deg));
                     ls += lsum_fx(l); lq += lsq_fx(l); lm = fmaxf(lm, l);
                 };
-                for (uint32_t i = tid; i < mine; i += CLUSTER_THREADS) add(ne[i] - ns[i]);
+                for (uint32_t i = tid; i < mine; i += CLUSTER_THREADS) add(nse[i].y - nse[i].x);
                 const uint32_t ov = f - listed_all, per = (ov + CLUSTER_CTAS - 1) / CLUSTER_CTAS;
                 const uint32_t ob = min(ov, rank * per), oe = min(ov, ob + per);
                 for (uint32_t i = ob + tid; i < oe; i += CLUSTER_THREADS) {
@@ -1183,7 +1179,8 @@ k_bfs_cluster(BfsArgs a)
                 if (lane == 0) { r_ls[wib] = ls; r_lq[wib] = lq; r_lm[wib] = lm; }
                 __syncthreads();
                 if (wib == 0) {
-                    ls = r_ls[lane]; lq = r_lq[lane]; lm = r_lm[lane];
+                    constexpr unsigned WARPS = CLUSTER_THREADS / 32;
+                    ls = lane < WARPS ? r_ls[lane] : 0; lq = lane < WARPS ? r_lq[lane] : 0; lm = lane < WARPS ? r_lm[lane] : 0.f;
                     for (int o = 16; o > 0; o >>= 1) {
                         ls += __shfl_xor_sync(FULL_MASK, ls, o);
                         lq += __shfl_xor_sync(FULL_MASK, lq, o);
@@ -1211,39 +1208,49 @@ k_bfs_cluster(BfsArgs a)
                 slot->lmax_bits = __float_as_uint(hlm);
                 slot->heavy = 0;
                 ctl->skip = 1;
+                ctl->visited += visited;                 // the step kernel's bookkeeping for the levels before
+                ctl->traversed += traversed;
+                ctl->levels_done = static_cast<uint32_t>(L);
+                ctl->depth = L;
             }
             cl.sync();                                   // no block leaves while others may read its shared memory
             return;
         }
-        if (leader) {                                      // the step kernel's bookkeeping for level L
-            LevelSlot sl;
-            sl.frontier = f;
-            sl.qlen = f;
-            sl.fedges = fe_all;
-            sl.lsum = ls_all;
-            sl.lsq = lq_all;
-            sl.lmax_bits = __float_as_uint(lm_all);
-            sl.heavy = static_cast<uint32_t>(ctl->variant);
-            if (a.log && static_cast<uint32_t>(L) < a.log_cap) a.log[L] = sl;
-            ctl->visited += f;
-            ctl->traversed += fe_all;
-            ctl->levels_done = static_cast<uint32_t>(L) + 1;
-            ctl->depth = L + 1;
-        }
-        // this block's equal share of the next frontier, gathered from the
-        // blocks' next lists (rank order) into the level buffer
-        {
-            const uint32_t per = (f + CLUSTER_CTAS - 1) / CLUSTER_CTAS;
-            const uint32_t b = min(f, rank * per), cnt = min(per, f - b);
-            for (uint32_t i = tid; i < cnt; i += CLUSTER_THREADS) {
-                const uint32_t j = b + i;
-                unsigned q = 0;
-                while (q + 1 < CLUSTER_CTAS && s_pre[q + 1] <= j) q++;
-                const uint32_t k = j - s_pre[q];
-                lst_s[0][i] = *cl.map_shared_rank(ns + k, q);
-                lst_e[0][i] = *cl.map_shared_rank(ne + k, q);
+        if (leader) {
+            if (a.log && static_cast<uint32_t>(L) < a.log_cap) {
+                LevelSlot sl;
+                sl.frontier = f;
+                sl.qlen = f;
+                sl.fedges = fe_all;
+                sl.lsum = ls_all;
+                sl.lsq = lq_all;
+                sl.lmax_bits = __float_as_uint(lm_all);
+                sl.heavy = static_cast<uint32_t>(ctl->variant);
+                a.log[L] = sl;
             }
-            if (tid == 0) s_cur_n = cnt;
+            visited += f;
+            traversed += fe_all;
+        }
+        if (longest <= CLUSTER_KEEP) {                   // short lists stay where they were found
+            cur = nse;
+            ncur = mine;
+        } else {
+            // this block's equal share of the next frontier, gathered from the
+            // blocks' next lists (rank order)
+            const uint32_t per = (f + CLUSTER_CTAS - 1) / CLUSTER_CTAS;
+            const uint32_t b = min(f, rank * per);
+            ncur = min(per, f - b);
+            for (uint32_t i0 = wib * 32; i0 < ncur; i0 += CLUSTER_THREADS) {
+                const uint32_t i = i0 + lane, j = b + i;
+                unsigned q = 0;
+#pragma unroll
+                for (unsigned r = 1; r < CLUSTER_CTAS; r++)
+                    if (__shfl_sync(FULL_MASK, pre, r) <= j) q = r;
+                const uint32_t k = j - __shfl_sync(FULL_MASK, pre, q);
+                if (i < ncur) share[i] = *cl.map_shared_rank(nse + k, q);
+            }
+            __syncthreads();
+            cur = share;
         }
         p ^= 1;
         L++;

@@ -39,8 +39,9 @@ size_t bfs_cluster_smem() { return CLUSTER_SMEM; }
 
 int bfs_cluster_prepare()
 {
-    for (BfsKernelFn k : {k_bfs_cluster<0>, k_bfs_cluster<1>, k_bfs_cluster<2>})
+    for (BfsKernelFn k : {k_bfs_cluster<0>, k_bfs_cluster<1>, k_bfs_cluster<2>}) {
         BW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(CLUSTER_SMEM)));
+    }
     return BW_OK;
 }
 

@@ -255,7 +255,7 @@ BfsKernelFn bfs_cluster_kernel(int stats);
 size_t bfs_cluster_smem();                    // its dynamic shared memory
 int bfs_cluster_prepare();                    // allows that much on the current device
 constexpr unsigned CLUSTER_CTAS = 8;
-constexpr unsigned CLUSTER_THREADS = 1024;
+constexpr unsigned CLUSTER_THREADS = 512;
 constexpr uint32_t CLUSTER_LIST = 4096;            // frontier entries per block list
 constexpr uint32_t CLUSTER_CAP = CLUSTER_LIST * CLUSTER_CTAS;   // frontier vertices the cluster kernel takes
 constexpr unsigned long long CLUSTER_EDGE_CAP = 65536;        // and their out-edges
