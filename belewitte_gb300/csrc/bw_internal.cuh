@@ -205,6 +205,36 @@ int ensure_level_events(bw_context *ctx, uint32_t count);
 
 inline cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
 
+#if defined(__CUDACC__)
+// A chain of short kernels: each is launched while the one before it runs
+// (early: the launch attribute), and waits before its first access, so that
+// launching costs the chain nothing.  A kernel launched so begins with
+// chain_wait() in every thread (without the attribute it does nothing); what
+// the kernels before it wrote is not read through the non-coherent path
+// (__ldg), whose lines may be older than the wait.
+__device__ __forceinline__ void chain_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template<class Kernel, class... Args>
+cudaError_t launch_chained(Kernel k, unsigned grid, unsigned block, size_t smem, cudaStream_t s, bool early,
+                           Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k, args...);
+}
+#endif
+
 // BW_LAUNCH_L2_WINDOW: an access-policy window that keeps [base, base +
 // bytes) persisting in L2 for the kernels of `s` (and of graphs captured
 // from it), with a persisting carve-out of the same size (at most the

@@ -400,6 +400,7 @@ __device__ __forceinline__ float consolidate_vertex(const PrArgs &a, float acc, 
 }
 __global__ void __launch_bounds__(256) k_consolidate_div(PrArgs a, int rowlen)
 {
+    chain_wait();
     float dsum = 0.0f;
     const uint64_t n = a.n;
     const uint32_t *deg = rowlen ? a.fwd_v : a.deg;
@@ -435,12 +436,13 @@ __global__ void __launch_bounds__(256) k_consolidate_div(PrArgs a, int rowlen)
 template<int LAYOUT>  // 0 fwd SoA, 2 fwd AoS
 __global__ void __launch_bounds__(256) k_pr_edge(PrArgs a)
 {
+    chain_wait();
     const uint64_t m = a.m;
     for (uint64_t e = gtid(); e < m; e += gthreads()) {
         uint32_t src, dst;
         if constexpr (LAYOUT == 0) { src = __ldcs(a.fwd_in + e); dst = __ldcs(a.fwd_e + e); }
         else { const uint2 p = __ldcs(a.fwd_s + e); src = p.x; dst = p.y; }
-        atomicAdd(&a.acc[dst], __ldg(a.contrib_in + src));
+        atomicAdd(&a.acc[dst], __ldca(a.contrib_in + src));
     }
 }
 
@@ -486,6 +488,7 @@ __device__ __forceinline__ void add_runs(float *acc, const uint4 &k, const float
 template<bool AOS, int U>
 __global__ void __launch_bounds__(256) k_pr_edge_runs(PrArgs a)
 {
+    chain_wait();
     const unsigned lane = threadIdx.x & 31;
     const uint64_t warp = gtid() >> 5, warps = gthreads() >> 5, m = a.m;
     const bool wide = AOS ? (reinterpret_cast<uintptr_t>(a.rev_s) & 15) == 0
@@ -518,10 +521,10 @@ __global__ void __launch_bounds__(256) k_pr_edge_runs(PrArgs a)
         float4 v[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            v[u].x = dst[u].x != NO_DST ? __ldg(a.contrib_in + src[u].x) : 0.0f;
-            v[u].y = dst[u].y != NO_DST ? __ldg(a.contrib_in + src[u].y) : 0.0f;
-            v[u].z = dst[u].z != NO_DST ? __ldg(a.contrib_in + src[u].z) : 0.0f;
-            v[u].w = dst[u].w != NO_DST ? __ldg(a.contrib_in + src[u].w) : 0.0f;
+            v[u].x = dst[u].x != NO_DST ? __ldca(a.contrib_in + src[u].x) : 0.0f;
+            v[u].y = dst[u].y != NO_DST ? __ldca(a.contrib_in + src[u].y) : 0.0f;
+            v[u].z = dst[u].z != NO_DST ? __ldca(a.contrib_in + src[u].z) : 0.0f;
+            v[u].w = dst[u].w != NO_DST ? __ldca(a.contrib_in + src[u].w) : 0.0f;
         }
 #pragma unroll
         for (int u = 0; u < U; u++) add_runs(a.acc, dst[u], v[u], lane);
@@ -611,6 +614,7 @@ __global__ void __launch_bounds__(256) k_hot_translate(const uint32_t *__restric
 template<int LAYOUT>  // 0 fwd SoA, 2 fwd AoS
 __global__ void __launch_bounds__(HOT_THREADS) k_pr_edge_hot(PrArgs a)
 {
+    chain_wait();
     extern __shared__ float hot[];                 // HOT_SLOTS floats
     const uint32_t slots = *a.hot_count;
     for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) hot[i] = 0.0f;
@@ -624,7 +628,7 @@ __global__ void __launch_bounds__(HOT_THREADS) k_pr_edge_hot(PrArgs a)
         uint32_t src, dst;
         if constexpr (LAYOUT == 0) { src = __ldcs(a.fwd_in + e); dst = __ldcs(a.hot_dst + e); }
         else { const uint2 p = __ldcs(a.hot_pairs + e); src = p.x; dst = p.y; }
-        const float val = __ldg(a.contrib_in + src);
+        const float val = __ldca(a.contrib_in + src);
         if (dst & HOT_BIT) atomicAdd(&hot[dst & ~HOT_BIT], val);
         else atomicAdd(&a.acc[dst], val);
     }
@@ -665,6 +669,7 @@ __device__ __forceinline__ void enqueue_tiles(const PrArgs &a, uint32_t unit, ui
 
 __global__ void __launch_bounds__(256) k_pr_vertex_push(PrArgs a)
 {
+    chain_wait();
     const unsigned lane = threadIdx.x & 31;
     for (uint64_t w0 = gtid() - lane; w0 < a.n; w0 += gthreads()) {
         const uint64_t v = w0 + lane;
@@ -708,6 +713,7 @@ __global__ void __launch_bounds__(256) k_pr_vertex_push(PrArgs a)
 // each lane finds the row of its edge by a cursor over the staged offsets.
 __global__ void __launch_bounds__(512) k_pr_vertex_push_warp(PrArgs a)
 {
+    chain_wait();
     extern __shared__ uint32_t smem[];
     const uint32_t W = a.warp_size, C = a.chunk_size;
     const uint32_t per_block = blockDim.x / W, vw = threadIdx.x / W, lane = threadIdx.x % W;
@@ -819,6 +825,7 @@ __device__ __forceinline__ float finish_vertex(const PrArgs &a, uint64_t v, floa
 template<bool NODIV>
 __global__ void __launch_bounds__(512) k_pr_vertex_pull_warp(PrArgs a)
 {
+    chain_wait();
     extern __shared__ uint32_t smem[];
     const uint32_t W = a.warp_size, C = a.chunk_size;
     const uint32_t per_block = blockDim.x / W, vw = threadIdx.x / W, lane = threadIdx.x % W;
@@ -892,6 +899,7 @@ __global__ void __launch_bounds__(512) k_pr_vertex_pull_warp(PrArgs a)
 template<int MODE>   // 0 vertex-push, 1 vertex-push-warp, 2 vertex-pull-warp, 3 vertex-pull-warp-nodiv
 __global__ void __launch_bounds__(256) k_pr_heavy_tiles(PrArgs a)
 {
+    chain_wait();
     constexpr uint32_t NO_ROW = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31;
     const uint32_t tiles = min(a.heavy_ctr[0], a.heavy_cap);
@@ -984,6 +992,7 @@ __global__ void __launch_bounds__(256) k_pr_heavy_tiles(PrArgs a)
 template<bool NODIV>
 __global__ void __launch_bounds__(256) k_pr_heavy_finish(PrArgs a)
 {
+    chain_wait();
     const unsigned lane = threadIdx.x & 31;
     const uint64_t warp = gtid() >> 5, warps = gthreads() >> 5;
     const uint32_t chunks = a.heavy_ctr[3];
@@ -1480,7 +1489,7 @@ __device__ __noinline__ float batch_sequential_sum(const float *vals, uint32_t b
 template<bool L1 = false>
 __device__ __forceinline__ float gather1(const float *__restrict__ src, const float *hub, uint32_t hubs, uint32_t i)
 {
-    if constexpr (L1) return __ldg(src + i);          // packed graphs
+    if constexpr (L1) return __ldca(src + i);         // packed graphs
     // L2 only: random lines would only evict one another from L1 (measured
     // on GB300: ER(4M, 67M) 278 -> 268 us per iteration; reading the next
     // tier of hubs through L1 instead gained nothing on R-MAT-22)
@@ -1831,6 +1840,7 @@ template<bool NODIV, int BLOCK, bool FIRST = false, bool MULTI = false>
 __global__ void __launch_bounds__(BLOCK, pull_min_blocks(BLOCK)) k_pr_pull_items(PrArgs a)
 {
     constexpr int PULL_WARPS = BLOCK / 32;
+    chain_wait();
     resolve_args(a);
     extern __shared__ __align__(16) float smem_f[];
     const unsigned lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1845,7 +1855,7 @@ __global__ void __launch_bounds__(BLOCK, pull_min_blocks(BLOCK)) k_pr_pull_items
     float *hub = smem_f + PULL_WARPS * (PULL_BUF + 33);
     const uint32_t hubs = pk ? 0u : a.hub_count;       // multiple of 4
     for (uint32_t i = threadIdx.x; i < hubs / 4; i += blockDim.x)
-        reinterpret_cast<float4 *>(hub)[i] = __ldg(reinterpret_cast<const float4 *>(src) + i);
+        reinterpret_cast<float4 *>(hub)[i] = __ldcg(reinterpret_cast<const float4 *>(src) + i);
     __syncthreads();
     float dsum = 0.0f;
     // Packed graphs: a block takes a chunk of items in list order at a time (at
@@ -1971,6 +1981,7 @@ template<bool NODIV, bool MULTI, uint32_t STAGES, int BLOCKS>
 __global__ void __launch_bounds__(LONG_SUM_THREADS, BLOCKS) k_pr_long_sums(PrArgs a, uint32_t *ctr)
 {
     extern __shared__ __align__(16) float long_smem[];   // per warp: the batch ring or a piece's stage
+    chain_wait();
     resolve_args(a);
     const unsigned lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     float *const ring = long_smem + wib * long_sum_warp_smem(STAGES);
@@ -2301,98 +2312,96 @@ void free_run(PrRun &run, cudaStream_t s)
 
 // The long-row sums of one iteration of the work-list variants.
 template<bool NODIV, bool MULTI, uint32_t STAGES, int BLOCKS>
-void launch_long_sums_as(const bw_context *ctx, const PrArgs &a, cudaStream_t s)
+cudaError_t launch_long_sums_as(const bw_context *ctx, const PrArgs &a, cudaStream_t s, bool early)
 {
     constexpr size_t smem = long_sum_smem(STAGES);
     auto k = k_pr_long_sums<NODIV, MULTI, STAGES, BLOCKS>;
-    // (no-op after the first call; a failure leaves the launch to report it)
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    k<<<ctx->sm_count * BLOCKS, LONG_SUM_THREADS, smem, s>>>(a, a.sum_ctr);
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    return launch_chained(k, ctx->sm_count * BLOCKS, LONG_SUM_THREADS, smem, s, early, a, a.sum_ctr);
 }
 template<bool NODIV, bool MULTI = false>
-void launch_long_sums(const bw_context *ctx, const PrArgs &a, cudaStream_t s)
+cudaError_t launch_long_sums(const bw_context *ctx, const PrArgs &a, cudaStream_t s, bool early = false)
 {
-    if (a.m < SUM_SMALL_EDGES) launch_long_sums_as<NODIV, MULTI, SUM_STAGES_SMALL, SUM_BLOCKS_SMALL>(ctx, a, s);
-    else launch_long_sums_as<NODIV, MULTI, SUM_STAGES, SUM_BLOCKS>(ctx, a, s);
+    if (a.m < SUM_SMALL_EDGES)
+        return launch_long_sums_as<NODIV, MULTI, SUM_STAGES_SMALL, SUM_BLOCKS_SMALL>(ctx, a, s, early);
+    return launch_long_sums_as<NODIV, MULTI, SUM_STAGES, SUM_BLOCKS>(ctx, a, s, early);
 }
 
 // The work-list kernel of the div variants; the first iteration's instance
 // translates the sources when first_pk is set.
-void launch_pull_items_div(const PrArgs &a, const Geometry &geo, cudaStream_t s)
+cudaError_t launch_pull_items_div(const PrArgs &a, const Geometry &geo, cudaStream_t s, bool early)
 {
     const size_t smem = geo.smem + a.hub_count * 4;
-    if (geo.block == PULL_WIDE) {
-        if (a.first_pk) k_pr_pull_items<false, PULL_WIDE, true><<<geo.grid, geo.block, smem, s>>>(a);
-        else k_pr_pull_items<false, PULL_WIDE><<<geo.grid, geo.block, smem, s>>>(a);
-    } else {
-        if (a.first_pk) k_pr_pull_items<false, PULL_NARROW, true><<<geo.grid, geo.block, smem, s>>>(a);
-        else k_pr_pull_items<false, PULL_NARROW><<<geo.grid, geo.block, smem, s>>>(a);
-    }
+    auto k = geo.block == PULL_WIDE ? (a.first_pk ? k_pr_pull_items<false, PULL_WIDE, true> : k_pr_pull_items<false, PULL_WIDE>)
+                                    : (a.first_pk ? k_pr_pull_items<false, PULL_NARROW, true> : k_pr_pull_items<false, PULL_NARROW>);
+    return launch_chained(k, geo.grid, geo.block, smem, s, early, a);
 }
 
-int launch_iteration(bw_context *ctx, int variant, PrArgs &a, const Geometry &geo, cudaStream_t s)
+// early: the iterations' kernels are launched as a chain (chain_wait), except
+// where each iteration is timed.  30 iterations on GB300 (device, us): R-MAT-14
+// rev-edge-list 257 -> 164, vertex-pull 687 -> 586; the 1531 x 2049 grid's
+// vertex-push 1066 -> 878; R-MAT-22 vertex-pull 8412 -> 8363.  (Both loop modes:
+// the iterations captured into one CUDA graph took longer at every length and
+// size measured, 30 iterations of the first 306 us, 200 of them 1675 for 1024.)
+int launch_iteration(bw_context *ctx, int variant, PrArgs &a, const Geometry &geo, cudaStream_t s, bool early)
 {
+    const unsigned sms = static_cast<unsigned>(ctx->sm_count);
+    auto run = [&](auto k, unsigned grid, unsigned block, size_t smem) {
+        ctx->launches++;
+        return launch_chained(k, grid, block, smem, s, early, a);
+    };
+    auto tiles = [&](auto k) { return run(k, sms * 4, 256, 0); };
     switch (variant) {
       case PR_EDGE_LIST:
-        if (a.hot_dst) k_pr_edge_hot<0><<<ctx->sm_count * 2, HOT_THREADS, HOT_SLOTS * sizeof(float), s>>>(a);
-        else k_pr_edge<0><<<geo.grid, geo.block, 0, s>>>(a);
+        if (a.hot_dst) BW_CUDA(run(k_pr_edge_hot<0>, sms * 2, HOT_THREADS, HOT_SLOTS * sizeof(float)));
+        else BW_CUDA(run(k_pr_edge<0>, geo.grid, geo.block, 0));
         break;
       case PR_REV_EDGE_LIST:
-        if (a.m < RUN_WIDE_EDGES) k_pr_edge_runs<false, 1><<<geo.grid, geo.block, 0, s>>>(a);
-        else k_pr_edge_runs<false, 2><<<geo.grid, geo.block, 0, s>>>(a);
+        BW_CUDA(run(a.m < RUN_WIDE_EDGES ? k_pr_edge_runs<false, 1> : k_pr_edge_runs<false, 2>, geo.grid, geo.block, 0));
         break;
       case PR_STRUCT_EDGE_LIST:
-        if (a.hot_pairs) k_pr_edge_hot<2><<<ctx->sm_count * 2, HOT_THREADS, HOT_SLOTS * sizeof(float), s>>>(a);
-        else k_pr_edge<2><<<geo.grid, geo.block, 0, s>>>(a);
+        if (a.hot_pairs) BW_CUDA(run(k_pr_edge_hot<2>, sms * 2, HOT_THREADS, HOT_SLOTS * sizeof(float)));
+        else BW_CUDA(run(k_pr_edge<2>, geo.grid, geo.block, 0));
         break;
       case PR_REV_STRUCT_EDGE_LIST:
-        if (a.m < RUN_WIDE_EDGES) k_pr_edge_runs<true, 1><<<geo.grid, geo.block, 0, s>>>(a);
-        else k_pr_edge_runs<true, 2><<<geo.grid, geo.block, 0, s>>>(a);
+        BW_CUDA(run(a.m < RUN_WIDE_EDGES ? k_pr_edge_runs<true, 1> : k_pr_edge_runs<true, 2>, geo.grid, geo.block, 0));
         break;
       case PR_VERTEX_PUSH:
-        k_pr_vertex_push<<<geo.grid, geo.block, 0, s>>>(a);
-        k_pr_heavy_tiles<0><<<ctx->sm_count * 4, 256, 0, s>>>(a);
-        ctx->launches++;
+        BW_CUDA(run(k_pr_vertex_push, geo.grid, geo.block, 0));
+        BW_CUDA(tiles(k_pr_heavy_tiles<0>));
         break;
       case PR_VERTEX_PUSH_WARP:
-        k_pr_vertex_push_warp<<<geo.grid, geo.block, geo.smem, s>>>(a);
-        k_pr_heavy_tiles<1><<<ctx->sm_count * 4, 256, 0, s>>>(a);
-        ctx->launches++;
+        BW_CUDA(run(k_pr_vertex_push_warp, geo.grid, geo.block, geo.smem));
+        BW_CUDA(tiles(k_pr_heavy_tiles<1>));
         break;
       case PR_VERTEX_PULL:
-        launch_pull_items_div(a, geo, s);
-        launch_long_sums<false>(ctx, a, s);
-        ctx->launches++;
+      case PR_PULL_SEGMENTED:
+        // (pull-segmented: the vertex-pull kernel pair under its own tuned shape)
+        BW_CUDA(launch_pull_items_div(a, geo, s, early));
+        BW_CUDA(launch_long_sums<false>(ctx, a, s, early));
+        ctx->launches += 2;
         break;
       case PR_VERTEX_PULL_NODIV:
-        if (geo.block == PULL_WIDE) k_pr_pull_items<true, PULL_WIDE><<<geo.grid, geo.block, geo.smem + a.hub_count * 4, s>>>(a);
-        else k_pr_pull_items<true, PULL_NARROW><<<geo.grid, geo.block, geo.smem + a.hub_count * 4, s>>>(a);
-        launch_long_sums<true>(ctx, a, s);
+        BW_CUDA(run(geo.block == PULL_WIDE ? k_pr_pull_items<true, PULL_WIDE> : k_pr_pull_items<true, PULL_NARROW>, geo.grid,
+                    geo.block, geo.smem + a.hub_count * 4));
+        BW_CUDA(launch_long_sums<true>(ctx, a, s, early));
         ctx->launches++;
         break;
       case PR_VERTEX_PULL_WARP:
-        k_pr_vertex_pull_warp<false><<<geo.grid, geo.block, geo.smem, s>>>(a);
-        k_pr_heavy_tiles<2><<<ctx->sm_count * 4, 256, 0, s>>>(a);
-        k_pr_heavy_finish<false><<<ctx->sm_count * 2, 256, 0, s>>>(a);
-        ctx->launches += 2;
+        BW_CUDA(run(k_pr_vertex_pull_warp<false>, geo.grid, geo.block, geo.smem));
+        BW_CUDA(tiles(k_pr_heavy_tiles<2>));
+        BW_CUDA(run(k_pr_heavy_finish<false>, sms * 2, 256, 0));
         break;
       case PR_VERTEX_PULL_WARP_NODIV:
-        k_pr_vertex_pull_warp<true><<<geo.grid, geo.block, geo.smem, s>>>(a);
-        k_pr_heavy_tiles<3><<<ctx->sm_count * 4, 256, 0, s>>>(a);
-        k_pr_heavy_finish<true><<<ctx->sm_count * 2, 256, 0, s>>>(a);
-        ctx->launches += 2;
-        break;
-      case PR_PULL_SEGMENTED:
-        // the vertex-pull kernel pair under the variant's own tuned shape
-        launch_pull_items_div(a, geo, s);
-        launch_long_sums<false>(ctx, a, s);
-        ctx->launches++;
+        BW_CUDA(run(k_pr_vertex_pull_warp<true>, geo.grid, geo.block, geo.smem));
+        BW_CUDA(tiles(k_pr_heavy_tiles<3>));
+        BW_CUDA(run(k_pr_heavy_finish<true>, sms * 2, 256, 0));
         break;
       default: return BW_ERR_UNKNOWN_VARIANT;
     }
-    ctx->launches++;
     if (!is_fused(variant)) {
-        k_consolidate_div<<<ctx->sm_count * 8, 256, 0, s>>>(a, uses_rowlen(variant) ? 1 : 0);
+        BW_CUDA(launch_chained(k_consolidate_div, sms * 8, 256, 0, s, early, a, uses_rowlen(variant) ? 1 : 0));
         ctx->launches++;
     }
     BW_CUDA(cudaGetLastError());
@@ -2504,7 +2513,7 @@ int run_edgeless(bw_context *ctx, uint64_t n, bool nodiv, uint32_t iterations, f
 
 int run_pagerank(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule,
                  uint32_t schedule_len, uint32_t iterations, float *ranks,
-                 const bw_launch_config *cfg, int loop_mode, int time_iterations,
+                 const bw_launch_config *cfg, int time_iterations,
                  float *iteration_ms, bw_pagerank_result *result, float *diffs_host,
                  void *stream)
 {
@@ -2692,37 +2701,19 @@ int run_pagerank(bw_context *ctx, const bw_graph_view *g, const int32_t *schedul
     ctx->launches++;
     BW_CUDA(cudaGetLastError());
 
-    // loop_mode 1: the iterations are captured (on a private stream: the
-    // caller's may be the legacy default stream, which cannot capture) into
-    // one CUDA graph that is then launched once on the caller's stream; the
-    // launches and their order are the same
-    cudaGraph_t loop_graph = nullptr;
-    cudaStream_t ls = s;
     // BW_LAUNCH_L2_WINDOW: the gathered vector persisting in L2 (div: both
     // contribution buffers; nodiv: the rank buffers it gathers from)
-    L2Window win, win_ls;
+    L2Window win;
     const bool l2w = cfg && (cfg->flags & BW_LAUNCH_L2_WINDOW);
     const void *l2_base = nodiv ? static_cast<const void *>(nb[0] < nb[1] ? nb[0] : nb[1])
                                 : static_cast<const void *>(ctx->pr_buf[0]);
     const size_t l2_bytes = nodiv ? n * sizeof(float)
                                   : static_cast<size_t>(ctx->pr_buf[1] - ctx->pr_buf[0] + n) * sizeof(float);
     if (l2w) BW_TRY(l2_window_begin(ctx, s, l2_base, l2_bytes, win));
-    if (loop_mode == 1) {
-        BW_CUDA(cudaStreamCreateWithFlags(&ls, cudaStreamNonBlocking));
-        if (l2w) {
-            const int rc = l2_window_begin(ctx, ls, l2_base, l2_bytes, win_ls, false);
-            if (rc != BW_OK) { cudaStreamDestroy(ls); return rc; }
-        }
-        const cudaError_t e = cudaStreamBeginCapture(ls, cudaStreamCaptureModeRelaxed);
-        if (e != cudaSuccess) {
-            cudaStreamDestroy(ls);
-            BW_CUDA(e);
-        }
-    }
     int loop_status = BW_OK;
     for (uint32_t j = 1; j <= iterations && loop_status == BW_OK; j++) {
         const int v = schedule[std::min<uint32_t>(j - 1, schedule_len - 1)];
-        if (time_iterations) BW_CUDA(cudaEventRecord(ctx->level_events[j - 1], ls));
+        if (time_iterations) BW_CUDA(cudaEventRecord(ctx->level_events[j - 1], s));
         a.not_last = iterations > j ? 1 : 0;
         a.diff = ctx->pr_diffs + (j - 1);
         a.first_pk = j == 1 ? rl.pk : nullptr;
@@ -2760,27 +2751,7 @@ int run_pagerank(bw_context *ctx, const bw_graph_view *g, const int32_t *schedul
         // both buffers once iterations 1 and 2 have written them
         a.count_dev = items.work ? ((!nodiv && j > 2) ? items.count_nonconst : items.count_all) : nullptr;
         Geometry geo = geometry(ctx, v, cfg);
-        loop_status = launch_iteration(ctx, v, a, geo, ls);
-    }
-    if (loop_mode == 1) {
-        const cudaError_t e = cudaStreamEndCapture(ls, &loop_graph);
-        l2_window_end(win_ls);
-        cudaStreamDestroy(ls);
-        if (loop_status == BW_OK && e != cudaSuccess) {
-            set_last_error(e, "cudaStreamEndCapture");
-            loop_status = BW_ERR_CUDA;
-        }
-        if (loop_status == BW_OK) {
-            cudaGraphExec_t exec = nullptr;
-            cudaError_t le = cudaGraphInstantiate(&exec, loop_graph, 0);
-            if (le == cudaSuccess) le = cudaGraphLaunch(exec, s);
-            if (exec) cudaGraphExecDestroy(exec);
-            if (le != cudaSuccess) {
-                set_last_error(le, "PageRank iteration graph");
-                loop_status = BW_ERR_CUDA;
-            }
-        }
-        if (loop_graph) cudaGraphDestroy(loop_graph);
+        loop_status = launch_iteration(ctx, v, a, geo, s, !time_iterations);
     }
     BW_TRY(loop_status);
     if (time_iterations) BW_CUDA(cudaEventRecord(ctx->level_events[iterations], s));
@@ -2840,10 +2811,10 @@ int bw_pagerank_variant_reps(int variant)
 
 int bw_pagerank_run(bw_context *ctx, const bw_graph_view *g, int variant,
                     uint32_t iterations, float *ranks, const bw_launch_config *cfg,
-                    int loop_mode, bw_pagerank_result *result, float *diffs, void *stream)
+                    int /*loop_mode*/, bw_pagerank_result *result, float *diffs, void *stream)
 {
     int32_t sched = variant;
-    return run_pagerank(ctx, g, &sched, 1, iterations, ranks, cfg, loop_mode, 0, nullptr,
+    return run_pagerank(ctx, g, &sched, 1, iterations, ranks, cfg, 0, nullptr,
                         result, diffs, stream);
 }
 
@@ -2901,7 +2872,7 @@ int bw::pagerank_run_packed(bw_context *ctx, const bw_graph_view *g, const uint3
             k_pr_pull_items<false, PULL_WIDE, false, true><<<ctx->sm_count, PULL_WIDE, smem, s>>>(a);
             PrArgs b = a;
             b.work = run.sorted;
-            launch_long_sums<false, true>(ctx, b, s);
+            BW_CUDA((launch_long_sums<false, true>(ctx, b, s)));
         }
         BW_CUDA(cudaGetLastError());
         return BW_OK;
@@ -2915,10 +2886,10 @@ int bw::pagerank_run_packed(bw_context *ctx, const bw_graph_view *g, const uint3
 // A schedule run in either loop mode, with the per-iteration diffs (the
 // learned PageRank run's entry).
 int bw::pagerank_run_schedule_loop(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule,
-                                   uint32_t schedule_len, uint32_t iterations, float *ranks, int loop_mode,
+                                   uint32_t schedule_len, uint32_t iterations, float *ranks, int /*loop_mode*/,
                                    bw_pagerank_result *result, float *diffs, cudaStream_t stream)
 {
-    return run_pagerank(ctx, g, schedule, schedule_len, iterations, ranks, nullptr, loop_mode, 0, nullptr, result,
+    return run_pagerank(ctx, g, schedule, schedule_len, iterations, ranks, nullptr, 0, nullptr, result,
                         diffs, stream);
 }
 
@@ -2929,7 +2900,7 @@ int bw_pagerank_run_schedule(bw_context *ctx, const bw_graph_view *g, const int3
                              const bw_launch_config *cfg, int time_iterations,
                              float *iteration_ms, bw_pagerank_result *result, void *stream)
 {
-    return run_pagerank(ctx, g, schedule, schedule_len, iterations, ranks, cfg, BW_LOOP_HOST,
+    return run_pagerank(ctx, g, schedule, schedule_len, iterations, ranks, cfg,
                         time_iterations, iteration_ms, result, nullptr, stream);
 }
 

@@ -359,7 +359,9 @@ typedef struct bw_bfs_result {
 
 enum bw_loop_mode {
     BW_LOOP_HOST = 0,    /* host loop, one frontier read-back per level */
-    BW_LOOP_GRAPH = 1    /* CUDA graph with a device-side conditional loop */
+    BW_LOOP_GRAPH = 1    /* levels counted and ended on the device: the first ones launched by
+                          * the host, a long traversal's rest in a CUDA graph with a
+                          * conditional loop */
 };
 
 /*
@@ -420,9 +422,9 @@ typedef struct bw_pagerank_result {
  * inside the call, as the reference does inside its timed region
  * (pagerank/pagerank.cpp:102-112).  `diffs` (optional, host) receives the
  * per-iteration diff the reference reads back (pagerank.cpp:124).
- * loop_mode 0 launches the iterations from the host; 1 captures them into
- * one CUDA graph and launches it once (the same kernels in the same order;
- * the call must not itself be made inside a stream capture).
+ * Either loop_mode enqueues all iterations without waiting, each kernel
+ * launched while the one before it runs; the call must not be made inside a
+ * stream capture.
  */
 int bw_pagerank_run(bw_context *ctx, const bw_graph_view *g, int variant,
                     uint32_t iterations, float *ranks,
