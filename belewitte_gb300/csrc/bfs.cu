@@ -105,6 +105,7 @@ namespace {
 // and of the totals: written to the host, then the number it waits for.
 __global__ void k_bfs_post(const BfsCtl *ctl, int slot, BfsMail *mail, uint32_t seq)
 {
+    chain_wait();
     mail->slot = ctl->slot[slot];
     mail->edges = ctl->edges;
     __threadfence_system();
@@ -143,6 +144,7 @@ __global__ void k_bfs_step(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap,
 // Launched by the host, which waits for it.
 __global__ void k_bfs_step_post(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap, BfsMail *mail, uint32_t seq)
 {
+    chain_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     mail->stop = step_level(ctl, log, log_cap) ? 1u : 0u;
     mail->status = ctl->status;
@@ -167,10 +169,14 @@ __global__ void k_traversed(const int32_t *levels, const uint32_t *off, uint64_t
 
 struct Launch {
     BfsKernelFn k;
-    BfsKernelFn k2;    // hub kernel after frontier-push
+    BfsKernelFn k2;    // the level's second kernel: hub chunks, or edge-list's edges
     unsigned block, grid;
     size_t smem;
-    unsigned grid2;    // of the hub kernel
+    unsigned grid2;    // of k2
+    // k2 may start while k ends: not the edges' kernel, one resident wave whose
+    // blocks would gather on the SMs that are free first (BA(8.4M, 8) 1000 ->
+    // 1050 us a traversal)
+    bool k2_early = true;
 };
 
 int plan_launch(const bw_context *ctx, const bw_graph_view *g, int variant, bool side, const bw_launch_config *cfg,
@@ -254,12 +260,12 @@ BfsArgs make_args(bw_context *ctx, const bw_graph_view *g, int32_t *levels, int3
     return a;
 }
 
-int launch(const Launch &l, const BfsArgs &a, cudaStream_t s)
+// early: as a chain (chain_wait), when the host waits for nothing in between
+int launch(const Launch &l, const BfsArgs &a, cudaStream_t s, bool early = false)
 {
-    l.k<<<l.grid, l.block, l.smem, s>>>(a);
+    BW_CUDA(launch_chained(l.k, l.grid, l.block, l.smem, s, early, a));
     // the hub-chunk kernel is built for 256-thread blocks
-    if (l.k2) l.k2<<<l.grid2, 256, 0, s>>>(a);
-    BW_CUDA(cudaGetLastError());
+    if (l.k2) BW_CUDA(launch_chained(l.k2, l.grid2, 256, 0, s, early && l.k2_early, a));
     return BW_OK;
 }
 
@@ -289,8 +295,7 @@ void fill_stats(const LevelSlot &s, int variant, bw_bfs_level_stats *out)
 int post_and_wait(bw_context *ctx, int slot, cudaStream_t s)
 {
     const uint32_t seq = ++ctx->mail_seq;
-    k_bfs_post<<<1, 1, 0, s>>>(ctx->bfs_ctl, slot, ctx->mail, seq);
-    BW_CUDA(cudaGetLastError());
+    BW_CUDA(launch_chained(k_bfs_post, 1, 1, 0, s, true, static_cast<const BfsCtl *>(ctx->bfs_ctl), slot, ctx->mail, seq));
     return bfs_wait(ctx, seq, s);
 }
 
@@ -321,6 +326,7 @@ void plan_chunks(const bw_context *ctx, int variant, bool side, Launch *l)
     l->k = bfs_edge_active_kernel();
     l->block = 256;
     l->k2 = bfs_edge_chunk_kernel(variant, side);
+    l->k2_early = false;
     l->grid = static_cast<unsigned>(ctx->sm_count) * 8;
     l->grid2 = static_cast<unsigned>(ctx->sm_count) * (side ? 4 : 5);      // one resident wave
 }
@@ -371,7 +377,7 @@ int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, u
             BW_TRY(bfs_edge_ranges(ctx, g, ctx->heavy, s));
             ranges = true;
         }
-        BW_TRY(launch(plans[v], a, s));
+        BW_TRY(launch(plans[v], a, s, !time_levels));
         if (time_levels) BW_CUDA(cudaEventRecord(ctx->level_events[1], s));
         BW_TRY(post_and_wait(ctx, static_cast<int>(level % 3), s));
         const LevelSlot sl = ctx->mail->slot;
@@ -434,10 +440,10 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
         a.log = log;
         a.log_cap = log_cap;
     }
-    auto level_kernels = [&](cudaStream_t to, bool small) {
-        if (cluster_path && small) bfs_cluster_kernel(side ? 1 : 0)<<<CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), to>>>(a);
-        plan.k<<<plan.grid, plan.block, plan.smem, to>>>(a);
-        if (plan.k2) plan.k2<<<plan.grid2, 256, 0, to>>>(a);
+    auto level_kernels = [&](cudaStream_t to, bool small, bool early) -> int {
+        if (cluster_path && small)
+            BW_CUDA(launch_chained(bfs_cluster_kernel(side ? 1 : 0), CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), to, early, a));
+        return launch(plan, a, to, early);
     };
     BfsMail end{};                          // the last round's
     auto traverse = [&]() -> int {
@@ -447,10 +453,9 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
         BW_CUDA(cudaEventRecord(ctx->ev_start, s));
         if (chunks) BW_TRY(bfs_edge_ranges(ctx, g, ctx->heavy, s));
         for (uint32_t i = 0; i < DEVICE_LOOP_LAUNCHED && !end.stop; i++) {
-            level_kernels(s, i == 0 || cluster_frontier(end.slot));
+            BW_TRY(level_kernels(s, i == 0 || cluster_frontier(end.slot), true));
             const uint32_t seq = ++ctx->mail_seq;
-            k_bfs_step_post<<<1, 32, 0, s>>>(ctx->bfs_ctl, log, log_cap, ctx->mail, seq);
-            BW_CUDA(cudaGetLastError());
+            BW_CUDA(launch_chained(k_bfs_step_post, 1, 32, 0, s, true, ctx->bfs_ctl, log, log_cap, ctx->mail, seq));
             BW_TRY(bfs_wait(ctx, seq, s));
             end = *ctx->mail;
         }
@@ -463,11 +468,12 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
                 L2Window win;
                 if (window) BW_TRY(l2_window_begin(ctx, cap, levels, n * sizeof(int32_t), win, false));
                 BW_CUDA(cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-                level_kernels(cap, true);
+                const int launched = level_kernels(cap, true, false);
                 k_bfs_step<<<1, 32, 0, cap>>>(ctx->bfs_ctl, log, log_cap, handle);
                 cudaGraph_t captured = body;
                 const cudaError_t e = cudaStreamEndCapture(cap, &captured);
                 l2_window_end(win);                 // before its stream goes
+                BW_TRY(launched);
                 BW_CUDA(e);
                 return BW_OK;
             };

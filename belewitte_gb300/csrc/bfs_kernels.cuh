@@ -238,6 +238,7 @@ __device__ __forceinline__ void relax_all(int32_t *lv, int32_t nd, const uint32_
 template<int RED, bool SIDE, int LAYOUT>
 __global__ void __launch_bounds__(512) k_bfs_edge(BfsArgs a)
 {
+    chain_wait();
     const int32_t depth = level_depth(a), nd = depth + 1;
     LevelSlot *slot = &a.ctl->slot[depth % 3];
     if (blockIdx.x == 0 && threadIdx.x == 0) reset_slot(&a.ctl->slot[(depth + 1) % 3]);
@@ -326,6 +327,7 @@ constexpr uint32_t ACTIVE_BATCH = 4;                // chunks a warp looks at, 1
 
 static __global__ void __launch_bounds__(256) k_edge_active(BfsArgs a)
 {
+    chain_wait();
     constexpr uint32_t RANGE = 2 * EDGE_CHUNK;
     __shared__ uint32_t s_count[8], s_base;
     const int32_t depth = level_depth(a);
@@ -383,6 +385,7 @@ static __global__ void __launch_bounds__(256) k_edge_active(BfsArgs a)
 template<int RED, bool SIDE>
 __global__ void __launch_bounds__(256, SIDE ? 4 : 5) k_bfs_edge_chunks(BfsArgs a)
 {
+    chain_wait();
     constexpr uint32_t STEPS = EDGE_CHUNK / 128;
     const int32_t depth = level_depth(a), nd = depth + 1;
     LevelSlot *slot = &a.ctl->slot[depth % 3];
@@ -397,7 +400,7 @@ __global__ void __launch_bounds__(256, SIDE ? 4 : 5) k_bfs_edge_chunks(BfsArgs a
     };
     const uint64_t m = a.m, steps = uint64_t(slot->heavy) * STEPS, warps = gthreads() >> 5;
     for (uint64_t t0 = (gtid() >> 5) * 2; t0 < steps; t0 += warps * 2) {      // (STEPS is even)
-        const uint64_t e = uint64_t(__ldg(a.active + t0 / STEPS)) * EDGE_CHUNK + (t0 % STEPS) * 128 + 4 * lane;
+        const uint64_t e = uint64_t(__ldca(a.active + t0 / STEPS)) * EDGE_CHUNK + (t0 % STEPS) * 128 + 4 * lane;
         if (e + 128 + 4 <= m) {
             const uint4 r0 = __ldcs(reinterpret_cast<const uint4 *>(a.fwd_in + e)), r1 = __ldcs(reinterpret_cast<const uint4 *>(a.fwd_in + e + 128));
             const uint4 q0 = __ldcs(reinterpret_cast<const uint4 *>(a.fwd_e + e)), q1 = __ldcs(reinterpret_cast<const uint4 *>(a.fwd_e + e + 128));
@@ -497,6 +500,7 @@ __device__ __forceinline__ void relax_neighbours(const BfsArgs &a, const uint32_
 template<int RED, bool SIDE>
 __global__ void __launch_bounds__(512) k_bfs_vertex_push(BfsArgs a)
 {
+    chain_wait();
     const int32_t depth = level_depth(a), nd = depth + 1;
     LevelSlot *slot = &a.ctl->slot[depth % 3];
     if (blockIdx.x == 0 && threadIdx.x == 0) reset_slot(&a.ctl->slot[(depth + 1) % 3]);
@@ -572,6 +576,7 @@ constexpr int BFS_PULL_UNROLL = 4;
 template<int RED, bool SIDE>
 __global__ void __launch_bounds__(512) k_bfs_vertex_pull(BfsArgs a)
 {
+    chain_wait();
     const int32_t depth = level_depth(a), nd = depth + 1;
     LevelSlot *slot = &a.ctl->slot[depth % 3];
     if (blockIdx.x == 0 && threadIdx.x == 0) reset_slot(&a.ctl->slot[(depth + 1) % 3]);
@@ -629,6 +634,7 @@ __device__ __forceinline__ unsigned subwarp_mask(uint32_t W)
 template<int RED, bool SIDE, bool PULL>
 __global__ void __launch_bounds__(512) k_bfs_vwarp(BfsArgs a)
 {
+    chain_wait();
     extern __shared__ uint32_t smem[];
     const int32_t depth = level_depth(a), nd = depth + 1;
     LevelSlot *slot = &a.ctl->slot[depth % 3];
@@ -712,6 +718,7 @@ constexpr int FRONTIER_UNROLL = 4;
 template<bool SIDE>
 __global__ void __launch_bounds__(256) k_bfs_frontier_push(BfsArgs a)
 {
+    chain_wait();
     __shared__ uint32_t s_stage[8][WARP_STAGE];
     if (a.skip_check && *((volatile uint32_t *) &a.ctl->skip)) return;
     const int32_t depth = level_depth(a), nd = depth + 1;
@@ -781,6 +788,7 @@ __global__ void __launch_bounds__(256) k_bfs_frontier_push(BfsArgs a)
 template<bool SIDE>
 __global__ void __launch_bounds__(256) k_bfs_hub_chunks(BfsArgs a)
 {
+    chain_wait();
     __shared__ uint32_t s_stage[8][WARP_STAGE];
     if (a.skip_check && *((volatile uint32_t *) &a.ctl->skip)) return;
     const int32_t depth = level_depth(a), nd = depth + 1;
@@ -833,6 +841,7 @@ __global__ void __launch_bounds__(256) k_bfs_hub_chunks(BfsArgs a)
 template<bool SIDE>
 __global__ void __launch_bounds__(256) k_bfs_frontier_pull(BfsArgs a)
 {
+    chain_wait();
     __shared__ uint32_t s_stage[8][WARP_STAGE];
     const int32_t depth = level_depth(a), nd = depth + 1;
     LevelSlot *slot = &a.ctl->slot[depth % 3];
@@ -948,6 +957,7 @@ template<int STATS>
 __global__ void __cluster_dims__(CLUSTER_CTAS, 1, 1) __launch_bounds__(CLUSTER_THREADS)
 k_bfs_cluster(BfsArgs a)
 {
+    chain_wait();
     extern __shared__ __align__(16) uint32_t cl_lists[];
     __shared__ ClusterCounts s_cnt[3];             // by level
     __shared__ unsigned long long r_ls[CLUSTER_THREADS / 32], r_lq[CLUSTER_THREADS / 32];

@@ -454,6 +454,7 @@ __global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_next(PredictArgs a, boo
                                                               BfsMail *mail, uint32_t seq)
 {
     __shared__ bool s_stop;
+    chain_wait();
     BfsCtl *c = a.ctl;
     if (threadIdx.x == 0) s_stop = step && step_learned(c, log, log_cap);
     __syncthreads();
@@ -925,8 +926,8 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
         const PredictArgs pa{ctx->bfs_ctl, sw->params, K, sw->fallback, sw->threshold, n, m, {}, false, cluster_k};
         for (uint32_t i = 0; i < ROUNDS_LAUNCHED; i++) {
             const uint32_t seq = ++ctx->mail_seq;
-            k_bfs_next<<<1, PREDICT_THREADS, param_count(K) * sizeof(float), s>>>(pa, i > 0, log, log_cap, ctx->mail, seq);
-            BW_CUDA(cudaGetLastError());
+            BW_CUDA(launch_chained(k_bfs_next, 1, PREDICT_THREADS, param_count(K) * sizeof(float), s, true, pa, i > 0, log,
+                                   log_cap, ctx->mail, seq));
             BW_TRY(bfs_wait(ctx, seq, s));
             end = *ctx->mail;
             if (end.stop) break;
@@ -934,13 +935,14 @@ int bw_bfs_run_learned(bw_context *ctx, const bw_graph_view *g, const bw_switch_
             // the level log needs every level's statistics; otherwise only a
             // handed-over level's, which the next prediction reads
             if (sw->candidates[end.variant] == 32 && cluster_frontier(end.slot))
-                bfs_cluster_kernel(log_cap ? 1 : 2)<<<CLUSTER_CTAS, CLUSTER_THREADS, bfs_cluster_smem(), s>>>(a);
-            p.k<<<p.grid, p.block, p.smem, s>>>(a);
-            if (p.k2) p.k2<<<p.grid2, 256, 0, s>>>(a);
+                BW_CUDA(launch_chained(bfs_cluster_kernel(log_cap ? 1 : 2), CLUSTER_CTAS, CLUSTER_THREADS,
+                                       bfs_cluster_smem(), s, true, a));
+            BW_CUDA(launch_chained(p.k, p.grid, p.block, p.smem, s, true, a));
+            if (p.k2) BW_CUDA(launch_chained(p.k2, p.grid2, 256, 0, s, true, a));
             if (i + 1 == ROUNDS_LAUNCHED) {      // the graph's first round predicts: close this one
                 const uint32_t last = ++ctx->mail_seq;
-                k_bfs_next<<<1, PREDICT_THREADS, param_count(K) * sizeof(float), s>>>(pa, true, log, log_cap, ctx->mail, last);
-                BW_CUDA(cudaGetLastError());
+                BW_CUDA(launch_chained(k_bfs_next, 1, PREDICT_THREADS, param_count(K) * sizeof(float), s, true, pa, true, log,
+                                       log_cap, ctx->mail, last));
                 BW_TRY(bfs_wait(ctx, last, s));
                 end = *ctx->mail;
             }
