@@ -336,6 +336,37 @@ void chunk_args(bw_context *ctx, BfsArgs *a)
     a->active = reinterpret_cast<uint32_t *>(ctx->heavy + (a->m + EDGE_CHUNK - 1) / EDGE_CHUNK);
 }
 
+// vertex-pull levels with the frontier's filter (k_bfs_pull_filter): `frontier`
+// vertices of this level, `visited` so far.  A level of ER(1M, 8M) takes 25 to
+// 29 us with it and 44 to 47 without while the frontier is under a 256th of the
+// vertices; at a 70th 42 and 53, from a 25th on the hits cost more than the
+// filter saves.  Once half the vertices are visited the plain kernel has few
+// rows left.  Whole traversals on GB300, every level plain and with the filter:
+// ER(1M, 16M) 524 -> 373 us, ER(4M, 67M) 1607 -> 960, ER(8M, 32M) 1871 -> 1593;
+// R-MAT and BA, whose second level is dense, as before.
+constexpr uint64_t FILTERED_EDGES = uint64_t(4) << 20;
+constexpr uint64_t FILTERED_SHARE = 256;
+bool filtered(const bw_context *ctx, const bw_graph_view *g, int variant, const bw_launch_config *cfg, uint64_t frontier,
+              uint64_t visited)
+{
+    return variant >= 20 && variant < 24 && g->edge_count >= FILTERED_EDGES && !(cfg && (cfg->block_size || cfg->grid_size)) &&
+           frontier * FILTERED_SHARE <= g->vertex_count && 2 * visited <= g->vertex_count &&
+           ctx->heavy_cap * sizeof(uint2) >= FILTER_BITS / 8;
+}
+int launch_filtered(bw_context *ctx, int variant, bool side, BfsArgs a, cudaStream_t s, bool early)
+{
+    uint32_t bits = 4096;
+    while (bits < a.n && bits < FILTER_BITS) bits *= 2;
+    a.filter = reinterpret_cast<uint32_t *>(ctx->heavy);
+    a.filter_mask = bits - 1;
+    const BfsKernelFn k = bfs_pull_filter_kernel(variant % 4, side);
+    const unsigned sms = static_cast<unsigned>(ctx->sm_count);
+    BW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(FILTER_BITS / 8)));
+    BW_CUDA(launch_chained(bfs_filter_kernel(), std::min(sms * 8, bits / 32 / 8), 256, 0, s, early, a));
+    BW_CUDA(launch_chained(k, sms, 1024, bits / 8, s, early, a));
+    return BW_OK;
+}
+
 // Host-loop traversal with a per-level variant schedule.
 int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, uint32_t sched_len,
              uint32_t root, int32_t *levels, const bw_launch_config *cfg, uint32_t max_levels,
@@ -377,7 +408,12 @@ int run_host(bw_context *ctx, const bw_graph_view *g, const int32_t *schedule, u
             BW_TRY(bfs_edge_ranges(ctx, g, ctx->heavy, s));
             ranges = true;
         }
-        BW_TRY(launch(plans[v], a, s, !time_levels));
+        if (filtered(ctx, g, v, cfg, level ? ctx->mail->slot.frontier : 1, visited)) {
+            BW_TRY(launch_filtered(ctx, v, side, a, s, !time_levels));
+            ranges = false;                 // the filter lies where they did
+        } else {
+            BW_TRY(launch(plans[v], a, s, !time_levels));
+        }
         if (time_levels) BW_CUDA(cudaEventRecord(ctx->level_events[1], s));
         BW_TRY(post_and_wait(ctx, static_cast<int>(level % 3), s));
         const LevelSlot sl = ctx->mail->slot;
@@ -453,7 +489,10 @@ int run_graph(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t roo
         BW_CUDA(cudaEventRecord(ctx->ev_start, s));
         if (chunks) BW_TRY(bfs_edge_ranges(ctx, g, ctx->heavy, s));
         for (uint32_t i = 0; i < DEVICE_LOOP_LAUNCHED && !end.stop; i++) {
-            BW_TRY(level_kernels(s, i == 0 || cluster_frontier(end.slot), true));
+            if (filtered(ctx, g, variant, cfg, i ? end.slot.frontier : 1, i ? end.visited : 1))
+                BW_TRY(launch_filtered(ctx, variant, side, a, s, true));
+            else
+                BW_TRY(level_kernels(s, i == 0 || cluster_frontier(end.slot), true));
             const uint32_t seq = ++ctx->mail_seq;
             BW_CUDA(launch_chained(k_bfs_step_post, 1, 32, 0, s, true, ctx->bfs_ctl, log, log_cap, ctx->mail, seq));
             BW_TRY(bfs_wait(ctx, seq, s));

@@ -615,6 +615,91 @@ __global__ void __launch_bounds__(512) k_bfs_vertex_pull(BfsArgs a)
     side.finish_block(slot);
 }
 
+// vertex-pull while the frontier is small and most vertices are open: nearly
+// every open vertex then looks at its whole in-row in vain, an L1TEX tag for
+// each index and one for each depth.  The frontier's bits (k_bfs_filter; folded
+// to FILTER_BITS where the graph has more vertices) go to every block's shared
+// memory, and a warp streams the in-rows of 32 neighbouring vertices, one
+// contiguous range, 32 edges a load: an edge costs a bit test, and only those
+// whose bit is set look for their row and at the depth.
+static __global__ void __launch_bounds__(256) k_bfs_filter(BfsArgs a)
+{
+    chain_wait();
+    const int32_t depth = level_depth(a);
+    const int32_t *lv = a.levels;
+    const unsigned lane = threadIdx.x & 31;
+    const uint64_t words = (uint64_t(a.filter_mask) + 1) / 32, n = a.n;
+    for (uint64_t w = gtid() >> 5; w < words; w += gthreads() >> 5) {
+        uint32_t bits = 0;
+#pragma unroll 4
+        for (uint64_t v0 = w * 32; v0 < n; v0 += uint64_t(a.filter_mask) + 1) {
+            const uint64_t v = v0 + lane;
+            bits |= __ballot_sync(FULL_MASK, v < n && lv[v] == depth);
+        }
+        if (lane == 0) a.filter[w] = bits;
+    }
+}
+
+constexpr int FILTER_UNROLL = 8;
+
+template<int RED, bool SIDE>
+__global__ void __launch_bounds__(1024, 1) k_bfs_pull_filter(BfsArgs a)
+{
+    extern __shared__ __align__(16) uint32_t s_filter[];
+    chain_wait();
+    const int32_t depth = level_depth(a), nd = depth + 1;
+    LevelSlot *slot = &a.ctl->slot[depth % 3];
+    if (blockIdx.x == 0 && threadIdx.x == 0) reset_slot(&a.ctl->slot[(depth + 1) % 3]);
+    uint32_t *qnext = (depth & 1) ? a.q0 : a.q1;
+    int32_t *lv = a.levels;
+    Counter<RED> cnt;
+    Side<SIDE> side;
+    const uint32_t mask = a.filter_mask, quads = (mask + 1) / 128;
+    for (uint32_t i = threadIdx.x; i < quads; i += blockDim.x)
+        reinterpret_cast<uint4 *>(s_filter)[i] = __ldcg(reinterpret_cast<const uint4 *>(a.filter) + i);
+    __syncthreads();
+    const unsigned lane = threadIdx.x & 31;
+    const uint64_t n = a.n, stride = gthreads();
+    // the next 32 rows' bounds and depths are loaded one step ahead
+    uint32_t next_off = 0, next_end = 0;
+    int32_t next_depth = 0;
+    auto fetch = [&](uint64_t v0) {
+        if (v0 >= n) return;
+        const uint64_t v = v0 + lane;
+        next_off = __ldg(a.rev_v + min(v, n));
+        next_end = __ldg(a.rev_v + min(v0 + 32, n));
+        next_depth = v < n ? lv[v] : 0;
+    };
+    fetch(gtid() - lane);
+    for (uint64_t v0 = gtid() - lane; v0 < n; v0 += stride) {
+        const uint32_t off = next_off, end = next_end;
+        const bool open = next_depth > nd;
+        fetch(v0 + stride);
+        if (!__any_sync(FULL_MASK, open)) continue;
+        const uint32_t base = __shfl_sync(FULL_MASK, off, 0), excl = off - base, total = end - base;
+        for (uint32_t k0 = 0; k0 < total; k0 += 32 * FILTER_UNROLL) {
+            uint32_t p[FILTER_UNROLL];
+#pragma unroll
+            for (int u = 0; u < FILTER_UNROLL; u++) {
+                const uint32_t k = k0 + u * 32 + lane;
+                p[u] = k < total ? __ldcs(a.rev_e + base + k) : NO_VERTEX;
+            }
+#pragma unroll
+            for (int u = 0; u < FILTER_UNROLL; u++) {
+                const bool hit = p[u] != NO_VERTEX && (s_filter[(p[u] & mask) >> 5] >> (p[u] & 31) & 1u);
+                if (!__any_sync(FULL_MASK, hit)) continue;
+                const uint32_t w = static_cast<uint32_t>(v0) + concat_row(excl, k0 + u * 32 + lane);
+                if (hit && lv[p[u]] == depth && lv[w] > nd && atomicMin(&lv[w], nd) > nd) {
+                    cnt.hit(&slot->frontier);
+                    side.visit(a, qnext, slot, w);
+                }
+            }
+        }
+    }
+    cnt.finish(&slot->frontier);
+    side.finish_block(slot);
+}
+
 // ---------------------------------------------------------------------------
 // Virtual-warp families (bfs/vertex_push_warp.cu:19-60,
 // vertex_pull_warp.cu:17-71): a virtual warp of W lanes (W | 32) takes a

@@ -29,6 +29,22 @@ BfsKernelFn bfs_vertex_kernel(int family, int reduction, bool side)
 BfsKernelFn bfs_frontier_push_kernel(bool side)
 { return side ? k_bfs_frontier_push<true> : k_bfs_frontier_push<false>; }
 
+BfsKernelFn bfs_filter_kernel() { return k_bfs_filter; }
+
+template<int RED>
+static BfsKernelFn pick_filter(bool side)
+{ return side ? k_bfs_pull_filter<RED, true> : k_bfs_pull_filter<RED, false>; }
+
+BfsKernelFn bfs_pull_filter_kernel(int reduction, bool side)
+{
+    switch (reduction) {
+      case RED_NORMAL: return pick_filter<RED_NORMAL>(side);
+      case RED_BULK: return pick_filter<RED_BULK>(side);
+      case RED_WARP: return pick_filter<RED_WARP>(side);
+      default: return pick_filter<RED_BLOCK>(side);
+    }
+}
+
 BfsKernelFn bfs_hub_kernel(bool side)
 { return side ? k_bfs_hub_chunks<true> : k_bfs_hub_chunks<false>; }
 

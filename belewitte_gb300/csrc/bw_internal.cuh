@@ -132,7 +132,11 @@ struct BfsArgs {
     uint32_t log_cap;
     const uint2 *ranges;          // edge-list by chunk: {least, largest} source of every EDGE_CHUNK edges
     uint32_t *active;             // its chunks with work in this level (slot->heavy of them)
+    uint32_t *filter;             // k_bfs_pull_filter: the frontier's bits, filter_mask + 1 of them
+    uint32_t filter_mask;
 };
+// Bits of the frontier filter at most (128 KB of a block's shared memory).
+constexpr uint32_t FILTER_BITS = 1u << 20;
 // Edges per range: 12 bytes a chunk, in the hub-chunk queue's 64 (ensure_bfs_scratch).
 constexpr uint32_t EDGE_CHUNK = 1024;
 
@@ -270,6 +274,8 @@ using BfsKernelFn = void (*)(BfsArgs);
 BfsKernelFn bfs_edge_kernel(int layout, int reduction, bool side);
 BfsKernelFn bfs_edge_active_kernel();
 BfsKernelFn bfs_edge_chunk_kernel(int reduction, bool side);
+BfsKernelFn bfs_filter_kernel();
+BfsKernelFn bfs_pull_filter_kernel(int reduction, bool side);
 int bfs_edge_ranges(const bw_context *ctx, const bw_graph_view *g, uint2 *ranges, cudaStream_t s);
 BfsKernelFn bfs_vertex_kernel(int family, int reduction, bool side);
 BfsKernelFn bfs_frontier_push_kernel(bool side);
