@@ -353,13 +353,19 @@ struct PredictArgs {
 // hidden units, lane 0 of warp 0 takes the softmax and the decision.
 constexpr int PREDICT_THREADS = 128;
 
-__device__ void predict_level(const PredictArgs &a)
+__device__ __forceinline__ void stage_params(const PredictArgs &a)
+{
+    extern __shared__ float sp[];
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < param_count(a.K); i += PREDICT_THREADS) sp[i] = a.params[i];
+}
+
+__device__ void predict_level(const PredictArgs &a)      // after stage_params()
 {
     extern __shared__ float sp[];
     __shared__ float x[F], h1[H], h2[H], z[BW_MLP_MAX_CLASSES];
     const int tid = threadIdx.x;
-    const uint32_t K = a.K, P = param_count(K);
-    for (uint32_t i = tid; i < P; i += PREDICT_THREADS) sp[i] = a.params[i];
+    const uint32_t K = a.K;
     BfsCtl *c = a.ctl;
     const int32_t L = c->depth;
     if (a.cluster_k >= 0) {
@@ -418,7 +424,11 @@ __device__ void predict_level(const PredictArgs &a)
     }
 }
 
-__global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_predict(PredictArgs a) { predict_level(a); }
+__global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_predict(PredictArgs a)
+{
+    stage_params(a);
+    predict_level(a);
+}
 
 // After every level: its entry in the log, the totals; true when the
 // traversal is over.
@@ -454,6 +464,7 @@ __global__ void __launch_bounds__(PREDICT_THREADS) k_bfs_next(PredictArgs a, boo
                                                               BfsMail *mail, uint32_t seq)
 {
     __shared__ bool s_stop;
+    stage_params(a);                     // while the level's kernels run
     chain_wait();
     BfsCtl *c = a.ctl;
     if (threadIdx.x == 0) s_stop = step && step_learned(c, log, log_cap);
