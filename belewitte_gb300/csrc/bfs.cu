@@ -157,7 +157,7 @@ __global__ void k_bfs_step_post(BfsCtl *ctl, LevelSlot *log, uint32_t log_cap, B
 
 // Sum of out-degrees of reached vertices (TEPS numerator).  Four vertices a
 // thread and load where the arrays allow it, two loads of each in flight; one
-// atomic per block.  16.7M vertices on GB300: 100 us with one at a time, 29
+// atomic per block.  16.7M vertices on GB300: 100 us with one at a time, 26
 // so.
 __global__ void __launch_bounds__(256) k_traversed(const int32_t *levels, const uint32_t *off, uint64_t n,
                                                    unsigned long long *out)
