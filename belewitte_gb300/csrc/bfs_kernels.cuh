@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(256) k_bfs_frontier_pull(BfsArgs a)
 //    The next lists alternate between two buffers, the counts between three,
 //    so nothing needs a second cluster barrier.
 // Bound by the latency of that chain: on GB300 a level of the 2048 x 2048 grid
-// took 4.5 to 5.0 us and takes 3.1 to 4.0, of a 300 x 300 grid 4.0 and 2.7.
+// took 4.5 to 5.0 us and takes 3.1 to 4.1, of a 300 x 300 grid 4.0 and 2.6.
 // More threads a block than the frontier fills only make the barriers dearer
 // (1024 instead of 512: 3.1 and 4.4 us), fewer leave wide frontiers behind
 // (256: 2.5 us on 300 x 300, but 7.4 instead of 6.8 on 5000 x 5000); 16 blocks
@@ -1039,7 +1039,7 @@ struct __align__(16) ClusterCounts {
 // per claim, for a level log); 2 only those of a level handed over (what
 // the next level's choice reads), computed from its frontier at handover.
 template<int STATS>
-__global__ void __cluster_dims__(CLUSTER_CTAS, 1, 1) __launch_bounds__(CLUSTER_THREADS)
+__global__ void __cluster_dims__(CLUSTER_CTAS, 1, 1) __launch_bounds__(CLUSTER_THREADS, 1)
 k_bfs_cluster(BfsArgs a)
 {
     chain_wait();
@@ -1101,6 +1101,25 @@ k_bfs_cluster(BfsArgs a)
         uint32_t fe = 0, heavy = 0;
         unsigned long long ls = 0, lq = 0;
         float lm = 0.f;
+        // Next-line prefetch: where vertex ids follow the graph's geometry
+        // (grids, meshes, road networks) the wavefront reaches a claimed
+        // vertex's id neighbours within a few levels, and the first touch of
+        // their lines would put an HBM miss on a level's critical path.  Done
+        // for a lane's last claims, while the cluster barrier waits (300 x 300
+        // grid 2.77 -> 2.60 us a level, 20,000 x 50 2.66 -> 2.31).
+        uint32_t claimed[CLUSTER_UNROLL], claimed_end[CLUSTER_UNROLL];
+#pragma unroll
+        for (int jj = 0; jj < CLUSTER_UNROLL; jj++) claimed[jj] = NO_VERTEX;
+        auto prefetch = [&]() {
+#pragma unroll
+            for (int jj = 0; jj < CLUSTER_UNROLL; jj++) {
+                if (claimed[jj] == NO_VERTEX) continue;
+                const uint64_t v = claimed[jj], e = claimed_end[jj];
+                if (e + 32 < a.m) prefetch_l2(a.fwd_e + e + 32);
+                if (v + 33 <= a.n) prefetch_l2(a.fwd_v + v + 33);
+                if (v + 32 < a.n) prefetch_l2(lv + v + 32);
+            }
+        };
         // Claims up to CLUSTER_UNROLL neighbours a lane.  A level is a chain
         // of dependent accesses, so every lane's neighbours go out together:
         // their row bounds (loaded whether or not the claim wins) and their
@@ -1148,14 +1167,8 @@ k_bfs_cluster(BfsArgs a)
                         const float l = __log2f(1.0f + static_cast<float>(ue[jj] - us[jj]));
                         ls += lsum_fx(l); lq += lsq_fx(l); lm = fmaxf(lm, l);
                     }
-                    // Next-line prefetch: where vertex ids follow the graph's
-                    // geometry (grids, meshes, road networks) the wavefront
-                    // reaches u's id neighbours within a few levels, and the
-                    // first touch of their lines would put an HBM miss on the
-                    // level's critical path.
-                    if (ue[jj] + 32 < a.m) prefetch_l2(a.fwd_e + ue[jj] + 32);
-                    if (u[jj] + 33 <= a.n) prefetch_l2(a.fwd_v + u[jj] + 33);
-                    if (u[jj] + 32 < a.n) prefetch_l2(lv + u[jj] + 32);
+                    claimed[jj] = u[jj];
+                    claimed_end[jj] = ue[jj];
                 }
                 base += __popc(wm[jj]);
             }
@@ -1211,7 +1224,10 @@ k_bfs_cluster(BfsArgs a)
                 atomicMax(&cnt->lm_bits, __float_as_uint(lm));
             }
         }
-        cl.sync();                                       // every block's counts, list and overflow are out
+        // every block's counts, list and overflow are out
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        prefetch();
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
         // The cluster's totals, read by every warp for itself: lane q holds
         // block q's list length and the exclusive prefix of the lists.
         if (tid == 0) s_cnt[(L + 2) % 3] = ClusterCounts{};     // last read before this barrier, next used after another
