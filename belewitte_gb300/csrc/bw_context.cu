@@ -2,7 +2,6 @@
 // Context, scratch management, launch geometry and representation builders.
 #include <chrono>
 #include <cstdio>
-#include <cstring>
 #include <new>
 
 #include "bw_internal.cuh"
@@ -44,41 +43,6 @@ void compute_division(uint64_t count, uint32_t sm, uint32_t max_tpb,
     *grid = static_cast<uint32_t>(g);
 }
 
-template<typename T>
-static int grow(T **ptr, uint64_t count)
-{
-    if (*ptr) { cudaFree(*ptr); *ptr = nullptr; }
-    if (count == 0) count = 1;
-    BW_CUDA(cudaMalloc(reinterpret_cast<void **>(ptr), count * sizeof(T)));
-    return BW_OK;
-}
-
-int ensure_bfs_scratch(bw_context *ctx, uint64_t n, uint64_t m)
-{
-    if (!ctx->bfs_ctl) {
-        BW_CUDA(cudaMalloc(reinterpret_cast<void **>(&ctx->bfs_ctl), sizeof(BfsCtl)));
-        BW_CUDA(cudaMemset(ctx->bfs_ctl, 0, sizeof(BfsCtl)));
-        constexpr size_t at = (sizeof(BfsCtl) + 127) & ~size_t(127);       // the mail on lines of its own
-        BW_CUDA(cudaMallocHost(reinterpret_cast<void **>(&ctx->bfs_ctl_host), at + sizeof(BfsMail)));
-        ctx->mail = reinterpret_cast<BfsMail *>(reinterpret_cast<char *>(ctx->bfs_ctl_host) + at);
-        std::memset(ctx->mail, 0, sizeof(BfsMail));
-        ctx->mail_seq = 0;
-    }
-    if (n > ctx->bfs_n_cap) {
-        BW_TRY(grow(&ctx->queue[0], n));
-        BW_TRY(grow(&ctx->queue[1], n));
-        ctx->bfs_n_cap = n;
-    }
-    // Hub chunks: every queued vertex has degree > 256 and yields at most
-    // 2*deg/256 chunks of 256 edges, so 2M/256 + N/256 bounds a level.
-    uint64_t hcap = 2 * m / 256 + n / 256 + 1024;
-    if (hcap > ctx->heavy_cap) {
-        BW_TRY(grow(&ctx->heavy, hcap));
-        ctx->heavy_cap = hcap;
-    }
-    return BW_OK;
-}
-
 // A level of a few microseconds is worth polling for; a longer one (or a
 // kernel that failed, which the synchronisation reports) is not.
 int bfs_wait(bw_context *ctx, uint32_t seq, cudaStream_t s)
@@ -108,35 +72,9 @@ __global__ void k_row_lengths(const uint32_t *__restrict__ off, uint64_t n,
 int ensure_outdeg(bw_context *ctx, const bw_graph_view *g, cudaStream_t s)
 {
     if (!g->fwd_vertices) return BW_ERR_MISSING_REPRESENTATION;
-    if (g->vertex_count > ctx->outdeg_cap) {
-        BW_TRY(grow(&ctx->outdeg, g->vertex_count));
-        ctx->outdeg_cap = g->vertex_count;
-    }
+    BW_TRY(ensure_outdeg_scratch(ctx, g->vertex_count));
     k_row_lengths<<<default_grid(ctx, 4), 256, 0, s>>>(g->fwd_vertices, g->vertex_count, ctx->outdeg);
     BW_CUDA(cudaGetLastError());
-    return BW_OK;
-}
-
-int ensure_pr_scratch(bw_context *ctx, uint64_t n, uint32_t iterations)
-{
-    if (n > ctx->pr_n_cap) {
-        ctx->pr_n_cap = 0;               // until all of them have grown
-        BW_TRY(grow(&ctx->pr_acc, n));
-        // both contribution buffers in one allocation, so one L2
-        // access-policy window covers the vector every iteration gathers;
-        // the second starts on a 256-byte boundary (the kernels read both
-        // with 16-byte vector loads)
-        const uint64_t stride = (n + 63) & ~uint64_t(63);
-        BW_TRY(grow(&ctx->pr_buf[0], 2 * stride));
-        ctx->pr_buf[1] = ctx->pr_buf[0] + stride;
-        BW_TRY(grow(&ctx->pr_deg, n));
-        ctx->pr_n_cap = n;
-    }
-    uint32_t need = iterations + 1;
-    if (need > ctx->pr_diff_cap) {
-        BW_TRY(grow(&ctx->pr_diffs, need));
-        ctx->pr_diff_cap = need;
-    }
     return BW_OK;
 }
 

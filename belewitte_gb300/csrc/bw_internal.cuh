@@ -190,6 +190,7 @@ struct bw_context {
 namespace bw {
 
 int ensure_bfs_scratch(bw_context *ctx, uint64_t n, uint64_t m);
+int ensure_outdeg_scratch(bw_context *ctx, uint64_t n);
 // Waits until the device has posted `seq` to ctx->mail on stream `s`.
 int bfs_wait(bw_context *ctx, uint32_t seq, cudaStream_t s);
 int ensure_outdeg(bw_context *ctx, const bw_graph_view *g, cudaStream_t s);
