@@ -409,8 +409,8 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
     unsigned grid = static_cast<unsigned>(ctx->sm_count) * static_cast<unsigned>(std::max(1, std::min(per_sm, 2)));
     if (cfg && cfg->grid_size) grid = cfg->grid_size;
     if (cfg && cfg->block_size && cfg->block_size != BATCH_THREADS) return BW_ERR_INVALID_ARGUMENT;
+    BW_CUDA(cudaEventRecord(ctx->ev_start, s));         // device_ms: also of a pass that is given back
     if (multi_source(g, mode)) {
-        BW_CUDA(cudaEventRecord(ctx->ev_start, s));
         uint64_t traversed = 0;
         bool done = false;
         BW_TRY(bfs_multi_source(ctx, g, roots, unit_count, levels, &traversed, &done, s));
@@ -439,7 +439,6 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
     a.levels = levels;
     a.ranks = ranks;
     const uint32_t pr = mode == BW_BATCH_GRAPHS ? pr_iterations : 0;
-    BW_CUDA(cudaEventRecord(ctx->ev_start, s));
     a.pr_iters = pr;
     if (pr && packed_pagerank(g, max_unit_vertices, pr)) {
         const int rc = pagerank_run_packed(ctx, g, graph_offsets, graph_count, pr, ranks, s);
