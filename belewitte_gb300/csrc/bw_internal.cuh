@@ -17,7 +17,9 @@ constexpr unsigned FULL_MASK = 0xffffffffu;
 // ---------------------------------------------------------------------------
 // Error handling: every CUDA call is checked, the message is kept per thread
 // and the C ABI returns BW_ERR_CUDA (the reference prints and exits instead,
-// CUDA.cpp:7-26).
+// CUDA.cpp:7-26).  A reported error is taken from the runtime, which would
+// hand a refused allocation to the next call's check after its launches (an
+// error that spoils the context stays with the runtime).
 // ---------------------------------------------------------------------------
 void set_last_error(cudaError_t e, const char *what);
 
@@ -26,6 +28,7 @@ void set_last_error(cudaError_t e, const char *what);
         cudaError_t bw_err_ = (call);                                       \
         if (bw_err_ != cudaSuccess) {                                       \
             ::bw::set_last_error(bw_err_, #call);                           \
+            cudaGetLastError();                                             \
             return bw_err_ == cudaErrorMemoryAllocation                     \
                        ? BW_ERR_OUT_OF_MEMORY : BW_ERR_CUDA;                \
         }                                                                   \
