@@ -413,7 +413,7 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
     if (multi_source(g, mode)) {
         uint64_t traversed = 0;
         bool done = false;
-        BW_TRY(bfs_multi_source(ctx, g, roots, unit_count, levels, &traversed, &done, s));
+        BW_TRY(bfs_multi_source(ctx, g, roots, order, unit_count, levels, &traversed, &done, s));
         if (done) {
             BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
             BW_CUDA(cudaEventSynchronize(ctx->ev_stop));

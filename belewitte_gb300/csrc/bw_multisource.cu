@@ -63,8 +63,9 @@ struct MsArgs {
     const uint32_t *off, *src;                     // reverse CSR
     const uint32_t *fwd_off;
     uint32_t n;
-    const uint32_t *roots;
-    uint32_t sources;                              // of this pass
+    const uint32_t *roots;                         // by unit
+    const uint32_t *order;                         // the units to run, as bw_batch_run takes them; nullptr: 0, 1, ..
+    uint32_t first, sources;                       // of this pass
     uint32_t *visited;                             // [n][W]
     uint32_t *front[2];                            // [n][W] by level parity
     uint32_t *bitmap[2];                           // a bit per vertex: in that frontier
@@ -73,8 +74,14 @@ struct MsArgs {
     uint32_t *heavy_acc;                           // [heavy][W]
     uint2 *chunk;                                  // {vertex, first edge}
     MsCtl *ctl;
-    int32_t *levels;                               // of the pass's first source
+    int32_t *levels;                               // [unit][n]
 };
+
+// The unit of the pass's source i.
+__device__ __forceinline__ uint32_t unit_of(const MsArgs &a, uint32_t i)
+{
+    return a.order ? a.order[a.first + i] : a.first + i;
+}
 
 // Bits of word w that belong to sources.
 __device__ __forceinline__ uint32_t valid_bits(uint32_t sources, uint32_t w)
@@ -88,7 +95,7 @@ __global__ void k_ms_roots(MsArgs a)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.sources) return;
-    const uint32_t r = a.roots[i], bit = 1u << (i & 31);
+    const uint32_t r = a.roots[unit_of(a, i)], bit = 1u << (i & 31);
     atomicOr(&a.visited[uint64_t(r) * W + (i >> 5)], bit);
     atomicOr(&a.front[0][uint64_t(r) * W + (i >> 5)], bit);
     atomicOr(&a.ctl->live[0][i >> 5], bit);
@@ -336,8 +343,8 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_depths(MsArgs a)
             trav += static_cast<unsigned long long>(__popc(vis[q])) * (a.fwd_off[v + 1] - a.fwd_off[v]);
         }
         const uint32_t cnt = min(32u, a.sources - 32 * w);
-        int32_t *out = a.levels + uint64_t(32 * w) * a.n + v0;
-        for (uint32_t b = 0; b < cnt; b++, out += a.n) {
+        for (uint32_t b = 0; b < cnt; b++) {
+            int32_t *out = a.levels + uint64_t(unit_of(a, 32 * w + b)) * a.n + v0;
 #pragma unroll
             for (int q = 0; q < MS_OUT; q++) {
                 int32_t d = 0;
@@ -387,8 +394,8 @@ int run_pass(bw_context *ctx, const MsArgs &a, uint32_t levels, bool &done, cuda
 // BFS from `count` sources; *done = false when the graph needs more levels
 // than the planes hold or memory is short, with nothing a caller may use
 // written.  traversed: out-edges of the reached vertices, summed over sources.
-int bfs_multi_source(bw_context *ctx, const bw_graph_view *g, const uint32_t *roots, uint32_t count, int32_t *levels,
-                     uint64_t *traversed, bool *done, cudaStream_t s)
+int bfs_multi_source(bw_context *ctx, const bw_graph_view *g, const uint32_t *roots, const uint32_t *order,
+                     uint32_t count, int32_t *levels, uint64_t *traversed, bool *done, cudaStream_t s)
 {
     *done = false;
     *traversed = 0;
@@ -410,6 +417,7 @@ int bfs_multi_source(bw_context *ctx, const bw_graph_view *g, const uint32_t *ro
     MsArgs a{};
     a.off = g->rev_vertices; a.src = g->rev_edges; a.fwd_off = g->fwd_vertices;
     a.n = n;
+    a.roots = roots; a.order = order; a.levels = levels;
     a.ctl = reinterpret_cast<MsCtl *>(mem);
     a.visited = reinterpret_cast<uint32_t *>(mem + o_vis);
     a.front[0] = a.visited + uint64_t(n) * W;
@@ -425,9 +433,8 @@ int bfs_multi_source(bw_context *ctx, const bw_graph_view *g, const uint32_t *ro
         BW_CUDA(cudaMemsetAsync(a.heavy_acc, 0, hcap * W * 4, s));
         k_ms_chunks<<<ctx->sm_count * 4, 256, 0, s>>>(a);
         for (uint32_t first = 0; first < count; first += 32 * W) {
-            a.roots = roots + first;
+            a.first = first;
             a.sources = std::min(count - first, 32 * W);
-            a.levels = levels + uint64_t(first) * n;
             bool ok = false;
             int rc = BW_ERR_INVALID_ARGUMENT;
             switch (W) {
