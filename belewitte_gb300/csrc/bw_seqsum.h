@@ -24,8 +24,9 @@
 // the new binade.  Partial sums of non-negative terms never decrease, so a
 // row crosses at most a few dozen binades.
 //
-// Terms outside the domain (negative, subnormal, infinite, NaN) and a sum
-// that overflows are reported to the caller, which then runs the plain loop.
+// Terms outside the domain (negative, infinite, NaN; for the term-by-term
+// maps subnormal ones too) and a sum that overflows are reported to the
+// caller, which then runs the plain loop.
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -91,8 +92,10 @@ BWS_HD bool step(uint32_t xb, uint32_t k, Map &m)
     return true;
 }
 
-// The same map without branches (selects only), for warps whose lanes take
-// different cases at once; `ok` is cleared for terms outside the domain.
+// The same map without branches (selects only); `ok` is cleared for terms
+// outside the domain.  The kernels take their maps from Chain (below); this
+// form, compose_short and saturated are the term-by-term one that the CPU
+// tests hold against step and the plain loop.
 // Both increments are one rounding of mx / 2^d (mx the term's significand,
 // d = k - kx): to nearest with ties to an even quotient (A even: the sum's
 // new significand is even) or to an odd one (A odd), each an addition and
