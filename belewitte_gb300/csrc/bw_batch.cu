@@ -57,14 +57,47 @@ struct BatchArgs {
     uint32_t vis_words;       // > 0: the unit's visited set is a shared-memory bitmap of this many words
     uint32_t bu_div;          // a level whose frontier holds more than 1/bu_div of the unit runs bottom-up
     unsigned long long *traversed;
+    // Many sources that bfs_multi_source has begun: the units of pass t / pass
+    // are done (MS_DONE), have their depths up to resume[t / pass], or start at
+    // their roots (0).  nullptr: all start at their roots.
+    const int32_t *resume;
+    uint32_t pass;
 };
 
 __device__ __forceinline__ bool relax_local(int32_t *lv, uint32_t v, int32_t nd)
 { return lv[v] > nd && atomicMin(&lv[v], nd) > nd; }
 
+// The frontier at depth `from` and the visited set from the depths of the
+// vertices 0 .. n - 1, RESUME_UNROLL loads in flight a lane.
+constexpr int RESUME_UNROLL = 8;
+__device__ void resume_unit(const int32_t *lv, uint32_t n, int32_t from, uint32_t *vis, uint32_t *queue, uint32_t *qlen,
+                            unsigned wib, unsigned lane)
+{
+    for (uint64_t v0 = wib * 32; v0 < n; v0 += uint64_t(BATCH_THREADS) * RESUME_UNROLL) {
+        int32_t d[RESUME_UNROLL];
+#pragma unroll
+        for (int j = 0; j < RESUME_UNROLL; j++) {
+            const uint64_t v = v0 + uint64_t(j) * BATCH_THREADS + lane;
+            d[j] = v < n ? lv[v] : INF;
+        }
+#pragma unroll
+        for (int j = 0; j < RESUME_UNROLL; j++) {
+            const uint64_t w0 = v0 + uint64_t(j) * BATCH_THREADS;
+            const unsigned seen = __ballot_sync(FULL_MASK, d[j] != INF), here = __ballot_sync(FULL_MASK, d[j] == from);
+            if (vis && lane == 0 && w0 < n) vis[w0 / 32] = seen;
+            if (here == 0) continue;
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(qlen, static_cast<uint32_t>(__popc(here)));
+            base = __shfl_sync(FULL_MASK, base, 0);
+            if (d[j] == from) queue[base + __popc(here & ((1u << lane) - 1u))] = static_cast<uint32_t>(w0) + lane;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(BATCH_THREADS, 2) k_batch(BatchArgs a)
 {
     __shared__ uint32_t s_unit, s_qlen[2], s_heavy_n;
+    __shared__ int32_t s_from;
     __shared__ uint32_t s_heavy[HEAVY_SLOTS];
     __shared__ uint32_t s_excl[BATCH_WARPS][32], s_start[BATCH_WARPS][32];
     __shared__ double s_base;
@@ -79,8 +112,11 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) k_batch(BatchArgs a)
                       a.contrib + static_cast<size_t>(blockIdx.x) * 2 * a.qcap + a.qcap};
     for (;;) {
         if (tid == 0) {
-            const uint32_t t = atomicAdd(a.cursor, 1u);
+            uint32_t t;
+            do t = atomicAdd(a.cursor, 1u);
+            while (a.resume && t < a.units && a.resume[t / a.pass] == MS_DONE);
             s_unit = t < a.units ? (a.order ? a.order[t] : t) : NO_UNIT;
+            s_from = a.resume && t < a.units ? a.resume[t / a.pass] : 0;
             s_trav = 0;
         }
         __syncthreads();
@@ -97,23 +133,30 @@ __global__ void __launch_bounds__(BATCH_THREADS, 2) k_batch(BatchArgs a)
             ve = static_cast<uint32_t>(a.n);
             lv = a.levels + static_cast<size_t>(unit) * a.n;
         }
-        const uint32_t root = a.roots[unit];
-        for (uint32_t v = vb + tid; v < ve; v += BATCH_THREADS) lv[v] = v == root ? 0 : INF;
+        const int32_t from = s_from;
         const bool bitmap = a.vis_words != 0;
-        if (bitmap) {
-            for (uint32_t w = tid; w < (ve - vb + 31) / 32; w += BATCH_THREADS) s_vis[w] = 0u;
+        if (from == 0) {
+            const uint32_t root = a.roots[unit];
+            for (uint32_t v = vb + tid; v < ve; v += BATCH_THREADS) lv[v] = v == root ? 0 : INF;
+            if (bitmap) {
+                for (uint32_t w = tid; w < (ve - vb + 31) / 32; w += BATCH_THREADS) s_vis[w] = 0u;
+                __syncthreads();
+            }
+            if (tid == 0) {
+                if (bitmap) s_vis[(root - vb) >> 5] = 1u << ((root - vb) & 31);
+                q[0][0] = root;
+                s_qlen[0] = 1;
+                s_qlen[1] = 0;
+                s_heavy_n = 0;
+            }
+        } else {
+            if (tid == 0) s_qlen[0] = s_qlen[1] = s_heavy_n = 0;
             __syncthreads();
-        }
-        if (tid == 0) {
-            if (bitmap) s_vis[(root - vb) >> 5] = 1u << ((root - vb) & 31);
-            q[0][0] = root;
-            s_qlen[0] = 1;
-            s_qlen[1] = 0;
-            s_heavy_n = 0;
+            resume_unit(lv, ve, from, bitmap ? s_vis : nullptr, q[from & 1], &s_qlen[from & 1], wib, lane);
         }
         __syncthreads();
         // ------------------------------ BFS ------------------------------
-        for (int32_t depth = 0;; depth++) {
+        for (int32_t depth = from;; depth++) {
             const uint32_t len = s_qlen[depth & 1];
             if (len == 0) break;
             const int32_t nd = depth + 1;
@@ -365,7 +408,12 @@ bool packed_pagerank(const bw_graph_view *g, uint32_t max_unit_vertices, uint32_
 // 30,000 vertices R-MAT 0.26 / 0.21 and 0.40 / 0.46, ER 0.26 / 0.17 and
 // 0.43 / 0.48; 60,000 R-MAT 0.31 / 0.52 and 0.45 / 0.83, BA 0.34 / 0.25 and
 // 0.57 / 0.76; 120,000 R-MAT 0.30 / 0.48 and 0.47 / 1.64, ER 0.28 / 0.82 and
-// 0.50 / 2.09, BA 0.36 / 0.46 and 0.63 / 1.57.
+// 0.50 / 2.09, BA 0.36 / 0.46 and 0.63 / 1.57.  A traversal of more than 31
+// levels is finished on CTAs from there: 4 and 512 sources on R-MAT-18
+// symmetrised with a path of 60 vertices 1.1 and 2.1 ms (all on CTAs 3.0 and
+// 4.9, without the path 0.50 and 0.94).  What is given back as a mesh costs
+// 0.1 to 0.3 ms first: 1 and 512 sources on the 512 x 512 grid 3.34 and 8.06
+// (3.26 and 7.93 on CTAs alone), on ER(500K, 1.5M) with one source 3.46 (3.24).
 bool multi_source(const bw_graph_view *g, int mode)
 {
     return mode == BW_BATCH_SOURCES && g->rev_vertices && g->rev_edges && g->vertex_count >= MULTI_MIN_VERTICES &&
@@ -410,11 +458,12 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
     if (cfg && cfg->grid_size) grid = cfg->grid_size;
     if (cfg && cfg->block_size && cfg->block_size != BATCH_THREADS) return BW_ERR_INVALID_ARGUMENT;
     BW_CUDA(cudaEventRecord(ctx->ev_start, s));         // device_ms: also of a pass that is given back
+    uint64_t traversed = 0;                             // of units that need no CTA
+    std::vector<int32_t> resume;
+    BatchArgs a{};
     if (multi_source(g, mode)) {
-        uint64_t traversed = 0;
-        bool done = false;
-        BW_TRY(bfs_multi_source(ctx, g, roots, order, unit_count, levels, &traversed, &done, s));
-        if (done) {
+        BW_TRY(bfs_multi_source(ctx, g, roots, order, unit_count, levels, &traversed, &a.pass, resume, s));
+        if (!resume.empty() && std::all_of(resume.begin(), resume.end(), [](int32_t d) { return d == MS_DONE; })) {
             BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
             BW_CUDA(cudaEventSynchronize(ctx->ev_stop));
             if (result) {
@@ -427,7 +476,6 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
             return BW_OK;
         }
     }
-    BatchArgs a{};
     a.fwd_v = g->fwd_vertices; a.fwd_e = g->fwd_edges; a.rev_v = g->rev_vertices; a.rev_e = g->rev_edges;
     a.n = g->vertex_count;
     a.mode = mode;
@@ -454,13 +502,18 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
     a.bu_div = (cfg && cfg->chunk_size) ? cfg->chunk_size : BATCH_BU_DIV;
     const size_t per_cta = static_cast<size_t>(2) * max_unit_vertices;
     char *scratch = nullptr;
-    const size_t bytes = 64 + grid * per_cta * sizeof(uint32_t) + (a.pr_iters ? grid * per_cta * sizeof(float) : 0);
+    const size_t head = 64 + ((resume.size() * sizeof(int32_t) + 63) & ~size_t(63));
+    const size_t bytes = head + grid * per_cta * sizeof(uint32_t) + (a.pr_iters ? grid * per_cta * sizeof(float) : 0);
     BW_CUDA(ctx_malloc_async(ctx, reinterpret_cast<void **>(&scratch), bytes, s));
     BW_CUDA(cudaMemsetAsync(scratch, 0, 64, s));
     a.cursor = reinterpret_cast<uint32_t *>(scratch);
     a.traversed = reinterpret_cast<unsigned long long *>(scratch + 8);
-    a.queues = reinterpret_cast<uint32_t *>(scratch + 64);
-    a.contrib = a.pr_iters ? reinterpret_cast<float *>(scratch + 64 + grid * per_cta * sizeof(uint32_t)) : nullptr;
+    if (!resume.empty()) {
+        BW_CUDA(cudaMemcpyAsync(scratch + 64, resume.data(), resume.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+        a.resume = reinterpret_cast<const int32_t *>(scratch + 64);
+    }
+    a.queues = reinterpret_cast<uint32_t *>(scratch + head);
+    a.contrib = a.pr_iters ? reinterpret_cast<float *>(scratch + head + grid * per_cta * sizeof(uint32_t)) : nullptr;
     k_batch<<<grid, BATCH_THREADS, dyn, s>>>(a);
     BW_CUDA(cudaGetLastError());
     BW_CUDA(cudaEventRecord(ctx->ev_stop, s));
@@ -472,7 +525,7 @@ extern "C" int bw_batch_run(bw_context *ctx, const bw_graph_view *g, int mode, c
         float ms = 0.0f;
         BW_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
         result->units = unit_count;
-        result->traversed_edges = trav;
+        result->traversed_edges = traversed + trav;
         result->device_ms = ms;
     }
     return BW_OK;

@@ -5,6 +5,8 @@
 
 #include <cstdint>
 #include <climits>
+#include <vector>
+
 #include <cuda_runtime.h>
 
 #include "belewitte_gb300.h"
@@ -203,7 +205,9 @@ int pagerank_run_schedule_loop(bw_context *ctx, const bw_graph_view *g, const in
 int pagerank_run_packed(bw_context *ctx, const bw_graph_view *g, const uint32_t *goff, uint32_t graphs,
                         uint32_t iterations, float *ranks, cudaStream_t s);
 int bfs_multi_source(bw_context *ctx, const bw_graph_view *g, const uint32_t *roots, const uint32_t *order,
-                     uint32_t count, int32_t *levels, uint64_t *traversed, bool *done, cudaStream_t s);
+                     uint32_t count, int32_t *levels, uint64_t *traversed, uint32_t *pass,
+                     std::vector<int32_t> &resume, cudaStream_t s);
+constexpr int32_t MS_DONE = -1;
 int pagerank_moments(bw_context *ctx, const bw_graph_view *g, float *ls, float *lq, float *lm, cudaStream_t s);
 void pagerank_feature_vector(const bw_graph_view *g, float ls, float lq, float lm, uint32_t iteration, float *x);
 int bfs_edgeless(bw_context *ctx, const bw_graph_view *g, int variant, uint32_t root, int32_t *levels,

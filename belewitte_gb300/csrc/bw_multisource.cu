@@ -10,8 +10,10 @@
 // frontier buffer is not cleared between the levels that use it: a stale
 // word's bits reached every out-neighbour one level after they were set, so
 // they add nothing.  Depths are kept as MS_PLANES bit planes and written out
-// once at the end, a 128-byte line per source and 32 vertices; a pass that
-// would need more levels (a mesh) is given back to the caller.
+// once at the end, a 128-byte line per source and 32 vertices.  Where the
+// planes end before the traversal does, the caller goes on from the depths
+// written by then, a CTA per source; a pass that has reached little after many
+// levels (a mesh) is given back as it came.
 //
 // Work split: a warp takes 32 consecutive vertices and sweeps the in-row of
 // each that misses a bit some frontier still carries, 32 edges at a time, W
@@ -320,10 +322,10 @@ __global__ void __launch_bounds__(MS_THREADS, 6) k_ms_level(MsArgs a, uint32_t l
 }
 
 // The depths: one warp per MS_OUT x 32 vertices, word by word, so that a row
-// of the result is written MS_OUT whole lines at a time.  Also the out-edges
-// of every reached (vertex, source) pair.
+// of the result is written MS_OUT whole lines at a time.  Also, where the
+// pass is `whole`, the out-edges of every reached (vertex, source) pair.
 template<uint32_t W>
-__global__ void __launch_bounds__(MS_THREADS) k_ms_depths(MsArgs a)
+__global__ void __launch_bounds__(MS_THREADS) k_ms_depths(MsArgs a, bool whole)
 {
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, words = (a.sources + 31) / 32;
     const uint64_t plane = uint64_t(a.n) * W;
@@ -355,14 +357,18 @@ __global__ void __launch_bounds__(MS_THREADS) k_ms_depths(MsArgs a)
         }
     }
     for (int o = 16; o > 0; o >>= 1) trav += __shfl_xor_sync(FULL_MASK, trav, o);
-    if (lane == 0 && trav) atomicAdd(&a.ctl->traversed, trav);
+    if (lane == 0 && trav && whole) atomicAdd(&a.ctl->traversed, trav);
 }
 
+// One pass.  resume: MS_DONE, or the depth up to which its sources' depths are
+// written, their frontiers being the vertices at that depth; 0 with nothing
+// written where `mesh` says that little had been reached (going on from there
+// instead: 512 sources on the 1024 x 1024 grid 45.0 ms, from the roots 43.7).
 template<uint32_t W>
-int run_pass(bw_context *ctx, const MsArgs &a, uint32_t levels, bool &done, cudaStream_t s)
+int run_pass(bw_context *ctx, const MsArgs &a, int32_t &resume, bool &mesh, cudaStream_t s)
 {
     const unsigned grid = static_cast<unsigned>(ctx->sm_count) * MS_BLOCKS_PER_SM;
-    done = false;
+    bool done = false;
     BW_CUDA(cudaMemsetAsync(a.visited, 0, uint64_t(a.n) * W * sizeof(uint32_t) * (3 + MS_PLANES), s));   // with the frontiers and planes
     BW_CUDA(cudaMemsetAsync(a.bitmap[0], 0, (a.n + 31) / 32 * sizeof(uint32_t), s));
     BW_CUDA(cudaMemsetAsync(a.ctl->active, 0, sizeof a.ctl->active, s));
@@ -370,8 +376,9 @@ int run_pass(bw_context *ctx, const MsArgs &a, uint32_t levels, bool &done, cuda
     BW_CUDA(cudaMemsetAsync(a.ctl->live, 0, sizeof a.ctl->live, s));
     k_ms_roots<W><<<(a.sources + 255) / 256, 256, 0, s>>>(a);
     MsCtl h;
-    for (uint32_t level = 0; level < levels && !done;) {
-        for (uint32_t end = std::min(level + MS_GROUP, levels); level < end; level++) {
+    uint32_t level = 0;
+    while (level < MS_LEVELS && !done && !mesh) {
+        for (uint32_t end = std::min(level + MS_GROUP, MS_LEVELS); level < end; level++) {
             k_ms_heavy<W><<<grid, MS_THREADS, 0, s>>>(a, level);
             k_ms_level<W><<<grid, MS_THREADS, 0, s>>>(a, level);
         }
@@ -379,25 +386,33 @@ int run_pass(bw_context *ctx, const MsArgs &a, uint32_t levels, bool &done, cuda
         BW_CUDA(cudaMemcpyAsync(&h, a.ctl, sizeof h, cudaMemcpyDeviceToHost, s));
         BW_CUDA(cudaStreamSynchronize(s));
         done = h.active[level] == 0;
-        // little reached after many levels (a mesh, a chain): not worth finishing.  Random graphs of average
-        // degree 4 have reached 1/16 of a million vertices by level 8.
-        if (!done && level >= 2 * MS_GROUP && h.bits < uint64_t(a.n) * a.sources / (level >= 4 * MS_GROUP ? 16 : 64))
-            return BW_OK;
+        // little reached after many levels (a mesh, a chain): not worth going on.  Random graphs of average
+        // degree 4 have reached 1/16 of a million vertices by level 8.  Under 48 vertices a source by level 4
+        // is less than 2.3 times as many at each level, which would not reach 1/64 of 98,304 by level 8.
+        const uint64_t pairs = uint64_t(a.n) * a.sources;
+        mesh = !done && h.bits < (level <= MS_GROUP ? uint64_t(48) * a.sources : pairs / (level < 4 * MS_GROUP ? 64 : 16));
     }
-    if (done) k_ms_depths<W><<<grid, MS_THREADS, 0, s>>>(a);
+    if (mesh) {
+        resume = 0;
+        return BW_OK;
+    }
+    k_ms_depths<W><<<grid, MS_THREADS, 0, s>>>(a, done);
     BW_CUDA(cudaGetLastError());
+    resume = done ? MS_DONE : static_cast<int32_t>(level);
     return BW_OK;
 }
 
 }  // namespace
 
-// BFS from `count` sources; *done = false when the graph needs more levels
-// than the planes hold or memory is short, with nothing a caller may use
-// written.  traversed: out-edges of the reached vertices, summed over sources.
+// BFS from `count` sources in passes of *pass.  resume[p]: how far pass p got,
+// MS_DONE or the depth to go on from (0: nothing written); empty when memory
+// is short, with nothing written.  traversed: out-edges of the reached
+// vertices, summed over the sources of the finished passes.
 int bfs_multi_source(bw_context *ctx, const bw_graph_view *g, const uint32_t *roots, const uint32_t *order,
-                     uint32_t count, int32_t *levels, uint64_t *traversed, bool *done, cudaStream_t s)
+                     uint32_t count, int32_t *levels, uint64_t *traversed, uint32_t *pass,
+                     std::vector<int32_t> &resume, cudaStream_t s)
 {
-    *done = false;
+    resume.clear();
     *traversed = 0;
     const uint32_t n = static_cast<uint32_t>(g->vertex_count);
     uint32_t W = 1;                                // words per vertex: all sources, while the scratch stays bounded
@@ -432,27 +447,28 @@ int bfs_multi_source(bw_context *ctx, const bw_graph_view *g, const uint32_t *ro
         BW_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(MsCtl), s));
         BW_CUDA(cudaMemsetAsync(a.heavy_acc, 0, hcap * W * 4, s));
         k_ms_chunks<<<ctx->sm_count * 4, 256, 0, s>>>(a);
-        for (uint32_t first = 0; first < count; first += 32 * W) {
+        *pass = 32 * W;
+        resume.assign((count + 32 * W - 1) / (32 * W), 0);
+        bool mesh = false;                         // then the passes that follow are left to the caller
+        for (uint32_t first = 0; first < count && !mesh; first += 32 * W) {
             a.first = first;
             a.sources = std::min(count - first, 32 * W);
-            bool ok = false;
+            int32_t &at = resume[first / (32 * W)];
             int rc = BW_ERR_INVALID_ARGUMENT;
             switch (W) {
-              case 1: rc = run_pass<1>(ctx, a, MS_LEVELS, ok, s); break;
-              case 2: rc = run_pass<2>(ctx, a, MS_LEVELS, ok, s); break;
-              case 4: rc = run_pass<4>(ctx, a, MS_LEVELS, ok, s); break;
-              case 8: rc = run_pass<8>(ctx, a, MS_LEVELS, ok, s); break;
-              case 16: rc = run_pass<16>(ctx, a, MS_LEVELS, ok, s); break;
-              case 32: rc = run_pass<32>(ctx, a, MS_LEVELS, ok, s); break;
+              case 1: rc = run_pass<1>(ctx, a, at, mesh, s); break;
+              case 2: rc = run_pass<2>(ctx, a, at, mesh, s); break;
+              case 4: rc = run_pass<4>(ctx, a, at, mesh, s); break;
+              case 8: rc = run_pass<8>(ctx, a, at, mesh, s); break;
+              case 16: rc = run_pass<16>(ctx, a, at, mesh, s); break;
+              case 32: rc = run_pass<32>(ctx, a, at, mesh, s); break;
             }
             BW_TRY(rc);
-            if (!ok) return BW_OK;
         }
         unsigned long long t = 0;
         BW_CUDA(cudaMemcpyAsync(&t, &a.ctl->traversed, sizeof t, cudaMemcpyDeviceToHost, s));
         BW_CUDA(cudaStreamSynchronize(s));
         *traversed = t;
-        *done = true;
         return BW_OK;
     };
     const int rc = passes();
