@@ -387,10 +387,11 @@ int run_pass(bw_context *ctx, const MsArgs &a, int32_t &resume, bool &mesh, cuda
         BW_CUDA(cudaStreamSynchronize(s));
         done = h.active[level] == 0;
         // little reached after many levels (a mesh, a chain): not worth going on.  Random graphs of average
-        // degree 4 have reached 1/16 of a million vertices by level 8.  Under 48 vertices a source by level 4
-        // is less than 2.3 times as many at each level, which would not reach 1/64 of 98,304 by level 8.
-        const uint64_t pairs = uint64_t(a.n) * a.sources;
-        mesh = !done && h.bits < (level <= MS_GROUP ? uint64_t(48) * a.sources : pairs / (level < 4 * MS_GROUP ? 64 : 16));
+        // degree 4 have reached 1/16 of a million vertices by level 8.  Four levels say nothing yet: a source
+        // at the end of a short path comes to the rest of its graph after them (one source, a path of 6 on
+        // R-MAT-19 symmetrised: 1.05 ms, 2.72 when given back at level 4).
+        mesh = !done && level >= 2 * MS_GROUP &&
+               h.bits < uint64_t(a.n) * a.sources / (level < 4 * MS_GROUP ? 64 : 16);
     }
     if (mesh) {
         resume = 0;

@@ -124,3 +124,19 @@ def test_a_long_path_costs_its_levels(ctx):
         took.append(min(_call(ctx, g, roots, None, levels)[1] for _ in range(6)))
     print(took)
     assert took[1] <= 4 * took[0], took
+
+
+def test_a_short_path_before_the_graph(ctx):
+    """One source at the end of a path of 6 and one at the hub the path leads
+    to: the path adds its few levels to the traversal, which stays
+    bit-parallel (given back after four levels it took 3.6 times as long)."""
+    import torch
+    h = _tailed(19, 16, 6)
+    g = bw.DeviceGraph(h, reps=CSR)
+    levels = torch.empty((1, h.vertex_count), dtype=torch.int32, device="cuda")
+    took = []
+    for source in (h.max_out_degree_vertex(), h.vertex_count - 1):
+        root = torch.tensor([source], dtype=torch.int32, device="cuda")
+        took.append(min(_call(ctx, g, root, None, levels)[1] for _ in range(8)))
+    print(took)
+    assert took[1] <= 2.5 * took[0], took
