@@ -48,7 +48,12 @@ constexpr uint32_t MS_LEVELS = (1u << MS_PLANES) - 1;
 constexpr uint32_t MS_HEAVY = 128;
 constexpr uint32_t MS_GROUP = 4;                   // levels launched between two looks at the counters
 constexpr uint32_t MS_PASS = 1024;                 // sources of a pass at most
-constexpr uint64_t MS_BYTES = uint64_t(24) << 30;  // scratch of a pass at most
+// A pass's words at most, unless one word a vertex takes more already (from
+// 805M vertices on).  The heavy rows' accumulators and chunks come on top,
+// about 1.1 bytes an edge with 32 words, and 4 bytes a vertex.  The context's
+// pool keeps at most this much of a call's scratch; what it took beyond goes
+// back to the device.
+constexpr uint64_t MS_BYTES = uint64_t(24) << 30;
 constexpr int MS_UNROLL = 8;                       // frontier words in flight per lane
 constexpr int MS_TEST = 4;                         // edges per lane and step of the bitmap test
 constexpr int MS_OUT = 4;                          // lines of a source's depths written together
@@ -478,6 +483,7 @@ int bfs_multi_source(bw_context *ctx, const bw_graph_view *g, const uint32_t *ro
     };
     const int rc = passes();
     cudaFreeAsync(mem, s);
+    if (bytes > MS_BYTES && ctx->pool && cudaStreamSynchronize(s) == cudaSuccess) cudaMemPoolTrimTo(ctx->pool, MS_BYTES);
     return rc;
 }
 
