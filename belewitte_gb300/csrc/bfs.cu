@@ -201,6 +201,13 @@ struct Launch {
     bool k2_early = true;
 };
 
+// Blocks of the hub-chunk kernel per SM, the resident ones: most levels have no
+// chunk, and starting and retiring blocks is all that it then does.  Eight (a
+// wave that waits for the first) on GB300: frontier-push on R-MAT-20
+// symmetrised 338 us a traversal, 320 so; vertex-push-warp on BA(4.2M, 12)
+// 1471 and 1404.
+constexpr unsigned HUB_BLOCKS = 4;
+
 int plan_launch(const bw_context *ctx, const bw_graph_view *g, int variant, bool side, const bw_launch_config *cfg,
                 Launch *out)
 {
@@ -256,7 +263,8 @@ int plan_launch(const bw_context *ctx, const bw_graph_view *g, int variant, bool
     else need = blocks(n, l.block);
     l.grid = static_cast<unsigned>(std::min<uint64_t>(l.grid, need));
     // at most this many hub chunks in a level (ensure_bfs_scratch), one per warp
-    l.grid2 = static_cast<unsigned>(std::min<uint64_t>(l.grid2, blocks(2 * m / 256 + n / 256, 8)));
+    l.grid2 = static_cast<unsigned>(std::min<uint64_t>(std::min(l.grid2, HUB_BLOCKS * static_cast<unsigned>(ctx->sm_count)),
+                                                       blocks(2 * m / 256 + n / 256, 8)));
     *out = l;
     return BW_OK;
 }
