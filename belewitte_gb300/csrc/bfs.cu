@@ -345,7 +345,9 @@ int traversed_edges(bw_context *ctx, const bw_graph_view *g, int32_t *levels, cu
 }
 
 // edge-list levels by chunk (k_bfs_edge_chunks), where a level would stream
-// the list from HBM and no launch shape is asked for.
+// the list from HBM and no launch shape is asked for (bfs() fills one in on
+// graphs near a class that the autotuner's cache holds, whose levels then run
+// whole: R-MAT-22 edge-list-bulk 765 us so, 552 by chunk).
 constexpr uint64_t CHUNKED_EDGES = uint64_t(16) << 20;
 bool chunked(const bw_graph_view *g, int variant, const bw_launch_config *cfg)
 {
@@ -374,15 +376,22 @@ void chunk_args(bw_context *ctx, BfsArgs *a)
 // filter saves.  Once half the vertices are visited the plain kernel has few
 // rows left.  Whole traversals on GB300, every level plain and with the filter:
 // ER(1M, 16M) 524 -> 373 us, ER(4M, 67M) 1607 -> 960, ER(8M, 32M) 1871 -> 1593;
-// R-MAT and BA, whose second level is dense, as before.
+// from the hub R-MAT-20 symmetrised 379 -> 230, R-MAT-22 1302 -> 505 and
+// BA(4.2M, 12) 1385 -> 549, from other roots (a thread per hub row then scans
+// all of it) 9.0 ms -> 0.32, 16.3 -> 0.68 and 8.5 -> 0.81.  No launch shape may
+// be asked for: bfs() fills one in on graphs near a class that the autotuner's
+// cache holds, whose levels then run plain.
 constexpr uint64_t FILTERED_EDGES = uint64_t(4) << 20;
 constexpr uint64_t FILTERED_SHARE = 256;
+// In the hub-chunk queue: the filter, then the heavy windows' pieces (a window
+// of more than FILTER_PIECE edges has at most twice edges / FILTER_PIECE).
+constexpr uint64_t FILTER_WORDS2 = FILTER_BITS / 64;
 bool filtered(const bw_context *ctx, const bw_graph_view *g, int variant, const bw_launch_config *cfg, uint64_t frontier,
               uint64_t visited)
 {
     return variant >= 20 && variant < 24 && g->edge_count >= FILTERED_EDGES && !(cfg && (cfg->block_size || cfg->grid_size)) &&
            frontier * FILTERED_SHARE <= g->vertex_count && 2 * visited <= g->vertex_count &&
-           ctx->heavy_cap * sizeof(uint2) >= FILTER_BITS / 8;
+           ctx->heavy_cap >= FILTER_WORDS2 + 2 * (g->edge_count / FILTER_PIECE);
 }
 int launch_filtered(bw_context *ctx, int variant, bool side, BfsArgs a, cudaStream_t s, bool early)
 {
@@ -390,6 +399,7 @@ int launch_filtered(bw_context *ctx, int variant, bool side, BfsArgs a, cudaStre
     while (bits < a.n && bits < FILTER_BITS) bits *= 2;
     a.filter = reinterpret_cast<uint32_t *>(ctx->heavy);
     a.filter_mask = bits - 1;
+    a.pieces = ctx->heavy + FILTER_WORDS2;
     const BfsKernelFn k = bfs_pull_filter_kernel(variant % 4, side);
     const unsigned sms = static_cast<unsigned>(ctx->sm_count);
     BW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(FILTER_BITS / 8)));

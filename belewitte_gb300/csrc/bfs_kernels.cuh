@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(512) k_bfs_edge(BfsArgs a)
 // (The reverse lists have work in nearly every chunk until their last levels.)
 // GB300, BA(8.4M, 8), 134M edges, a traversal from a hub: 1289 us with every
 // level streamed whole, 1029 by chunk (a quiet level 171 -> 25 us, the ranges
-// 80; the two large levels are 60M gathers each).  R-MAT-22 696 -> 687, a root
-// without edges there 94 -> 91.
+// 80; the two large levels are 60M gathers each).  R-MAT-22 with no launch
+// shape asked for 696 -> 687, a root without edges there 94 -> 91.
 constexpr uint32_t ACTIVE_BATCH = 4;                // chunks a warp looks at, 128 depths each in flight
 
 static __global__ void __launch_bounds__(256) k_edge_active(BfsArgs a)
@@ -619,16 +619,35 @@ __global__ void __launch_bounds__(512) k_bfs_vertex_pull(BfsArgs a)
 // every open vertex then looks at its whole in-row in vain, an L1TEX tag for
 // each index and one for each depth.  The frontier's bits (k_bfs_filter; folded
 // to FILTER_BITS where the graph has more vertices) go to every block's shared
-// memory, and a warp streams the in-rows of 32 neighbouring vertices, one
-// contiguous range, 32 edges a load: an edge costs a bit test, and only those
-// whose bit is set look for their row and at the depth.
+// memory, and a warp streams the in-rows of 32 neighbouring vertices (a
+// window), one contiguous range, 32 edges a load: an edge costs a bit test, and
+// only those whose bit is set look for their row and at the depth.  Windows of
+// more than FILTER_PIECE edges (R-MAT's hubs are neighbours in id) are cut into
+// pieces of so many, listed by k_bfs_filter: as one task of one warp such a
+// window held the level, R-MAT-20 symmetrised from its hub 2020 us.
 static __global__ void __launch_bounds__(256) k_bfs_filter(BfsArgs a)
 {
+    const unsigned lane = threadIdx.x & 31;
+    const uint64_t words = (uint64_t(a.filter_mask) + 1) / 32, n = a.n, windows = (n + 31) / 32;
+    auto edges_of = [&](uint64_t j) {
+        return j < windows ? __ldg(a.rev_v + min(32 * j + 32, n)) - __ldg(a.rev_v + 32 * j) : 0u;
+    };
+    uint32_t total = edges_of(gtid());                 // before the wait: the graph is older than the run
     chain_wait();
     const int32_t depth = level_depth(a);
     const int32_t *lv = a.levels;
-    const unsigned lane = threadIdx.x & 31;
-    const uint64_t words = (uint64_t(a.filter_mask) + 1) / 32, n = a.n;
+    // the heavy windows' pieces
+    for (uint64_t j0 = gtid() - lane; j0 < windows; j0 += gthreads(), total = edges_of(j0 + lane)) {
+        for (unsigned heavy = __ballot_sync(FULL_MASK, total > FILTER_PIECE); heavy; heavy &= heavy - 1) {
+            const int l = __ffs(heavy) - 1;
+            const uint32_t count = __shfl_sync(FULL_MASK, (total - 1) / FILTER_PIECE + 1, l);
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&a.ctl->slot[depth % 3].heavy, count);
+            at = __shfl_sync(FULL_MASK, at, 0);
+            for (uint32_t c = lane; c < count; c += 32)
+                a.pieces[at + c] = make_uint2(static_cast<uint32_t>(j0) + l, c * FILTER_PIECE);
+        }
+    }
     for (uint64_t w = gtid() >> 5; w < words; w += gthreads() >> 5) {
         uint32_t bits = 0;
 #pragma unroll 4
@@ -654,45 +673,93 @@ __global__ void __launch_bounds__(1024, 1) k_bfs_pull_filter(BfsArgs a)
     int32_t *lv = a.levels;
     Counter<RED> cnt;
     Side<SIDE> side;
+    const unsigned lane = threadIdx.x & 31;
+    const uint64_t n = a.n, windows = (n + 31) / 32, tasks = windows + slot->heavy, warps = gthreads() >> 5;
+    // the windows, then the pieces of the heavy ones; the next task's rows'
+    // bounds and depths are loaded one task ahead
+    uint32_t next_off = 0, next_end = 0, next_k0 = 0, next_v0 = 0;
+    int32_t next_depth = 0;
+    auto fetch = [&](uint64_t t) {
+        if (t >= tasks) return;
+        uint64_t w = t;
+        if (t >= windows) {
+            const uint2 piece = a.pieces[t - windows];
+            w = piece.x;
+            next_k0 = piece.y;
+        }
+        const uint64_t v = 32 * w + lane;
+        next_v0 = static_cast<uint32_t>(32 * w);
+        next_off = __ldg(a.rev_v + min(v, n));
+        next_end = __ldg(a.rev_v + min(32 * w + 32, n));
+        next_depth = v < n ? lv[v] : 0;
+    };
+    fetch(gtid() >> 5);
     const uint32_t mask = a.filter_mask, quads = (mask + 1) / 128;
     for (uint32_t i = threadIdx.x; i < quads; i += blockDim.x)
         reinterpret_cast<uint4 *>(s_filter)[i] = __ldcg(reinterpret_cast<const uint4 *>(a.filter) + i);
     __syncthreads();
-    const unsigned lane = threadIdx.x & 31;
-    const uint64_t n = a.n, stride = gthreads();
-    // the next 32 rows' bounds and depths are loaded one step ahead
-    uint32_t next_off = 0, next_end = 0;
-    int32_t next_depth = 0;
-    auto fetch = [&](uint64_t v0) {
-        if (v0 >= n) return;
-        const uint64_t v = v0 + lane;
-        next_off = __ldg(a.rev_v + min(v, n));
-        next_end = __ldg(a.rev_v + min(v0 + 32, n));
-        next_depth = v < n ? lv[v] : 0;
-    };
-    fetch(gtid() - lane);
-    for (uint64_t v0 = gtid() - lane; v0 < n; v0 += stride) {
-        const uint32_t off = next_off, end = next_end;
-        const bool open = next_depth > nd;
-        fetch(v0 + stride);
-        if (!__any_sync(FULL_MASK, open)) continue;
-        const uint32_t base = __shfl_sync(FULL_MASK, off, 0), excl = off - base, total = end - base;
-        for (uint32_t k0 = 0; k0 < total; k0 += 32 * FILTER_UNROLL) {
-            uint32_t p[FILTER_UNROLL];
+    // up to FILTER_UNROLL in-edges a lane: in-neighbour p of the row that
+    // row_of gives for load u (every lane calls it, where some lane has a hit)
+    auto test = [&](const uint32_t (&p)[FILTER_UNROLL], auto row_of) {
+        bool hit[FILTER_UNROLL];
+        bool any = false;
 #pragma unroll
-            for (int u = 0; u < FILTER_UNROLL; u++) {
-                const uint32_t k = k0 + u * 32 + lane;
-                p[u] = k < total ? __ldcs(a.rev_e + base + k) : NO_VERTEX;
+        for (int u = 0; u < FILTER_UNROLL; u++) {
+            hit[u] = p[u] != NO_VERTEX && (s_filter[(p[u] & mask) >> 5] >> (p[u] & 31) & 1u);
+            any = any || hit[u];
+        }
+        if (!__any_sync(FULL_MASK, any)) return;
+        int32_t d[FILTER_UNROLL];
+#pragma unroll
+        for (int u = 0; u < FILTER_UNROLL; u++) d[u] = hit[u] ? lv[p[u]] : nd;
+#pragma unroll
+        for (int u = 0; u < FILTER_UNROLL; u++) {
+            if (!__any_sync(FULL_MASK, d[u] == depth)) continue;
+            const uint32_t w = row_of(u);
+            if (d[u] == depth && lv[w] > nd && atomicMin(&lv[w], nd) > nd) {
+                cnt.hit(&slot->frontier);
+                side.visit(a, qnext, slot, w);
             }
+        }
+    };
+    for (uint64_t t = gtid() >> 5; t < tasks; t += warps) {
+        const uint32_t off = next_off, end = next_end, v0 = next_v0, k0 = next_k0;
+        const bool open = next_depth > nd;
+        fetch(t + warps);
+        const uint32_t base = __shfl_sync(FULL_MASK, off, 0), excl = off - base, total = end - base;
+        if (t < windows && total > FILTER_PIECE) continue;
+        const uint32_t k1 = k0 + min(total - k0, FILTER_PIECE);
+        const uint32_t below = __shfl_down_sync(FULL_MASK, off, 1);
+        const uint32_t s = max(off, base + k0), e = min(lane == 31 ? end : below, base + k1);
+        const uint32_t len = open && e > s ? e - s : 0u, wanted = __reduce_add_sync(FULL_MASK, len);
+        if (wanted == 0) continue;
+        if (wanted >= (k1 - k0) / 2) {
+            for (uint32_t b = k0; b < k1; b += 32 * FILTER_UNROLL) {
+                uint32_t p[FILTER_UNROLL];
 #pragma unroll
-            for (int u = 0; u < FILTER_UNROLL; u++) {
-                const bool hit = p[u] != NO_VERTEX && (s_filter[(p[u] & mask) >> 5] >> (p[u] & 31) & 1u);
-                if (!__any_sync(FULL_MASK, hit)) continue;
-                const uint32_t w = static_cast<uint32_t>(v0) + concat_row(excl, k0 + u * 32 + lane);
-                if (hit && lv[p[u]] == depth && lv[w] > nd && atomicMin(&lv[w], nd) > nd) {
-                    cnt.hit(&slot->frontier);
-                    side.visit(a, qnext, slot, w);
+                for (int u = 0; u < FILTER_UNROLL; u++) {
+                    const uint32_t k = b + u * 32 + lane;
+                    p[u] = k < k1 ? __ldcs(a.rev_e + base + k) : NO_VERTEX;
                 }
+                test(p, [&](int u) { return v0 + concat_row(excl, b + u * 32 + lane); });
+            }
+        } else {
+            // mostly rows already reached: the open ones' edges one after the other
+            uint32_t incl = len;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL_MASK, incl, o);
+                if (lane >= static_cast<unsigned>(o)) incl += y;
+            }
+            const uint32_t before = incl - len, from = s - before;
+            for (uint32_t b = 0; b < wanted; b += 32 * FILTER_UNROLL) {
+                uint32_t p[FILTER_UNROLL];
+#pragma unroll
+                for (int u = 0; u < FILTER_UNROLL; u++) {
+                    const uint32_t k = b + u * 32 + lane;
+                    const uint32_t i = __shfl_sync(FULL_MASK, from, concat_row(before, k)) + k;
+                    p[u] = k < wanted ? __ldcs(a.rev_e + i) : NO_VERTEX;
+                }
+                test(p, [&](int u) { return v0 + concat_row(before, b + u * 32 + lane); });
             }
         }
     }

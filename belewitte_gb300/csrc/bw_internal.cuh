@@ -139,9 +139,12 @@ struct BfsArgs {
     uint32_t *active;             // its chunks with work in this level (slot->heavy of them)
     uint32_t *filter;             // k_bfs_pull_filter: the frontier's bits, filter_mask + 1 of them
     uint32_t filter_mask;
+    uint2 *pieces;                // its heavy windows' pieces {window, first edge} (slot->heavy of them)
 };
 // Bits of the frontier filter at most (128 KB of a block's shared memory).
 constexpr uint32_t FILTER_BITS = 1u << 20;
+// In-edges of a window (32 neighbouring vertices) that one warp takes at once.
+constexpr uint32_t FILTER_PIECE = 2048;
 // Edges per range: 12 bytes a chunk, in the hub-chunk queue's 64 (ensure_bfs_scratch).
 constexpr uint32_t EDGE_CHUNK = 1024;
 
