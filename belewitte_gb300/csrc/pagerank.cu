@@ -161,18 +161,45 @@ __device__ __forceinline__ void resolve_args(PrArgs &a)
 // arithmetic where it decides the result, else integer arithmetic
 // (bw_consolidate.h).  Integers alone are about 190 instructions a vertex
 // with the rest of k_consolidate_div and bound it: 3.1M vertices on GB300 20.2
-// us, with the floats first 13.6.  vertex-pull: grid 2048^2 110.6 -> 104.4 us
-// an iteration, R-MAT-22 278.5 -> 272.4.
+// us, with the floats first 13.6.
+__device__ __forceinline__ float consolidate_exact(float scaled, double base)
+{
+    bool ok;
+    const uint32_t r = bwcons::add_round_bits(static_cast<uint64_t>(__double_as_longlong(base)),
+                                              __float_as_uint(scaled), ok);
+    if (ok) return __uint_as_float(r);
+    return __double2float_rn(__dadd_rn(base, static_cast<double>(scaled)));   // outside the emulated domain
+}
+__device__ __noinline__ float consolidate_exact_call(float scaled, double base) { return consolidate_exact(scaled, base); }
+
+// How a lane whose floats do not decide gets to the integers.  The pull
+// kernels' loads and stores around the rounding are latency bound, and a branch
+// of single lanes among them costs far more than its instructions (iterations
+// on GB300, us; integers alone / EACH / as used):
+//   work list, R-MAT of 8.0M vertices, in-edgeless rows too   449 / 645 / 379
+//   work list, R-MAT-23, hub order                            334 / 299 / 295
+//   work list, BA(4.2M, 8), hub order                         324 / 336 / 322
+//   vertex-pull-warp, R-MAT of 8.0M vertices                  702 / 931 / 728
+// N a power of two makes ties, and so the integers, common (R-MAT): there
+// k_consolidate_div loses by the vote, rev-edge-list on R-MAT-23 281 -> 289.
+enum Rounding {
+    EACH,                // the lane by itself
+    VOTE,                // the active lanes together, where one has to
+    VOTE_CALL            // the same, out of line: its registers apart from the caller's
+};
+template<int R>
 __device__ __forceinline__ float consolidate_div(float acc, const BaseTerm &base)
 {
     const float scaled = __fmul_rn(DAMPING, acc);
     bool ok;
     const float f = bwcons::add_round_split(base.split, scaled, ok);
-    if (ok) return f;
-    const uint32_t r = bwcons::add_round_bits(static_cast<uint64_t>(__double_as_longlong(base.d)),
-                                              __float_as_uint(scaled), ok);
-    if (ok) return __uint_as_float(r);
-    return __double2float_rn(__dadd_rn(base.d, static_cast<double>(scaled)));   // outside the emulated domain
+    if constexpr (R == EACH) {
+        if (ok) return f;
+        return consolidate_exact(scaled, base.d);
+    }
+    if (!__any_sync(__activemask(), !ok)) return f;
+    const float exact = R == VOTE ? consolidate_exact(scaled, base.d) : consolidate_exact_call(scaled, base.d);
+    return ok ? f : exact;
 }
 
 // The graph of vertex v of packed graphs: the last that starts at v or
@@ -393,7 +420,7 @@ __global__ void __launch_bounds__(256) k_relabel_edges(const uint32_t *__restric
 __device__ __forceinline__ float consolidate_vertex(const PrArgs &a, float acc, float prev, uint32_t d, float &dsum,
                                                     float &contrib)
 {
-    const float nr = consolidate_div(acc, a.base_div);
+    const float nr = consolidate_div<EACH>(acc, a.base_div);
     dsum += fabsf(nr - prev);
     contrib = d ? __fdiv_rn(nr, static_cast<float>(d)) : 0.0f;
     return nr;
@@ -773,12 +800,12 @@ __device__ __forceinline__ FinishIn finish_load(const PrArgs &a, uint64_t v)
     return in;
 }
 
-template<bool NODIV>
+template<bool NODIV, int R>
 __device__ __forceinline__ float finish_store(const PrArgs &a, uint64_t v, float sum, float base_nd, FinishIn in,
                                               const BaseTerm &base)
 {
     if constexpr (!NODIV) {
-        const float nr = consolidate_div(sum, base);
+        const float nr = consolidate_div<R>(sum, base);
         a.pr_out[v] = nr;
         a.contrib_out[in.at] = in.dg ? __fdiv_rn(nr, static_cast<float>(in.dg)) : 0.0f;
         return fabsf(nr - in.prev);
@@ -799,16 +826,16 @@ __device__ __forceinline__ float finish_row(const PrArgs &a, uint64_t v, float s
 {
     if constexpr (MULTI) {
         if (g == NO_GRAPH) return 0.0f;
-        return finish_store<NODIV>(a, v, sum, base_nd, in, a.gbase[g]);
+        return finish_store<NODIV, VOTE_CALL>(a, v, sum, base_nd, in, a.gbase[g]);
     } else {
-        return finish_store<NODIV>(a, v, sum, base_nd, in, a.base_div);
+        return finish_store<NODIV, VOTE_CALL>(a, v, sum, base_nd, in, a.base_div);
     }
 }
 
 template<bool NODIV>
 __device__ __forceinline__ float finish_vertex(const PrArgs &a, uint64_t v, float sum, float base_nd)
 {
-    return finish_store<NODIV>(a, v, sum, base_nd, finish_load<NODIV>(a, v), a.base_div);
+    return finish_store<NODIV, VOTE>(a, v, sum, base_nd, finish_load<NODIV>(a, v), a.base_div);
 }
 
 // ----------------------------- pull variants ------------------------------
