@@ -849,6 +849,11 @@ __device__ __forceinline__ float finish_vertex(const PrArgs &a, uint64_t v, floa
 // flight; each lane adds the terms of its run of one row in a register and
 // flushes the run into the row's shared-memory accumulator; then the lanes
 // consolidate the chunk's vertices together.
+// The rank difference: on large graphs an atomic per warp, whose blocks then do
+// not wait for their last one (iterations on GB300, us, per block / per warp:
+// R-MAT of 8.0M vertices 726 / 685, R-MAT-22 498 / 464, BA(4.2M, 8) 505 / 505;
+// the 1000 x 1001 grid 31 / 35, where the atomics are what is left at the end).
+constexpr uint64_t DIFF_BY_WARP = uint64_t(1) << 22;
 template<bool NODIV>
 __global__ void __launch_bounds__(512) k_pr_vertex_pull_warp(PrArgs a)
 {
@@ -913,7 +918,8 @@ __global__ void __launch_bounds__(512) k_pr_vertex_pull_warp(PrArgs a)
         for (uint32_t i = lane; i < cnt; i += W) dsum += finish_vertex<NODIV>(a, v0 + i, my_acc[i], base_nd);
         __syncwarp(mask);
     }
-    add_diff_block(a.diff, dsum);
+    if (n >= DIFF_BY_WARP) add_diff(a.diff, dsum);
+    else add_diff_block(a.diff, dsum);
 }
 
 // Tiles of the heavy units queued by this iteration's first kernel
