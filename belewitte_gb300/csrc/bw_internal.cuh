@@ -227,9 +227,12 @@ inline cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
 // chain_wait() in every thread (without the attribute it does nothing); what
 // the kernels before it wrote is not read through the non-coherent path
 // (__ldg), whose lines may be older than the wait.
-__device__ __forceinline__ void chain_wait()
+// late: the next kernel is launched when this one's blocks have ended, not as
+// soon as the last has begun.  For kernels whose blocks end at different times:
+// the next one's would gather on the SMs that are free first.
+__device__ __forceinline__ void chain_wait(bool late = false)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template<class Kernel, class... Args>

@@ -135,6 +135,7 @@ struct PrArgs {
     const uint32_t *goff;
     const BaseTerm *gbase;
     uint32_t graphs;
+    bool late;                 // vertex-push-warp and its consolidation: see LATE_EDGES
 };
 
 __device__ __forceinline__ uint64_t gtid() { return blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; }
@@ -427,7 +428,7 @@ __device__ __forceinline__ float consolidate_vertex(const PrArgs &a, float acc, 
 }
 __global__ void __launch_bounds__(256) k_consolidate_div(PrArgs a, int rowlen)
 {
-    chain_wait();
+    chain_wait(a.late);
     float dsum = 0.0f;
     const uint64_t n = a.n;
     const uint32_t *deg = rowlen ? a.fwd_v : a.deg;
@@ -696,7 +697,7 @@ __device__ __forceinline__ void enqueue_tiles(const PrArgs &a, uint32_t unit, ui
 
 __global__ void __launch_bounds__(256) k_pr_vertex_push(PrArgs a)
 {
-    chain_wait();
+    chain_wait(true);
     const unsigned lane = threadIdx.x & 31;
     for (uint64_t w0 = gtid() - lane; w0 < a.n; w0 += gthreads()) {
         const uint64_t v = w0 + lane;
@@ -740,7 +741,7 @@ __global__ void __launch_bounds__(256) k_pr_vertex_push(PrArgs a)
 // each lane finds the row of its edge by a cursor over the staged offsets.
 __global__ void __launch_bounds__(512) k_pr_vertex_push_warp(PrArgs a)
 {
-    chain_wait();
+    chain_wait(a.late);
     extern __shared__ uint32_t smem[];
     const uint32_t W = a.warp_size, C = a.chunk_size;
     const uint32_t per_block = blockDim.x / W, vw = threadIdx.x / W, lane = threadIdx.x % W;
@@ -857,7 +858,7 @@ constexpr uint64_t DIFF_BY_WARP = uint64_t(1) << 22;
 template<bool NODIV>
 __global__ void __launch_bounds__(512) k_pr_vertex_pull_warp(PrArgs a)
 {
-    chain_wait();
+    chain_wait(true);
     extern __shared__ uint32_t smem[];
     const uint32_t W = a.warp_size, C = a.chunk_size;
     const uint32_t per_block = blockDim.x / W, vw = threadIdx.x / W, lane = threadIdx.x % W;
@@ -932,7 +933,7 @@ __global__ void __launch_bounds__(512) k_pr_vertex_pull_warp(PrArgs a)
 template<int MODE>   // 0 vertex-push, 1 vertex-push-warp, 2 vertex-pull-warp, 3 vertex-pull-warp-nodiv
 __global__ void __launch_bounds__(256) k_pr_heavy_tiles(PrArgs a)
 {
-    chain_wait();
+    chain_wait(MODE != 1);                           // (vertex-push-warp: either is the same)
     constexpr uint32_t NO_ROW = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31;
     const uint32_t tiles = min(a.heavy_ctr[0], a.heavy_cap);
@@ -1025,7 +1026,7 @@ __global__ void __launch_bounds__(256) k_pr_heavy_tiles(PrArgs a)
 template<bool NODIV>
 __global__ void __launch_bounds__(256) k_pr_heavy_finish(PrArgs a)
 {
-    chain_wait();
+    chain_wait(true);
     const unsigned lane = threadIdx.x & 31;
     const uint64_t warp = gtid() >> 5, warps = gthreads() >> 5;
     const uint32_t chunks = a.heavy_ctr[3];
@@ -2379,9 +2380,19 @@ cudaError_t launch_pull_items_div(const PrArgs &a, const Geometry &geo, cudaStre
 // vertex-push 1066 -> 878; R-MAT-22 vertex-pull 8412 -> 8363.  (Both loop modes:
 // the iterations captured into one CUDA graph took longer at every length and
 // size measured, 30 iterations of the first 306 us, 200 of them 1675 for 1024.)
+// On skewed graphs the push and warp variants' kernels end block by block, and
+// what is launched among them gathers on few SMs; they launch the next one late
+// (an iteration, us, unchained / early / late: vertex-pull-warp BA(300K, 20)
+// 178 / 213 / 168, BA(4.2M, 8) 516 / 560 / 513; vertex-push BA(1M, 6) 228 / 212 /
+// 187, R-MAT-20 368 / 365 / 341; vertex-push-warp BA(300K, 20) 221 / 235 / 195,
+// R-MAT-20 322 / 309 / 305).  vertex-push-warp on large graphs gains by the
+// early launch (R-MAT-23 1091 / 1014 / 1073, R-MAT-21 symmetrised 687 / 653 /
+// 673).
+constexpr uint64_t LATE_EDGES = 24 * MEGA;
 int launch_iteration(bw_context *ctx, int variant, PrArgs &a, const Geometry &geo, cudaStream_t s, bool early)
 {
     const unsigned sms = static_cast<unsigned>(ctx->sm_count);
+    a.late = variant == PR_VERTEX_PUSH_WARP && a.m < LATE_EDGES;
     auto run = [&](auto k, unsigned grid, unsigned block, size_t smem) {
         ctx->launches++;
         return launch_chained(k, grid, block, smem, s, early, a);
