@@ -181,6 +181,7 @@ __device__ __noinline__ float consolidate_exact_call(float scaled, double base) 
 //   work list, R-MAT-23, hub order                            334 / 299 / 295
 //   work list, BA(4.2M, 8), hub order                         324 / 336 / 322
 //   vertex-pull-warp, R-MAT of 8.0M vertices                  702 / 931 / 728
+// (packed graphs take VOTE: 26.95 ms for 512 graphs, 27.04 with the call).
 // N a power of two makes ties, and so the integers, common (R-MAT): there
 // k_consolidate_div loses by the vote, rev-edge-list on R-MAT-23 281 -> 289.
 enum Rounding {
@@ -827,7 +828,7 @@ __device__ __forceinline__ float finish_row(const PrArgs &a, uint64_t v, float s
 {
     if constexpr (MULTI) {
         if (g == NO_GRAPH) return 0.0f;
-        return finish_store<NODIV, VOTE_CALL>(a, v, sum, base_nd, in, a.gbase[g]);
+        return finish_store<NODIV, VOTE>(a, v, sum, base_nd, in, a.gbase[g]);
     } else {
         return finish_store<NODIV, VOTE_CALL>(a, v, sum, base_nd, in, a.base_div);
     }
