@@ -11,6 +11,13 @@ virtual-warp width and chunk -- on the device, and keeps the fastest per
 identical for every configuration (BFS depths bit-exact, PageRank within
 the variant's tolerance), so tuning changes time only.
 
+BFS configurations are ranked by the device loop's device_ms, which includes
+the host's gaps between the first 48 levels: on graphs whose levels take a few
+microseconds the differences between configurations are small beside them.
+A BFS configuration with a block or grid size also keeps a level's plain
+kernel: the edge lists' chunks and vertex-pull's frontier filter are taken only
+where neither is given (csrc/bfs.cu, chunked and filtered).
+
 The batched launch (bw_batch_run) switches each BFS level between
 top-down and bottom-up by a divisor: bottom-up once the frontier holds more
 than 1/divisor of the unit's vertices.  ``tune_batch`` times the batched

@@ -1,5 +1,5 @@
 """Batched persistent traversal (bw_batch_run): many graphs or many sources
-in one launch fed by a device work queue.
+in one call (bw_batch_run says which parts run as one persistent launch).
 
 Workload A (many graphs): graphs of uneven size packed into one
 concatenated CSR (global vertex ids, per-graph vertex offsets); each unit is
@@ -70,7 +70,7 @@ def pack(graphs: list[DeviceGraph], device: int = 0) -> PackedGraphs:
 
 def run_graphs(ctx, packed: PackedGraphs, pr_iterations: int = 20, levels=None, ranks=None, grid: int = 0,
                stream=None, bu_div: int | None = None):
-    """Workload A: per graph a BFS and a PageRank, in one persistent launch.
+    """Workload A: per graph a BFS and a PageRank, in one call.
     bu_div: the push/pull divisor (None: the autotuner's, else the
     library default)."""
     import torch

@@ -415,8 +415,9 @@ bool packed_pagerank(const bw_graph_view *g, uint32_t max_unit_vertices, uint32_
 // levels is finished on CTAs from there: 4 and 512 sources on R-MAT-18
 // symmetrised with a path of 60 vertices 1.1 and 2.1 ms (all on CTAs 3.0 and
 // 4.9, without the path 0.50 and 0.94).  What is given back as a mesh costs
-// 0.1 to 0.3 ms first: 1 and 512 sources on the 512 x 512 grid 3.34 and 8.06
-// (3.26 and 7.93 on CTAs alone), on ER(500K, 1.5M) with one source 3.46 (3.24).
+// 0.2 to 0.9 ms first: 1 and 512 sources on the 512 x 512 grid 3.43 and 8.21
+// (3.20 and 7.77 on CTAs alone), on the 1024 x 1024 grid 10.1 and 44.1 (9.7 and
+// 43.2).
 bool multi_source(const bw_graph_view *g, int mode)
 {
     return mode == BW_BATCH_SOURCES && g->rev_vertices && g->rev_edges && g->vertex_count >= MULTI_MIN_VERTICES &&

@@ -12,15 +12,15 @@ GTEPS = edges x iterations / time.
 The same JSON line carries:
   * learned_switch: BFS on the symmetrised R-MAT scale-24 graph, the 4096 x
     4096 grid and BA(8M, 8), 16 seeded sources of the giant component each --
-    the learned per-level switch (shipped predictor, device-side decisions in
-    a CUDA graph) against every fixed candidate variant; every depth array is
+    the learned per-level switch (shipped predictor, device-side decisions)
+    against every fixed candidate variant; every depth array is
     checked against the oracle; the learned runs' fraction of the top-down
     compulsory bytes.
   * learned_pagerank: the learned per-iteration PageRank choice (shipped
     predictor) against every fixed div-class variant, 30 iterations, on the
     headline R-MAT graph and a 4096 x 4096 grid.
   * batched: many graphs (BFS + 20-iteration PageRank each) and many BFS
-    sources, each in one persistent launch.
+    sources, each in one call.
   * parity: the headline ranks against the oracle (bit for bit) and FP64.
   * roofline of the PageRank iteration, e2e through the C ABI with host
     buffers, the CPU baselines (PageRank, and BFS on the R-MAT-24 sources),
@@ -324,7 +324,7 @@ def batched(ctx, dev, graphs: int):
     _, _, res = batch.run_graphs(ctx, packed, pr_iterations=20)
     out["graphs"] = {"workload": f"{graphs} R-MAT graphs, vertex counts log-uniform in 1,000..200,000, "
                                  "edge factor 8-32; "
-                                 "BFS from each max-degree vertex + 20 PageRank iterations, one persistent launch",
+                                 "BFS from each max-degree vertex + 20 PageRank iterations, one call",
                      "vertices": packed.vertex_count, "edges": packed.edge_count, "ms": round(res.device_ms, 3),
                      "gteps": round((res.traversed_edges + 20 * packed.edge_count) / (res.device_ms * 1e-3) / 1e9, 2),
                      "generation_s": round(gen_s, 1)}
@@ -335,7 +335,7 @@ def batched(ctx, dev, graphs: int):
     srcs = np.random.default_rng(20).choice(reach, 1024, replace=False)
     batch.run_sources(ctx, g, srcs[:64])
     levels, res = batch.run_sources(ctx, g, srcs)
-    out["sources"] = {"workload": "1024 BFS sources on R-MAT scale 20 (symmetrised), one persistent launch",
+    out["sources"] = {"workload": "1024 BFS sources on R-MAT scale 20 (symmetrised), one call",
                       "ms": round(res.device_ms, 3), "gteps": round(res.traversed_edges / (res.device_ms * 1e-3) / 1e9, 2)}
     del levels, g
     torch.cuda.empty_cache()

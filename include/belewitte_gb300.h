@@ -354,9 +354,12 @@ typedef struct bw_bfs_result {
     uint32_t reserved;
     uint64_t visited;             /* vertices with a finite depth */
     uint64_t traversed_edges;     /* sum of out-degrees of visited vertices */
-    double device_ms;             /* traversal time on the device */
+    double device_ms;             /* between events on the stream around the levels, the gaps
+                                   * included in which the host reads a level and launches the next */
 } bw_bfs_result;
 
+/* While it waits for a level the calling thread polls for up to a millisecond,
+ * then synchronises the stream. */
 enum bw_loop_mode {
     BW_LOOP_HOST = 0,    /* host loop, one frontier read-back per level */
     BW_LOOP_GRAPH = 1    /* levels counted and ended on the device: the first ones launched by
@@ -422,9 +425,9 @@ typedef struct bw_pagerank_result {
  * inside the call, as the reference does inside its timed region
  * (pagerank/pagerank.cpp:102-112).  `diffs` (optional, host) receives the
  * per-iteration diff the reference reads back (pagerank.cpp:124).
- * Either loop_mode enqueues all iterations without waiting, each kernel
- * launched while the one before it runs; the call must not be made inside a
- * stream capture.
+ * loop_mode has no effect (any value is taken): all iterations are enqueued
+ * without waiting, each kernel launched while the one before it runs.  The
+ * call must not be made inside a stream capture.
  */
 int bw_pagerank_run(bw_context *ctx, const bw_graph_view *g, int variant,
                     uint32_t iterations, float *ranks,
@@ -544,9 +547,11 @@ enum { BW_SWITCH_MLP_ONLY = 1 };
 
 /*
  * BFS whose every level runs the variant the MLP picks from that level's
- * features (fallback below the confidence threshold).  BW_LOOP_GRAPH runs
- * the prediction on the device inside the CUDA graph (a SWITCH conditional
- * node selects the level kernel); BW_LOOP_HOST predicts on the host.  The
+ * features (fallback below the confidence threshold).  BW_LOOP_GRAPH
+ * predicts on the device: for the first 48 rounds (a level each, or the many
+ * that frontier-push's cluster kernel runs) the host reads the choice and
+ * launches the level, after that a CUDA graph does both (a SWITCH conditional
+ * node selects the level kernel).  BW_LOOP_HOST predicts on the host.  The
  * depths are bit-identical to every fixed variant's; stats[level].variant
  * records the choices.
  */
@@ -592,11 +597,21 @@ int bw_pagerank_run_learned(bw_context *ctx, const bw_graph_view *g,
 /* Batched persistent traversal                                              */
 /* ------------------------------------------------------------------------ */
 /*
- * Many independent units in one persistent launch fed by a device work
- * queue (an atomic cursor over a list ordered largest first); each CTA takes
- * a unit and runs it to completion with CTA-level barriers between levels
- * and iterations.  No counterpart in the reference, which runs one
- * traversal per process (kernel-runner.cpp:222-256).
+ * Many independent units in one call.  The general form is one persistent
+ * launch fed by a device work queue (an atomic cursor over a list ordered
+ * largest first); each CTA takes a unit and runs it to completion with
+ * CTA-level barriers between levels and iterations.  No counterpart in the
+ * reference, which runs one traversal per process (kernel-runner.cpp:222-256).
+ * Two forms run part of it differently, with the same depths and ranks:
+ * - many graphs of which the largest has at least 4096 vertices, and times the
+ *   iterations at least 16384: their PageRank runs over the whole GPU, all
+ *   graphs' rows as one set, before the launch that does the traversals;
+ * - many sources on a graph of 98,304 to 2^31 vertices with a reverse CSR: they
+ *   run together, a bit per source and vertex and a kernel pair per level, up
+ *   to 1024 sources a pass.  What is not done after 31 levels goes on in the
+ *   general form from there, and a pass that has reached little by level 8 or
+ *   later (a mesh) is left to the general form.
+ * Either falls back to the general form where its scratch does not fit.
  *
  * BW_BATCH_GRAPHS: `g` is one concatenated CSR (forward + reverse, global
  *   vertex ids) of graph_count graphs; graph i owns vertices
@@ -609,10 +624,12 @@ int bw_pagerank_run_learned(bw_context *ctx, const bw_graph_view *g,
  *   depths into levels[i * vertex_count + v].
  * graph_offsets, roots and `order` (unit ids, largest first; NULL = 0..n-1)
  * are device arrays.
- * cfg (optional): grid_size (0: two CTAs per SM where they fit), block_size
- * (0 or 512), and chunk_size as the push/pull divisor -- a BFS level whose
- * frontier holds more than 1/chunk_size of the unit's vertices runs
- * bottom-up (0: 24; the autotuner's tune_batch picks it per graph class).
+ * cfg (optional), for the general form only: grid_size (0: two CTAs per SM
+ * where they fit), block_size (0 or 512), and chunk_size as the push/pull
+ * divisor -- a BFS level whose frontier holds more than 1/chunk_size of the
+ * unit's vertices runs bottom-up (0: 24; the autotuner's tune_batch picks it
+ * per graph class).  They steer nothing in sources that run together, nor in
+ * the PageRank that runs as one set of rows.
  */
 enum bw_batch_mode { BW_BATCH_GRAPHS = 0, BW_BATCH_SOURCES = 1 };
 
